@@ -822,8 +822,7 @@ int reina_postprocess_device(reina_ctx* ctx, const void* d_accum, uint32_t width
         need((uint64_t)width * height <= (1ull << 28), "image too large");
         use_device(ctx);
         rt::postprocess(ctx->post, static_cast<const float*>(d_accum), (int)width, (int)height, *bloom, *tm,
-                        static_cast<uint8_t*>(d_rgba8), static_cast<float*>(d_combined), ctx->sm_count,
-                        static_cast<cudaStream_t>(stream));
+                        static_cast<uint8_t*>(d_rgba8), static_cast<float*>(d_combined), static_cast<cudaStream_t>(stream));
     });
 }
 
@@ -841,7 +840,7 @@ int reina_postprocess(reina_ctx* ctx, const float* accum, uint32_t width, uint32
         if (combined) ctx->combined.reserve(n * 4 * sizeof(float));
         check_cuda(cudaMemcpyAsync(ctx->accum.get(), accum, n * 4 * sizeof(float), cudaMemcpyHostToDevice, st), "H2D");
         rt::postprocess(ctx->post, ctx->accum.as<float>(), (int)width, (int)height, *bloom, *tm, ctx->rgba8.as<uint8_t>(),
-                        combined ? ctx->combined.as<float>() : nullptr, ctx->sm_count, st);
+                        combined ? ctx->combined.as<float>() : nullptr, st);
         check_cuda(cudaMemcpyAsync(rgba8, ctx->rgba8.get(), n * 4, cudaMemcpyDeviceToHost, st), "D2H");
         if (combined)
             check_cuda(cudaMemcpyAsync(combined, ctx->combined.get(), n * 4 * sizeof(float), cudaMemcpyDeviceToHost, st), "D2H");

@@ -12,8 +12,8 @@
 namespace rt {
 
 struct PostWorkspace {
-    DeviceBuffer ping, pong, weights;
-    void ensure(size_t pixels, int k);
+    DeviceBuffer ping, weights;   // blurX's output (a plane per channel); weight tables and row flags
+    void ensure(size_t pixels, size_t words);
 
 private:
     size_t cap_px_ = 0, cap_w_ = 0;
@@ -21,6 +21,6 @@ private:
 
 // accum (W*H RGBA32F) -> rgba8 (W*H*4 bytes); `d_combined` (optional) receives the bloomed HDR image.
 void postprocess(PostWorkspace& ws, const float* d_accum, int W, int H, const BloomPushConsts& bloom,
-                 const TonemappingPushConsts& tm, uint8_t* d_rgba8, float* d_combined, int sm_count, cudaStream_t st);
+                 const TonemappingPushConsts& tm, uint8_t* d_rgba8, float* d_combined, cudaStream_t st);
 
 }  // namespace rt
