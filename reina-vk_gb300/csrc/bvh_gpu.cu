@@ -2,15 +2,15 @@
 // collapse to 8-wide nodes, conservative 8-bit quantization) as CUDA kernels, writing the same bytes.
 //
 // Why the bytes agree: every decision depends only on the set of primitives of a binary node (bounds are
-// minima and maxima, bin counts are counts, the SAH sweeps run serially in one lane in the host's order,
-// and all arithmetic is the shared, explicitly rounded code of bvh_sah.h); the leaf triangles of a leaf
+// minima and maxima, bin counts are counts, the SAH sweeps are scans of these with the host's choice among
+// equal costs, and all arithmetic is the shared, explicitly rounded code of bvh_sah.h); the leaf triangles of a leaf
 // child are written in ascending id order by both builders; and the wide nodes are laid out in the host's
 // depth-first order from subtree sizes (below).
 //
 // Binary build, level-synchronous: each binary node of the current level is a task over a contiguous
-// range of the primitive index array.  A task of at most kSmall primitives is handled by one warp
-// (bounds, bins in shared memory, SAH sweeps, stable ballot partition, child allocation); a larger task
-// is cut into work items of kItem primitives, which accumulate its bounds and bins with global atomics
+// range of the primitive index array.  A task of at most kTiny primitives is handled by 8 lanes in registers, one
+// of at most kSmall by one warp (bounds, bins in shared memory, SAH sweeps, stable ballot partition, child
+// allocation); a larger task is cut into work items, which accumulate its bounds and bins with global atomics
 // before one warp chooses the split and the items partition their ranges at offsets from a scan.  An
 // object-median split (forced past the median depth, or when no axis can be binned) selects the pivot
 // key (centroid, id) by rank in a warp, or by an 8-pass radix select in a block for larger tasks.
@@ -38,8 +38,15 @@ namespace {
 
 constexpr int kBT = 128;                 // threads per block (4 warps)
 constexpr int kWarps = kBT / 32;
-constexpr uint32_t kSmall = 2048;        // tasks of at most this many primitives: one warp per level step
-constexpr uint32_t kItem = 4096;         // primitives per work item of a larger task
+// Tasks of at most kSmall primitives take one warp per level step, larger ones go through work items of at least
+// kItem (item_size below): with 2048 and 4096 the top levels ran on a handful of warps, each walking its
+// primitives one dependent load after the other (327,680 triangles, kernel time under the profiler: the
+// large-task kernels 6.1 ms, now 1.1 ms).
+constexpr uint32_t kSmall = 512;
+constexpr uint32_t kItem = 256;
+// Tasks of at most kTiny primitives take 8 lanes: four of them share a warp (with the parallel sweeps below,
+// the small-task levels of the same build 2.5 ms, now 0.75 ms).
+constexpr uint32_t kTiny = 8;
 constexpr int kMaxBins = kMaxDeviceSahBins;
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
@@ -90,8 +97,13 @@ struct Ctx {
     uint32_t* lbins;            // per large task: [3][kMaxBins][7] words (box lo, box hi, count)
     uint32_t max_large, max_items, max_nodes;
     uint32_t n;                 // primitives
+    uint32_t item;              // primitives per work item
     int bins, median_depth;
 };
+
+// Work items of a build: enough of them to fill the chip, few enough that the scan over a task's items (one
+// warp, k_large_alloc) stays short.
+static uint32_t item_size(uint32_t n) { return std::max(kItem, (n / 16384u + 31u) / 32u * 32u); }
 
 // Every index the build computes from its own tables is checked before use: a failed check records the
 // site and the index (ctr[kCtrSite]) and raises kErrInternal, and the access is skipped or redirected to
@@ -172,36 +184,84 @@ __device__ void warp_bounds(const Ctx& c, uint32_t b, uint32_t n, int lane, floa
     }
 }
 
+struct BinBox {   // a run of bins: box and count
+    float lo[3], hi[3];
+    uint32_t cnt;
+};
+__device__ __forceinline__ BinBox empty_bins() {
+    return BinBox{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}, 0u};
+}
+__device__ __forceinline__ void join(BinBox& a, const BinBox& b) {
+    for (int k = 0; k < 3; ++k) {
+        a.lo[k] = fminf(a.lo[k], b.lo[k]);
+        a.hi[k] = fmaxf(a.hi[k], b.hi[k]);
+    }
+    a.cnt += b.cnt;
+}
+__device__ __forceinline__ BinBox from_lane(const BinBox& a, int lane) {
+    BinBox r;
+    for (int k = 0; k < 3; ++k) {
+        r.lo[k] = __shfl_sync(0xFFFFFFFFu, a.lo[k], lane);
+        r.hi[k] = __shfl_sync(0xFFFFFFFFu, a.hi[k], lane);
+    }
+    r.cnt = __shfl_sync(0xFFFFFFFFu, a.cnt, lane);
+    return r;
+}
+
 // The host's two sweeps over the bins of one axis (bins[i * 7 + 0..5] encoded box, [6] count): the first
 // cheapest split (bin index of its last left bin) and its cost, INFINITY when no split has both sides.
-__device__ void sah_axis(const uint32_t* bins, int nb, float parent, float* rarea, uint32_t* rcnt, float& best_cost,
-                         int& best_bin) {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    uint32_t cnt = 0;
-    for (int i = nb - 1; i > 0; --i) {
-        const uint32_t* b = bins + 7 * i;
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fmin_h(lo[k], unord(b[k]));
-            hi[k] = fmax_h(hi[k], unord(b[3 + k]));
+// A lane per bin (two rounds for more than 32): prefix and suffix scans of boxes and counts, whose minima, maxima
+// and sums do not depend on the order, then every split's cost by its own lane.  (The sweeps in one lane per
+// axis took ~3000 instructions a node, at 5 of 32 lanes active over the whole level.)
+__device__ void sah_axis(const uint32_t* bins, int nb, float parent, int lane, float& best_cost, int& best_bin) {
+    const int rounds = (nb + 31) / 32;   // 1 or 2
+    BinBox pre[2], suf[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (h >= rounds) break;
+        const int i = 32 * h + lane;
+        BinBox v = empty_bins();
+        if (i < nb) {
+            const uint32_t* b = bins + 7 * i;
+            for (int k = 0; k < 3; ++k) {
+                v.lo[k] = unord(b[k]);
+                v.hi[k] = unord(b[3 + k]);
+            }
+            v.cnt = b[6];
         }
-        cnt += b[6];
-        rarea[i] = sah::half_area(lo, hi);
-        rcnt[i] = cnt;
+        pre[h] = suf[h] = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const BinBox u = from_lane(pre[h], lane - o < 0 ? lane : lane - o);
+            const BinBox d = from_lane(suf[h], lane + o > 31 ? lane : lane + o);
+            if (lane >= o) join(pre[h], u);
+            if (lane + o < 32) join(suf[h], d);
+        }
     }
-    for (int k = 0; k < 3; ++k) { lo[k] = INFINITY; hi[k] = -INFINITY; }
-    cnt = 0;
+    if (rounds == 2) {
+        join(pre[1], from_lane(pre[0], 31));
+        join(suf[0], from_lane(suf[1], 0));
+    }
     best_cost = INFINITY;
     best_bin = -1;
-    for (int i = 0; i < nb - 1; ++i) {
-        const uint32_t* b = bins + 7 * i;
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fmin_h(lo[k], unord(b[k]));
-            hi[k] = fmax_h(hi[k], unord(b[3 + k]));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (h >= rounds) break;
+        BinBox right = from_lane(suf[h], lane < 31 ? lane + 1 : 31);
+        if (rounds == 2) {
+            const BinBox next = from_lane(suf[1], 0);
+            if (h == 0 && lane == 31) right = next;
         }
-        cnt += b[6];
-        if (cnt == 0 || rcnt[i + 1] == 0) continue;
-        const float cost = sah::split_cost(sah::half_area(lo, hi), cnt, rarea[i + 1], rcnt[i + 1], parent);
-        if (cost < best_cost) { best_cost = cost; best_bin = i; }
+        float cost = INFINITY;
+        if (32 * h + lane < nb - 1 && pre[h].cnt != 0 && right.cnt != 0)
+            cost = sah::split_cost(sah::half_area(pre[h].lo, pre[h].hi), pre[h].cnt, sah::half_area(right.lo, right.hi),
+                                   right.cnt, parent);
+        if (!(cost < INFINITY)) cost = INFINITY;   // (a NaN cost is never chosen)
+        const float least = warp_min(cost);
+        if (least < best_cost) {
+            best_cost = least;
+            best_bin = 32 * h + __ffs(__ballot_sync(0xFFFFFFFFu, cost == least)) - 1;
+        }
     }
 }
 
@@ -230,19 +290,17 @@ __device__ __forceinline__ void bin_prim(const Ctx& c, uint32_t p, uint32_t* bin
     }
 }
 
-// Picks the split from the three axes' sweeps (lanes 0..2), the host's order: axis 0, 1, 2, strict less.
-__device__ void choose_split(const uint32_t* bins, int nb, float parent, const bool ok[3], float* rarea,
-                             uint32_t* rcnt, int lane, float& best_cost, int& best_axis, int& best_bin) {
-    float cost = INFINITY;
-    int bin = -1;
-    if (lane < 3 && ok[lane])
-        sah_axis(bins + 7 * lane * kMaxBins, nb, parent, rarea + lane * kMaxBins, rcnt + lane * kMaxBins, cost, bin);
+// Picks the split from the three axes' sweeps, the host's order: axis 0, 1, 2, strict less.
+__device__ void choose_split(const uint32_t* bins, int nb, float parent, const bool ok[3], int lane, float& best_cost,
+                             int& best_axis, int& best_bin) {
     best_cost = INFINITY;
     best_axis = -1;
     best_bin = -1;
     for (int k = 0; k < 3; ++k) {
-        const float ck = __shfl_sync(0xFFFFFFFFu, cost, k);
-        const int bk = __shfl_sync(0xFFFFFFFFu, bin, k);
+        if (!ok[k]) continue;   // the same for all lanes
+        float ck;
+        int bk;
+        sah_axis(bins + 7 * k * kMaxBins, nb, parent, lane, ck, bk);
         if (bk >= 0 && ck < best_cost) { best_cost = ck; best_axis = k; best_bin = bk; }
     }
 }
@@ -263,9 +321,8 @@ __device__ __forceinline__ bool goes_left(const Ctx& c, uint32_t p, uint32_t mod
     return median_key(c, p, axis) < pivot;
 }
 
-// Two children over [first, first + nl) and [first + nl, first + count); returns the left child.
-__device__ void alloc_children(const Ctx& c, uint32_t node, uint32_t first, uint32_t count, uint32_t nl) {
-    const uint32_t l = atomicAdd(&c.ctr[kCtrNodes], 2u);
+// Two children, l and l + 1, over [first, first + nl) and [first + nl, first + count).
+__device__ void set_children(const Ctx& c, uint32_t node, uint32_t first, uint32_t count, uint32_t nl, uint32_t l) {
     if (!checked(c, (uint64_t)l + 1u, c.max_nodes, 4) || !checked(c, node, c.max_nodes, 5)) return;
     BNodeD* L = c.nodes + l;
     L[0].first = first;
@@ -275,6 +332,9 @@ __device__ void alloc_children(const Ctx& c, uint32_t node, uint32_t first, uint
     L[1].count = count - nl;
     L[1].left = 0;
     c.nodes[node].left = l;
+}
+__device__ void alloc_children(const Ctx& c, uint32_t node, uint32_t first, uint32_t count, uint32_t nl) {
+    set_children(c, node, first, count, nl, atomicAdd(&c.ctr[kCtrNodes], 2u));
     if (nl > kSmall) atomicAdd(&c.ctr[kCtrNextLarge], 1u);
     if (count - nl > kSmall) atomicAdd(&c.ctr[kCtrNextLarge], 1u);
 }
@@ -287,8 +347,6 @@ __device__ __forceinline__ uint32_t lanemask_lt_() {
 
 struct WarpShared {
     uint32_t bins[3 * kMaxBins * 7];
-    float rarea[3 * kMaxBins];
-    uint32_t rcnt[3 * kMaxBins];
     unsigned long long pivot;
 };
 
@@ -339,21 +397,15 @@ __global__ void k_level_reset(uint32_t* ctr) {
     if (threadIdx.x == 0) ctr[kCtrLarge] = ctr[kCtrItems] = ctr[kCtrNextLarge] = 0u;
 }
 
-// One level of the binary build for the tasks of at most kSmall primitives (one warp each); larger tasks
-// are queued with their work items.
-__global__ void __launch_bounds__(kBT) k_level_small(Ctx c, uint32_t lb, uint32_t le, int depth) {
-    __shared__ WarpShared ws[kWarps];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t node = lb + blockIdx.x * kWarps + wid;
-    if (node >= le) return;
-    WarpShared& S = ws[wid];
+// One task of the level by one warp, or (more than kSmall primitives) its queueing.
+__device__ __noinline__ void small_task(const Ctx& c, WarpShared& S, uint32_t node, int lane, int depth) {
     if (!checked(c, node, c.max_nodes, 6)) return;
     const uint32_t first = c.nodes[node].first, count = c.nodes[node].count;
     if (!checked(c, (uint64_t)first + count, (uint64_t)c.n + 1u, 7)) return;
 
     if (count > kSmall) {
         uint32_t t = 0, i0 = 0;
-        const uint32_t nit = (count + kItem - 1) / kItem;
+        const uint32_t nit = (count + c.item - 1) / c.item;
         if (lane == 0) {
             t = atomicAdd(&c.ctr[kCtrLarge], 1u);
             i0 = atomicAdd(&c.ctr[kCtrItems], nit);
@@ -379,8 +431,8 @@ __global__ void __launch_bounds__(kBT) k_level_small(Ctx c, uint32_t lb, uint32_
         for (uint32_t j = lane; j < nit; j += 32) {
             Item& I = c.items[i0 + j];
             I.task = t;
-            I.begin = first + j * kItem;
-            I.count = min(kItem, count - j * kItem);
+            I.begin = first + j * c.item;
+            I.count = min(c.item, count - j * c.item);
         }
         init_bins(c.lbins + (size_t)t * 3 * kMaxBins * 7, c.bins, lane, 32);
         return;
@@ -412,7 +464,7 @@ __global__ void __launch_bounds__(kBT) k_level_small(Ctx c, uint32_t lb, uint32_
         const float parent = ha < 1e-30f ? 1e-30f : ha;
         float best_cost;
         int best_axis, best_bin;
-        choose_split(S.bins, c.bins, parent, ok, S.rarea, S.rcnt, lane, best_cost, best_axis, best_bin);
+        choose_split(S.bins, c.bins, parent, ok, lane, best_cost, best_axis, best_bin);
         if (count <= (uint32_t)kMaxLeafTris && sah::u2f(count) <= best_cost) mode = kModeLeaf;
         else if (best_axis < 0) mode = count <= (uint32_t)kMaxLeafTris ? kModeLeaf : kModeMedian;
         else {
@@ -480,6 +532,149 @@ __global__ void __launch_bounds__(kBT) k_level_small(Ctx c, uint32_t lb, uint32_
     if (lane == 0) alloc_children(c, node, first, count, nl);
 }
 
+// Tasks of at most kTiny primitives, four to a warp: the 8 lanes of group `lane / 8` hold one primitive each of
+// task `node` (has: the group has a task; count <= kTiny).  The decisions are those of the warp's path below:
+// a split's cost depends on the primitives left and right of a bin boundary, and of the boundaries with the
+// same sides the sweep keeps the first, which follows the bin of the last primitive on the left; so the
+// candidates are the primitives' own bins, and every lane prices the three splits after its own.  All 32
+// lanes call it together.
+__device__ void tiny_tasks(const Ctx& c, uint32_t node, uint32_t first, uint32_t count, bool has, int lane, int depth) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const int sub = lane & 7;
+    const uint32_t group = 0xFFu << (lane & 24);
+    const bool mine = has && (uint32_t)sub < count;
+    const uint32_t p = mine ? idx_at(c, (uint64_t)first + sub, 50) : 0u;
+    float pl[3] = {INFINITY, INFINITY, INFINITY}, ph[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (mine) load_box(c, p, pl, ph);
+    float ce[3], lo[3], hi[3], clo[3], chi[3];
+    for (int k = 0; k < 3; ++k) {
+        ce[k] = mine ? sah::centroid(pl[k], ph[k]) : 0.0f;
+        lo[k] = pl[k];
+        hi[k] = ph[k];
+        clo[k] = mine ? ce[k] : INFINITY;
+        chi[k] = mine ? ce[k] : -INFINITY;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(kAll, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kAll, hi[k], o));
+            clo[k] = fminf(clo[k], __shfl_xor_sync(kAll, clo[k], o));
+            chi[k] = fmaxf(chi[k], __shfl_xor_sync(kAll, chi[k], o));
+        }
+    }
+    if (has && sub == 0) {
+        BNodeD& N = c.nodes[node];
+        for (int k = 0; k < 3; ++k) { N.lo[k] = lo[k]; N.hi[k] = hi[k]; }
+        N.left = 0;
+    }
+    const bool sah_split = depth < c.median_depth;
+    float best = INFINITY;
+    int axis = -1, bin = -1, bk[3] = {0, 0, 0};
+    if (sah_split) {   // the same for the whole level
+        bool ok[3];
+        BinBox left[3], right[3];
+        for (int k = 0; k < 3; ++k) {
+            float sc = 0.0f;
+            ok[k] = sah::bin_scale(clo[k], chi[k], c.bins, sc);
+            bk[k] = mine && ok[k] ? sah::bin_of(ce[k], clo[k], sc, c.bins) : 0;
+            left[k] = right[k] = empty_bins();
+        }
+#pragma unroll
+        for (int j = 0; j < (int)kTiny; ++j) {
+            const int src = (lane & 24) + j;
+            const bool there = __shfl_sync(kAll, mine, src);
+            BinBox q;
+            for (int k = 0; k < 3; ++k) {
+                q.lo[k] = __shfl_sync(kAll, pl[k], src);
+                q.hi[k] = __shfl_sync(kAll, ph[k], src);
+            }
+            q.cnt = there ? 1u : 0u;
+            for (int k = 0; k < 3; ++k) {
+                const int b = __shfl_sync(kAll, bk[k], src);
+                if (b <= bk[k]) join(left[k], q);
+                else join(right[k], q);
+            }
+        }
+        const float ha = sah::half_area(lo, hi);
+        const float parent = ha < 1e-30f ? 1e-30f : ha;
+        for (int k = 0; k < 3; ++k) {
+            float cost = INFINITY;
+            if (mine && ok[k] && right[k].cnt != 0)
+                cost = sah::split_cost(sah::half_area(left[k].lo, left[k].hi), left[k].cnt,
+                                       sah::half_area(right[k].lo, right[k].hi), right[k].cnt, parent);
+            if (!(cost < INFINITY)) cost = INFINITY;
+            float least = cost;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(kAll, least, o));
+            int b = cost == least && cost < INFINITY ? bk[k] : 0x7FFFFFFF;   // the lowest bin of that cost
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) b = min(b, __shfl_xor_sync(kAll, b, o));
+            if (least < best) { best = least; axis = k; bin = b; }
+        }
+    }
+    const bool leaf = !has || count <= 1 ||
+                      (count <= (uint32_t)kMaxLeafTris && (!sah_split || axis < 0 || sah::u2f(count) <= best));
+    const bool median = !leaf && axis < 0;
+    bool goes = false;
+    if (!leaf && !median) goes = mine && (axis == 0 ? bk[0] : (axis == 1 ? bk[1] : bk[2])) <= bin;
+    if (__any_sync(kAll, median)) {   // the first count / 2 primitives by (centroid, id)
+        const int ma = median_axis(clo, chi);
+        const float cm = ma == 0 ? ce[0] : (ma == 1 ? ce[1] : ce[2]);
+        const unsigned long long key = ((unsigned long long)ord(sah::median_key(cm)) << 32) | p;
+        uint32_t rank = 0;
+#pragma unroll
+        for (int j = 0; j < (int)kTiny; ++j) {
+            const int src = (lane & 24) + j;
+            const unsigned long long kj = __shfl_sync(kAll, key, src);
+            const bool there = __shfl_sync(kAll, mine, src);
+            rank += there && kj < key ? 1u : 0u;
+        }
+        if (median) goes = mine && rank < count / 2;
+    }
+    const uint32_t bl = __ballot_sync(kAll, !leaf && mine && goes) & group, br = __ballot_sync(kAll, !leaf && mine && !goes) & group;
+    const uint32_t nl = (uint32_t)__popc(bl);
+    if (!leaf && mine) {
+        const uint64_t dst = goes ? first + __popc(bl & lanemask_lt_()) : first + nl + __popc(br & lanemask_lt_());
+        if (checked(c, dst, (uint64_t)first + count, 51)) c.idx[dst] = p;
+    }
+    // children: one allocation for the warp's tasks
+    const uint32_t split = __ballot_sync(kAll, !leaf && sub == 0);
+    if (!split) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&c.ctr[kCtrNodes], 2u * (uint32_t)__popc(split));
+    base = __shfl_sync(kAll, base, 0);
+    if (!leaf && sub == 0) set_children(c, node, first, count, nl, base + 2u * (uint32_t)__popc(split & lanemask_lt_()));
+}
+
+// One level of the binary build for the tasks of at most kSmall primitives; larger tasks are queued with their
+// work items.  FOUR: a warp takes four consecutive tasks, its 8-lane groups those of at most kTiny primitives
+// at once, then the warp the others one by one; otherwise a warp takes one task.  The launch picks FOUR once
+// a level's tasks hold at most 2 * kTiny primitives on average, which also leaves warps enough.
+template <bool FOUR>
+__global__ void __launch_bounds__(kBT) k_level_small(Ctx c, uint32_t lb, uint32_t le, int depth) {
+    __shared__ WarpShared ws[kWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t warp = blockIdx.x * kWarps + wid;
+    if (!FOUR) {
+        if (lb + warp < le) small_task(c, ws[wid], lb + warp, lane, depth);
+        return;
+    }
+    const uint32_t base = lb + 4u * warp;
+    if (base >= le) return;
+    const uint32_t node = base + (uint32_t)(lane >> 3);
+    uint32_t first = 0, count = 0;
+    if (node < le && checked(c, node, c.max_nodes, 52)) {
+        first = c.nodes[node].first;
+        count = c.nodes[node].count;
+    }
+    const bool tiny = node < le && count <= kTiny && checked(c, (uint64_t)first + count, (uint64_t)c.n + 1u, 53);
+    const uint32_t rest = __ballot_sync(0xFFFFFFFFu, node < le && count > kTiny && (lane & 7) == 0);
+    tiny_tasks(c, node, first, count, tiny, lane, depth);
+    for (uint32_t m = rest; m; m &= m - 1u) {
+        __syncwarp();
+        small_task(c, ws[wid], base + (uint32_t)(__ffs(m) - 1) / 8u, lane, depth);
+    }
+}
+
 __device__ __forceinline__ uint32_t global_warp() { return (blockIdx.x * kBT + threadIdx.x) >> 5; }
 
 // Large tasks: bounds of every work item into its task.
@@ -542,8 +737,7 @@ __global__ void __launch_bounds__(kBT) k_large_bins(Ctx c, int depth) {
 
 // Large tasks: the split decision (one warp per task).
 __global__ void __launch_bounds__(kBT) k_large_split(Ctx c, int depth) {
-    __shared__ WarpShared ws[kWarps];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const uint32_t t = global_warp();
     if (t >= min(c.ctr[kCtrLarge], c.max_large)) return;
     LargeTask& T = c.large[t];
@@ -566,8 +760,7 @@ __global__ void __launch_bounds__(kBT) k_large_split(Ctx c, int depth) {
         const float parent = ha < 1e-30f ? 1e-30f : ha;
         float best_cost;
         int best_axis, best_bin;
-        choose_split(c.lbins + (size_t)t * 3 * kMaxBins * 7, c.bins, parent, ok, ws[wid].rarea, ws[wid].rcnt, lane,
-                     best_cost, best_axis, best_bin);
+        choose_split(c.lbins + (size_t)t * 3 * kMaxBins * 7, c.bins, parent, ok, lane, best_cost, best_axis, best_bin);
         if (best_axis >= 0) {
             mode = kModeSplit;
             axis = best_axis;
@@ -1005,7 +1198,8 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
 
     const uint32_t max_nodes = 2u * n;
     const uint32_t max_large = n / kSmall + 2;
-    const uint32_t max_items = n / kItem + max_large + 2;
+    const uint32_t item = item_size(n);
+    const uint32_t max_items = n / item + max_large + 2;
     DeviceBuffer d_verts(9ull * n * sizeof(float)), d_plo(16ull * n), d_phi(16ull * n), d_idx(4ull * n), d_tmp(4ull * n),
         d_nodes((size_t)max_nodes * sizeof(BNodeD)), d_ctr(kCtrWords * sizeof(uint32_t)),
         d_large((size_t)max_large * sizeof(LargeTask)), d_items((size_t)max_items * sizeof(Item)),
@@ -1036,6 +1230,7 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     c.max_items = max_items;
     c.max_nodes = max_nodes;
     c.n = n;
+    c.item = item;
     c.bins = bins;
     c.median_depth = opt.median_depth;
 
@@ -1058,9 +1253,12 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     uint32_t lb = 0, le = 1, n_large = n > kSmall ? 1u : 0u;
     for (int depth = 0; lb < le; ++depth) {
         k_level_reset<<<1, 32, 0, st>>>(ctr);
-        k_level_small<<<blocks_for(le - lb, kWarps), kBT, 0, st>>>(c, lb, le, depth);
+        if ((uint64_t)n <= (uint64_t)(le - lb) * 2u * kTiny)
+            k_level_small<true><<<blocks_for(le - lb, 4 * kWarps), kBT, 0, st>>>(c, lb, le, depth);
+        else
+            k_level_small<false><<<blocks_for(le - lb, kWarps), kBT, 0, st>>>(c, lb, le, depth);
         if (n_large > 0) {
-            const uint32_t item_blocks = blocks_for(std::min<uint64_t>(max_items, (uint64_t)n / kItem + n_large + 1), kWarps);
+            const uint32_t item_blocks = blocks_for(std::min<uint64_t>(max_items, (uint64_t)n / item + n_large + 1), kWarps);
             const uint32_t task_blocks = blocks_for(n_large, kWarps);
             k_large_bounds<<<item_blocks, kBT, 0, st>>>(c);
             k_large_bins<<<item_blocks, kBT, 0, st>>>(c, depth);
