@@ -68,12 +68,11 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  * whose traversal and scheduling belong to the Vulkan implementation).  Every setting gives the same results; only speed
  * differs.  0 selects the default of a field.
  *   refill: the traversal launch form.  1..32 (0 = the default, 8): the warp-cooperative persistent form
- *            (flat scenes; block 128, stack 12): warps keep 32 rays in flight, take new rays once `refill`
- *            of their lanes are idle, and share each step's triangle tests and the finished rays' hit
- *            refinement over all 32 lanes; REINA_REFILL_GRID: one thread per ray (the grid form, the
- *            only form of two-level scenes, which use it whatever this field says).  On the
- *            1.3M-triangle ray cast (2,097,152 rays) closest hit 0.58 ms cooperative against 0.82 ms
- *            grid, any hit 0.36 against 0.51 ms.  Ray casts only: the wavefront kernels of frames and
+ *            (block 128): warps keep 32 rays in flight, take new rays once `refill` of their lanes are idle,
+ *            and share each step's triangle tests and the finished rays' hit refinement over all 32 lanes;
+ *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
+ *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
+ *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and
  *            batches take wave_refill, whose default is the grid form (a 1920x1080 64-spp frame of that
  *            scene 318 ms grid against 352 ms cooperative, a 256x256 Cornell room 2.48 against 3.79 ms).
  *   trace_block: threads per block of the grid-form traversal kernels (ray cast, wavefront extend and

@@ -134,22 +134,20 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) kb_extend(BatchLaunch B, 
 // Cooperative persistent form of the extension kernel (coop_trace.cuh; waves of flat scenes): warps
 // refill idle lanes from the active queue once at most `refill_at` lanes still trace; each lane's ray
 // uses its own job's scene.
-__global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) kb_extend_coop(BatchLaunch B, const JobGpu* __restrict__ jobs, int cur,
+__global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) kb_extend_coop(const __grid_constant__ BatchLaunch B, const JobGpu* __restrict__ jobs, int cur,
                                                              uint32_t refill_at) {
-    __shared__ CoopWarp warps[kTraceBlock / 32];
-    __shared__ uint2 stack[kSmemStack * kTraceBlock];
     const PathState& ps = B.bp.ps;
     const uint32_t n = ps.counters[kCntActive + cur];
     const uint32_t* q = ps.q_active[cur];
     TraceCounters c{0u, 0u};
-    auto load = [&](uint32_t i, TraceRay& r, CoopScene& sc) {
+    auto load = [&](uint32_t i, float4& o, float4& d) {
         const uint32_t p = checked_index(q[i], B.P, ps.counters + kCntError);
-        const DeviceScene& s = jobs[B.bp.job[p]].s;
-        r = make_trace_ray(ps.ox[p], ps.oy[p], ps.oz[p], ps.dx[p], ps.dy[p], ps.dz[p], 0.0f, 10000.0f);
-        sc = CoopScene{s.nodes, s.tris, s.node_count};
-        return true;
+        o = make_float4(ps.ox[p], ps.oy[p], ps.oz[p], 0.0f);
+        d = make_float4(ps.dx[p], ps.dy[p], ps.dz[p], 10000.0f);
+        return &jobs[B.bp.job[p]].s;
     };
-    auto store = [&](uint32_t i, const Hit& h, bool valid) {   // called by all 32 lanes
+    auto store = [&](uint32_t i, const CoopHit& c, bool valid) {   // called by all 32 lanes
+        const Hit& h = c.h;
         int m = -1;
         uint32_t p = 0;
         if (valid) {
@@ -169,10 +167,8 @@ __global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) kb_extend_coop(Ba
             if (mine) ps.q_shade[(size_t)k * B.P + checked_index(pos, B.P, ps.counters + kCntError)] = p;
         }
     };
-    const uint32_t e = coop_trace<false, true, true, true, kSmemStack>(CoopScene{nullptr, nullptr, 0u}, n,
-                                                                       ps.counters + kCntFetchExtend, refill_at,
-                                                                 warps[threadIdx.x >> 5], stack + threadIdx.x,
-                                                                 kTraceBlock, load, store, c);
+    const uint32_t e = coop_trace<false, true, true, true, false>(DeviceScene{}, n, ps.counters + kCntFetchExtend, refill_at,
+                                                                  load, store, c);
     if (e) atomicOr(ps.counters + kCntError, e);
     coop_add_counts(c, ps.counters, kCntNodes, kCntTris);
 }
@@ -297,31 +293,26 @@ __global__ void __launch_bounds__(BLOCK) kb_shadow(BatchLaunch B, const JobGpu* 
 }
 
 // Cooperative persistent form of the shadow kernel (waves of flat scenes).
-__global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) kb_shadow_coop(BatchLaunch B, const JobGpu* __restrict__ jobs,
+__global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) kb_shadow_coop(const __grid_constant__ BatchLaunch B, const JobGpu* __restrict__ jobs,
                                                              uint32_t refill_at) {
-    __shared__ CoopWarp warps[kTraceBlock / 32];
-    __shared__ uint2 stack[kSmemStack * kTraceBlock];
     const PathState& ps = B.bp.ps;
     const uint32_t n = ps.counters[kCntShadow];
     TraceCounters c{0u, 0u};
-    auto load = [&](uint32_t i, TraceRay& r, CoopScene& sc) {
+    auto load = [&](uint32_t i, float4& o, float4& d) {
         const uint32_t p = checked_index(ps.q_shadow[i], B.P, ps.counters + kCntError);
-        const DeviceScene& s = jobs[B.bp.job[p]].s;
-        r = make_trace_ray(ps.s_ox[i], ps.s_oy[i], ps.s_oz[i], ps.s_dx[i], ps.s_dy[i], ps.s_dz[i], 0.0f, ps.s_tmax[i]);
-        sc = CoopScene{s.nodes, s.tris, s.node_count};
-        return true;
+        o = make_float4(ps.s_ox[i], ps.s_oy[i], ps.s_oz[i], 0.0f);
+        d = make_float4(ps.s_dx[i], ps.s_dy[i], ps.s_dz[i], ps.s_tmax[i]);
+        return &jobs[B.bp.job[p]].s;
     };
-    auto store = [&](uint32_t i, const Hit& h, bool valid) {   // called by all 32 lanes
-        if (valid && h.prim == kMiss) {
+    auto store = [&](uint32_t i, const CoopHit& c, bool valid) {   // called by all 32 lanes
+        if (valid && c.h.prim == kMiss) {
             const uint32_t p = checked_index(ps.q_shadow[i], B.P, ps.counters + kCntError);
             store_rad(ps, p, load_rad(ps, p) + V3{ps.s_cr[i], ps.s_cg[i], ps.s_cb[i]});
         }
         warp_count64(reinterpret_cast<unsigned long long*>(ps.counters + kCntShadowRays), valid);
     };
-    const uint32_t e = coop_trace<true, true, false, true, kSmemStack>(CoopScene{nullptr, nullptr, 0u}, n,
-                                                                       ps.counters + kCntFetchShadow, refill_at,
-                                                                 warps[threadIdx.x >> 5], stack + threadIdx.x,
-                                                                 kTraceBlock, load, store, c);
+    const uint32_t e = coop_trace<true, true, false, true, false>(DeviceScene{}, n, ps.counters + kCntFetchShadow, refill_at,
+                                                                  load, store, c);
     if (e) atomicOr(ps.counters + kCntError, e);
     coop_add_counts(c, ps.counters, kCntShadowNodes, kCntShadowTris);
 }
@@ -440,8 +431,8 @@ BatchEngine::BatchEngine(int device, int sm_count, uint32_t wave_capacity, bool 
         throw;
     }
     if (trace_.refill > 0) {
-        blocks_ext_ = resident_grid((const void*)kb_extend_coop, kTraceBlock, sm_count);
-        blocks_sh_ = resident_grid((const void*)kb_shadow_coop, kTraceBlock, sm_count);
+        blocks_ext_ = resident_grid((const void*)kb_extend_coop, kTraceBlock, sm_count, coop_shared_bytes<true, false>());
+        blocks_sh_ = resident_grid((const void*)kb_shadow_coop, kTraceBlock, sm_count, coop_shared_bytes<true, false>());
     } else {
         with_trace_variant(trace_, [&](auto B, auto S) {
             blocks_ext_ = resident_grid((const void*)kb_extend<B.value, S.value, false>, B.value, sm_count);
@@ -546,7 +537,7 @@ void BatchEngine::launch_body(Lane& L, const Packed& pk, cudaStream_t st) {
             else if (two)   // a two-level scene in the wave: the default grid variant, both traversals
                 kb_extend<kTraceBlock, kDefaultTraceStack, true><<<blocks_ext_two_, kTraceBlock, 0, s>>>(B, B.jobs, cur);
             else if (trace_.refill > 0)
-                kb_extend_coop<<<blocks_ext_, kTraceBlock, 0, s>>>(B, B.jobs, cur, (uint32_t)(32 - trace_.refill));
+                kb_extend_coop<<<blocks_ext_, kTraceBlock, coop_shared_bytes<true, false>(), s>>>(B, B.jobs, cur, (uint32_t)(32 - trace_.refill));
             else if (count)
                 kb_extend<kTraceBlock, kDefaultTraceStack, false, true><<<blocks_ext_cnt_, kTraceBlock, 0, s>>>(B, B.jobs, cur);
             else
@@ -563,7 +554,7 @@ void BatchEngine::launch_body(Lane& L, const Packed& pk, cudaStream_t st) {
             else if (any_nee && two)
                 kb_shadow<kTraceBlock, kDefaultTraceStack, true><<<blocks_sh_two_, kTraceBlock, 0, s>>>(B, B.jobs);
             else if (any_nee && trace_.refill > 0)
-                kb_shadow_coop<<<blocks_sh_, kTraceBlock, 0, s>>>(B, B.jobs, (uint32_t)(32 - trace_.refill));
+                kb_shadow_coop<<<blocks_sh_, kTraceBlock, coop_shared_bytes<true, false>(), s>>>(B, B.jobs, (uint32_t)(32 - trace_.refill));
             else if (any_nee && count)
                 kb_shadow<kTraceBlock, kDefaultTraceStack, false, true><<<blocks_sh_cnt_, kTraceBlock, 0, s>>>(B, B.jobs);
             else if (any_nee)

@@ -1,20 +1,21 @@
-// Warp-cooperative persistent BVH8 traversal: the default launch form for flat scenes.
+// Warp-cooperative persistent BVH8 traversal, of flat and of two-level scenes: the default launch form.
 //
 // The per-thread traversal of trace_device.cuh loses most of a warp's issue slots to divergence on
 // incoherent rays: lanes whose rays have ended wait for the warp's longest ray, and the triangle tests
 // run with the few lanes whose node had leaf children.  Here a warp keeps 32 rays in flight and shares
 // the work that diverges:
-//   * refill (Aila and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): when at
-//     most `refill_at` lanes still trace, the idle lanes take the next rays from a warp-private chunk of
-//     the global fetch counter;
-//   * node visits: every tracing lane visits its nearest pending child node (the step of trace_device.cuh:
-//     box test of the 8 quantized children, near-to-far order by ray octant), kCoopVisits times between
-//     two rounds of the warp's bookkeeping (refill, list tests, finishing), so that the bookkeeping is
-//     paid once per several visits;
-//   * triangle tests: a node's leaf triangles are not tested by the lane that found them; the warp
-//     collects (ray, triangle group) pairs in a shared list and, once it holds kFlushTris triangles (or a
-//     lane with groups in the list has no nodes left), tests them with one (ray, triangle) pair per lane,
-//     the closest (t, prim) per ray kept by a 64-bit atomic minimum in shared memory;
+//   * rays are fetched 32 at a time (a chunk of the global fetch counter, one ray per lane, into shared
+//     memory), and idle lanes take the next staged ray once at most `refill_at` lanes still trace (refill: Aila
+//     and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009);
+//   * node visits: every tracing lane visits its nearest pending child node (box test of the 8 quantized
+//     children, near-to-far order by ray octant), VISITS times between two rounds of the warp's bookkeeping
+//     (refill, list tests, finishing), so that the bookkeeping is paid once per several visits;
+//   * triangle tests: a node's leaf triangles are not tested by the lane that found them; the warp collects
+//     them in a shared list, a group per node, and once it holds kFlushGroups groups (or a lane with groups in it
+//     has nothing else to do) tests them with one (ray, triangle) pair per lane, the closest (t, prim) per ray
+//     kept by a 64-bit atomic minimum in shared memory;
+//   * instances (TWO): a lane that reaches a top-level leaf enters its instances one after the other; the
+//     lanes that want to enter one do it together, once per round, and the world ray waits in shared memory;
 //   * finishing: ended rays go to a shared list that the warp refines (refine_hit) and stores one per
 //     lane once it is full, so the hit refinement also runs at full width.
 // The closest hit is the lowest (t, prim) over the triangles hit in [tmin, tmax], as in every other form,
@@ -23,52 +24,89 @@
 
 #include <stdint.h>
 
+#include <type_traits>
+
+#include "kernels.h"
 #include "trace_device.cuh"
 
 namespace rt {
 
-// Per-warp shared state of the cooperative traversal.
-struct CoopWarp {
-    float4 ray_a[32];                 // per lane: origin, tmin of its ray (for the triangle tests)
-    float4 ray_b[32];                 // per lane: shear constants sx, sy, sz, axes kx | ky << 2 | kz << 4
-    unsigned long long best[32];      // per lane: ordered(t) << 32 | prim of the closest hit so far
-    float4 best_hit[32];              // per lane: triangle record (bits), t, u, v of that hit
-    const float4* tris[32];           // per lane: triangle records of its ray's scene
-    uint32_t gbase[64];               // triangle groups: first triangle record
-    uint32_t gmo[64];                 // triangle groups: owner lane << 24 | triangle hit mask
-    uint32_t gprefix[64];             // inclusive prefix of the groups' triangle counts
-    float4 fin_o[32];                 // finished rays: origin, t
-    float4 fin_d[32];                 // finished rays: direction, u
-    uint4 fin_i[32];                  // finished rays: item, prim, triangle record, v (bits)
-    const float4* fin_tris[32];       // finished rays: triangle records of their scene
-};
-
-// Scene of one item (per lane: batched waves mix scenes).
-struct CoopScene {
-    const Bvh8Node* nodes;
-    const TriRecord* tris;
-    uint32_t node_count;
-};
-
-// Items per warp-private fetch chunk.  Small chunks interleave the warps over the item list, so the last
-// items end together (1.3M-triangle ray cast: chunks of 32 0.568 ms, 128 0.656 ms, 512 0.822 ms).
+// Items per fetch: one per lane.  Small chunks also interleave the warps over the item list, so the last
+// items end together.
 constexpr uint32_t kCoopChunk = 32;
-// Blocks of 128 threads per SM the cooperative kernels are compiled for: 7 (at most 72 registers; 30 KB of
-// shared memory each, 210 KB per SM).
+// Blocks of 128 threads per SM the cooperative kernels are compiled for: 7 (at most 72 registers, 30.4 KB of shared
+// memory each): 0.418 ms against 0.423 ms with 6 and 0.444 ms with 8 (and a 6-entry stack).
 #ifndef RT_COOP_MINB
 #define RT_COOP_MINB 7
 #endif
 constexpr int kCoopMinBlocks = RT_COOP_MINB;
-#ifndef RT_COOP_FLUSH_TRIS
-#define RT_COOP_FLUSH_TRIS 24
+// Blocks per SM of the two-level form, which keeps more state (5 blocks: 5 % slower; 7: the same, with spills).
+#ifndef RT_COOP_MINB_TWO
+#define RT_COOP_MINB_TWO 6
 #endif
-constexpr uint32_t kFlushTris = RT_COOP_FLUSH_TRIS;   // triangles collected before the warp tests them
-// Node visits per lane per round of bookkeeping (1.3M-triangle ray cast, closest hit: 1 visit 0.539 ms,
-// 2 visits 0.505 ms with 0.7 % more node visits, 3 visits 0.556 ms, 4 visits 0.620 ms).
+constexpr int kCoopMinBlocksTwo = RT_COOP_MINB_TWO;
+#ifndef RT_COOP_FLUSH
+#define RT_COOP_FLUSH 12
+#endif
+constexpr uint32_t kFlushGroups = RT_COOP_FLUSH;   // groups (two triangles on average) collected before the test
+// Node visits per lane per round of bookkeeping (1.3M-triangle ray cast, closest hit: 1 visit 0.436 ms, 2 visits
+// 0.418 ms, 3 visits 0.420 ms; 256 instances: 0.952, 0.930 and 1.127 ms).
 #ifndef RT_COOP_VISITS
 #define RT_COOP_VISITS 2
 #endif
 constexpr int kCoopVisits = RT_COOP_VISITS;
+// Shared-memory stack entries per thread (deeper levels spill to local memory): what fits beside the lists.
+#ifndef RT_COOP_STACK
+#define RT_COOP_STACK 8
+#endif
+constexpr int kCoopStack = RT_COOP_STACK;
+constexpr uint32_t kCoopGroups = 64;   // list capacity: a visit adds at most 32, and a flush comes before the next
+
+// Per-warp shared state of the cooperative traversal.
+struct CoopWarpFlat {
+    float4 ray_o[32];                 // per lane: origin, tmin of its ray (in its instance's space while in one)
+    float4 ray_s[32];                 // per lane: shear constants sx, sy, sz, axes kx | ky << 2 | kz << 4
+    float4 ray_d[32];                 // per lane: direction, tmax (world space)
+    unsigned long long best[32];      // per lane: ordered(t) << 32 | prim of the closest hit so far
+    uint2 best_rec[32];               // per lane: triangle record and t (as tested) of that hit
+    uint32_t g_base[kCoopGroups];     // groups: first triangle record of the node
+    uint32_t g_meta[2][kCoopGroups];  // groups: meta bytes of the hit leaf children, by child slot
+    uint16_t g_prefix[kCoopGroups];   // groups: inclusive prefix of their triangle counts
+    uint8_t g_own[kCoopGroups];       // groups: lane of the ray
+    float4 fin_o[32];                 // finished rays: origin, t
+    float4 fin_d[32];                 // finished rays: direction
+    uint4 fin_i[32];                  // finished rays: item, prim, triangle record, instance
+    float4 stage_o[32], stage_d[32];  // fetched rays: origin, tmin; direction, tmax
+};
+struct CoopWarpTwo {
+    float4 world_o[32];               // per lane: origin, tmin in world space
+    uint32_t inst[32];                // per lane: instance its ray is in
+    uint32_t best_inst[32];           // per lane: instance of the closest hit
+    uint32_t first[32];               // per lane: first global triangle of that instance
+};
+struct CoopWarpMixed {
+    const DeviceScene* scene[32];     // per lane: its ray's scene
+    const DeviceScene* fin_scene[32]; // finished rays: their scene
+    const DeviceScene* stage_scene[32];
+};
+struct CoopNotTwo {};
+struct CoopNotMixed {};
+template <bool MIXED, bool TWO>
+struct CoopWarp : CoopWarpFlat,
+                  std::conditional_t<TWO, CoopWarpTwo, CoopNotTwo>,
+                  std::conditional_t<MIXED, CoopWarpMixed, CoopNotMixed> {};
+
+// The cooperative kernels' dynamic shared memory: a CoopWarp per warp, then the threads' stacks.  The functions
+// below reach it through this symbol, so that they access it as shared memory also where they are not inlined.
+extern __shared__ __align__(16) unsigned char coop_shared[];
+template <bool MIXED, bool TWO>
+__device__ __forceinline__ CoopWarp<MIXED, TWO>& coop_warp() {
+    return reinterpret_cast<CoopWarp<MIXED, TWO>*>(coop_shared)[threadIdx.x >> 5];
+}
+template <bool MIXED, bool TWO>
+constexpr size_t coop_shared_bytes() {
+    return (kTraceBlock / 32) * sizeof(CoopWarp<MIXED, TWO>) + kTraceBlock * kCoopStack * sizeof(uint2);
+}
 
 __device__ __forceinline__ uint32_t coop_ordered(float f) {
     const uint32_t b = __float_as_uint(f);
@@ -96,207 +134,270 @@ __device__ __forceinline__ void coop_add_counts(const TraceCounters& c, uint32_t
     }
 }
 
-// Tests the collected triangle groups, one (ray, triangle) pair per lane per round.  MIXED: each lane's ray
-// has its own scene (S.tris); otherwise every ray uses `tris`.  Not inlined, like coop_store_finished: both
-// run once per several traversal steps, and kept out of the traversal loop they leave it more registers
-// (1.3M-triangle ray cast: 0.566 -> 0.534 ms, the loop's register copies moved off the ALU pipe).
-template <bool COUNT, bool MIXED>
-__device__ __noinline__ void coop_test_groups(CoopWarp& S, uint32_t lane, uint32_t n_groups, const float4* tris,
-                                                 TraceCounters& cnt) {
-    const uint32_t c0 = lane < n_groups ? __popc(S.gmo[lane] & 0x00FFFFFFu) : 0u;
-    const uint32_t c1 = lane + 32u < n_groups ? __popc(S.gmo[lane + 32u] & 0x00FFFFFFu) : 0u;
-    uint32_t i0 = c0, i1 = c1;
+// What a finished ray hands to its caller: the hit, its instance (two-level scenes) and the words that the
+// triangle record carries beside its vertices (flat scenes; see TriRecord).
+struct CoopHit {
+    Hit h;
+    uint32_t inst;
+    uint32_t pad1, pad2;
+};
+
+// Tests the n collected groups, one (ray, triangle) pair per lane per round.  Not inlined, like
+// coop_store_finished: both run once per several traversal steps, and kept out of the traversal loop they leave
+// it more registers (1.3M-triangle ray cast: 0.566 -> 0.534 ms when they moved out).
+template <bool COUNT, bool MIXED, bool TWO>
+__device__ __noinline__ uint32_t coop_test_groups(uint32_t n, const float4* tris) {
+    CoopWarp<MIXED, TWO>& S = coop_warp<MIXED, TWO>();
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t total = 0, tested = 0;
+    for (uint32_t h = 0; h < n; h += 32u) {
+        const uint32_t g = h + lane;
+        uint32_t c = g < n ? __popc(leaf_bits(S.g_meta[0][g])) + __popc(leaf_bits(S.g_meta[1][g])) : 0u;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y0 = __shfl_up_sync(0xFFFFFFFFu, i0, o);
-        const uint32_t y1 = __shfl_up_sync(0xFFFFFFFFu, i1, o);
-        if (lane >= (uint32_t)o) { i0 += y0; i1 += y1; }
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, c, o);
+            if (lane >= (uint32_t)o) c += y;
+        }
+        c += total;
+        if (g < n) S.g_prefix[g] = (uint16_t)c;
+        total = __shfl_sync(0xFFFFFFFFu, c, 31);
     }
-    const uint32_t t0 = __shfl_sync(0xFFFFFFFFu, i0, 31);
-    const uint32_t total = t0 + __shfl_sync(0xFFFFFFFFu, i1, 31);
-    S.gprefix[lane] = i0;
-    S.gprefix[lane + 32u] = i1 + t0;
     __syncwarp();
     for (uint32_t b0 = 0; b0 < total; b0 += 32u) {
         const uint32_t p = b0 + lane;
         bool hit = false;
         uint32_t o = 0, rec = 0;
         unsigned long long key = 0;
-        float t = 0.0f, u = 0.0f, v = 0.0f;
+        float t = 0.0f;
         if (p < total) {
             uint32_t g = 0;   // the group holding pair p: binary search over the prefix
+            if (n > 32u && S.g_prefix[31] <= p) g = 32u;
 #pragma unroll
-            for (uint32_t s = 32; s; s >>= 1)
-                if (g + s - 1 < n_groups && S.gprefix[g + s - 1] <= p) g += s;
-            const uint32_t k = p - (g ? S.gprefix[g - 1] : 0u);
-            const uint32_t mo = S.gmo[g];
-            o = mo >> 24;
-            rec = S.gbase[g] + (uint32_t)__fns(mo & 0x00FFFFFFu, 0u, (int)k + 1);
-            const float4* tp = (MIXED ? S.tris[o] : tris) + 3ull * rec;
+            for (uint32_t s = 16; s; s >>= 1)
+                if (g + s - 1 < n && S.g_prefix[g + s - 1] <= p) g += s;
+            uint32_t k = p - (g ? S.g_prefix[g - 1] : 0u);   // the k-th triangle of the group
+            uint32_t m = S.g_meta[0][g];
+            uint32_t bits = leaf_bits(m);
+            const uint32_t c0 = (uint32_t)__popc(bits);
+            if (k >= c0) {
+                k -= c0;
+                m = S.g_meta[1][g];
+                bits = leaf_bits(m);
+            }
+            for (; k; --k) bits &= bits - 1u;
+            const uint32_t at = (uint32_t)__ffs(bits) - 1u;   // bit of the triangle within its child's byte
+            rec = S.g_base[g] + ((m >> (at & 24u)) & 31u) + (at & 7u);
+            o = S.g_own[g];
+            const float4* tp = tris;
+            if constexpr (MIXED) tp = reinterpret_cast<const float4*>(S.scene[o]->tris);
+            tp += 3ull * rec;
             const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-            const float4 ra = S.ray_a[o], rb = S.ray_b[o];
+            const float4 ra = S.ray_o[o], rb = S.ray_s[o];
             TraceRay q;
             q.ox = ra.x; q.oy = ra.y; q.oz = ra.z; q.tmin = ra.w;
             q.sx = rb.x; q.sy = rb.y; q.sz = rb.z;
             const uint32_t kk = __float_as_uint(rb.w);
             q.kx = (int)(kk & 3u); q.ky = (int)((kk >> 2) & 3u); q.kz = (int)((kk >> 4) & 3u);
-            if (COUNT) cnt.tris++;
+            if (COUNT) ++tested;
+            float u, v;
             if (intersect_triangle(q, a, b, c, coop_unordered((uint32_t)(S.best[o] >> 32)), t, u, v)) {
                 hit = true;
-                key = ((unsigned long long)coop_ordered(t + 0.0f) << 32) | __float_as_uint(a.w);
+                uint32_t prim = __float_as_uint(a.w);
+                if constexpr (TWO) prim += S.first[o];
+                key = ((unsigned long long)coop_ordered(t + 0.0f) << 32) | prim;
                 atomicMin(&S.best[o], key);
             }
         }
         __syncwarp();
-        if (hit && S.best[o] == key) S.best_hit[o] = make_float4(__uint_as_float(rec), t, u, v);
+        if (hit && S.best[o] == key) {
+            S.best_rec[o] = make_uint2(rec, __float_as_uint(t));
+            if constexpr (TWO) S.best_inst[o] = S.inst[o];
+        }
         __syncwarp();
     }
+    return tested;
 }
 
 // Refines (REFINE) and stores the finished rays of the list, one per lane; store is called by all lanes.
-template <bool REFINE, bool MIXED, class Store>
-__device__ __noinline__ void coop_store_finished(CoopWarp& S, uint32_t lane, uint32_t n_fin, const float4* tris,
-                                                    Store& store) {
+template <bool REFINE, bool MIXED, bool TWO, class Store>
+__device__ __noinline__ void coop_store_finished(uint32_t n_fin, const DeviceScene& uniform, Store& store) {
+    CoopWarp<MIXED, TWO>& S = coop_warp<MIXED, TWO>();
+    const uint32_t lane = threadIdx.x & 31u;
     __syncwarp();
     const bool valid = lane < n_fin;
-    Hit h;
-    h.prim = kMiss; h.t = 0.0f; h.u = 0.0f; h.v = 0.0f;
+    CoopHit c;
+    c.h.prim = kMiss; c.h.t = 0.0f; c.h.u = 0.0f; c.h.v = 0.0f;
+    c.inst = 0; c.pad1 = 0; c.pad2 = 0;
     uint32_t item = 0;
     if (valid) {
         const float4 o = S.fin_o[lane], d = S.fin_d[lane];
         const uint4 fi = S.fin_i[lane];
         item = fi.x;
-        h.prim = fi.y;
-        h.t = o.w;
-        h.u = d.w;
-        h.v = __uint_as_float(fi.w);
-        if (REFINE && h.prim != kMiss) {
+        c.h.prim = fi.y;
+        c.h.t = o.w;
+        c.inst = fi.w;
+        if (REFINE && c.h.prim != kMiss) {
+            const DeviceScene* sc = &uniform;
+            if constexpr (MIXED) sc = S.fin_scene[lane];
+            const float4* tp = reinterpret_cast<const float4*>(sc->tris) + 3ull * fi.z;
+            const float4 a = __ldg(tp), b = __ldg(tp + 1), v = __ldg(tp + 2);
             TraceRay r;
             r.ox = o.x; r.oy = o.y; r.oz = o.z;
             r.dx = d.x; r.dy = d.y; r.dz = d.z;
-            const float4* tp = (MIXED ? S.fin_tris[lane] : tris) + 3ull * fi.z;
-            refine_hit(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), h);
+            r.tmin = 0.0f; r.tmax = 0.0f;
+            if (TWO && sc->inst_trav) r = instance_ray(r, sc->inst_trav + fi.w);
+            if (!refine_hit(r, a, b, v, c.h)) {   // the test's own t, u, v stand (a degenerate determinant)
+                TraceRay q = make_trace_ray(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, -INFINITY, INFINITY);
+                intersect_triangle(q, a, b, v, INFINITY, c.h.t, c.h.u, c.h.v);
+            }
+            c.pad1 = __float_as_uint(b.w);
+            c.pad2 = __float_as_uint(v.w);
         }
     }
     __syncwarp();
-    store(item, h, valid);
+    store(item, c, valid);
 }
 
-// Traces items [0, n) of the caller's list: load(i, ray, scene) -> false if item i has no ray to trace (it
-// is stored as a miss with t = its tmax); with MIXED, load also names the item's scene (batched waves mix
-// scenes), otherwise every item uses `uniform`; store(i, hit, valid) is called by all 32 lanes together with
-// up to 32 finished items (valid marks the lanes holding one).  `next` is the global fetch counter (zero
-// at launch); a warp refills its idle lanes once at most `refill_at` lanes still trace.  Requires
-// blockDim.x to be a multiple of 32; `stack` points at this thread's first shared stack entry, entries
-// `stride` apart.  Returns the device error bits of the warp's rays.
-// CHUNK, FLUSH: the fetch chunk and the triangle flush size; VISITS: node visits per lane between two
-// rounds of the warp's bookkeeping (the triangles found meanwhile are tested at the next flush, so the
-// closest distance a visit culls with may lag by up to VISITS - 1 visits: a few more nodes, same hits).
-template <bool ANY, bool COUNT, bool REFINE, bool MIXED, int SS, uint32_t CHUNK = kCoopChunk, uint32_t FLUSH = kFlushTris,
+// Traces items [0, n) of the caller's list.  load(i, o, d) gives item i's ray (origin and tmin, direction and
+// tmax); with MIXED it also returns the item's scene (batched waves mix scenes), otherwise every item uses
+// `uniform`.  store(i, hit, valid) is called by all 32 lanes together with up to 32 finished items (valid
+// marks the lanes holding one).  `next` is the global fetch counter (zero at launch); a warp refills its idle
+// lanes once at most `refill_at` lanes still trace.  Requires blocks of kTraceBlock threads and
+// coop_shared_bytes() of dynamic shared memory.  Returns the device error bits of the warp's rays.  TWO: scenes may be two-level.  VISITS: node visits per lane between two rounds of the
+// warp's bookkeeping (the triangles found meanwhile are tested at the next flush, so the closest distance a
+// visit culls with may lag by up to VISITS - 1 visits: a few more nodes, same hits).
+template <bool ANY, bool COUNT, bool REFINE, bool MIXED, bool TWO, int SS = kCoopStack, uint32_t FLUSH = kFlushGroups,
           int VISITS = kCoopVisits, class Load, class Store>
-__device__ __forceinline__ uint32_t coop_trace(const CoopScene& uniform, uint32_t n, uint32_t* next, uint32_t refill_at,
-                                               CoopWarp& S, uint2* stack, int stride, Load load, Store store,
-                                               TraceCounters& cnt) {
+__device__ __forceinline__ uint32_t coop_trace(const DeviceScene& uniform, uint32_t n, uint32_t* next, uint32_t refill_at,
+                                               Load load, Store store, TraceCounters& cnt) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    constexpr int stride = kTraceBlock;
+    CoopWarp<MIXED, TWO>& S = coop_warp<MIXED, TWO>();
+    uint2* stack = reinterpret_cast<uint2*>(coop_shared + (kTraceBlock / 32) * sizeof(CoopWarp<MIXED, TWO>)) + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     uint2 spill[kTotalStack - SS];
     uint32_t err = 0;
     bool has = false;
-    TraceRay r;
-    CoopScene sc = uniform;
+    TraceRay r;                                     // origin, reciprocal direction, tmin, octant: the box test's part
+    uint32_t wlo = 0, whi = 0;                      // octant_weights of the ray
+    const uint4* nodes = reinterpret_cast<const uint4*>(uniform.nodes);
     const float4* utris = reinterpret_cast<const float4*>(uniform.tris);
     uint32_t item = 0;
     uint2 group = make_uint2(0u, 0u);
+    uint2 entry = make_uint2(0u, 0u);               // TWO: instances to enter (first leaf entry, hits)
+    bool in_blas = false;                           // TWO: the ray is in an instance's space (or its scene is flat)
+    bool at_marker = false;                         // TWO: popped the end of an instance, waits to leave it
     int sp = 0;
     uint32_t steps = 0;
     float best_t = 0.0f;
-    uint32_t my_groups = 0;                         // this lane's groups in the list
-    uint32_t n_groups = 0, n_tris = 0, n_fin = 0;   // warp-uniform list sizes
-    uint32_t chunk_next = 0, chunk_end = 0;         // warp-uniform: unclaimed items [next, end) of the chunk
+    bool pending = false;                           // this lane has groups in the list
+    uint32_t n_groups = 0, n_fin = 0;               // warp-uniform list sizes
+    uint32_t st_next = 0, st_count = 0, st_base = 0;   // warp-uniform: staged rays not taken yet, item of the first
     bool exhausted = false;
-    // tests the warp's triangle list (all lanes together) and takes each lane's result
+
+    auto pop = [&]() {
+        --sp;
+        group = sp < SS ? stack[sp * stride] : spill[sp - SS];
+    };
+    auto push = [&](uint2 g) {
+        if (sp < SS) {
+            stack[sp * stride] = g;
+            ++sp;
+        } else if (sp < kTotalStack) {
+            spill[sp - SS] = g;
+            ++sp;
+        } else {
+            err |= kErrStackOverflow;
+        }
+    };
+    // tests the warp's list (all lanes together) and takes each lane's result
     auto flush = [&]() {
         __syncwarp();
-        coop_test_groups<COUNT, MIXED>(S, lane, n_groups, utris, cnt);
+        cnt.tris += coop_test_groups<COUNT, MIXED, TWO>(n_groups, utris);
         n_groups = 0;
-        n_tris = 0;
-        if (has && my_groups) {
+        if (pending) {
             const unsigned long long key = S.best[lane];
             if (ANY) {
-                if ((uint32_t)key != 0xFFFFFFFFu) { group = make_uint2(0u, 0u); sp = 0; }
+                if ((uint32_t)key != 0xFFFFFFFFu) {
+                    group = make_uint2(0u, 0u);
+                    sp = 0;
+                    if (TWO) { entry.y = 0u; at_marker = false; }
+                }
             } else {
                 best_t = coop_unordered((uint32_t)(key >> 32));
             }
         }
-        my_groups = 0;
+        pending = false;
     };
+
     for (;;) {
-        // refill idle lanes
-        const uint32_t active = __ballot_sync(0xFFFFFFFFu, has);
-        const uint32_t n_active = (uint32_t)__popc(active);
-        if (!exhausted && n_active <= refill_at) {
-            const uint32_t idle = ~active;
-            const uint32_t n_idle = 32u - n_active;
-            const uint32_t rem = chunk_end - chunk_next;
-            uint32_t base = 0;
-            if (rem < n_idle) {
-                if (lane == 0) base = atomicAdd(next, CHUNK);
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            }
-            bool empty_item = false;
-            if (!has) {
-                const uint32_t rank = (uint32_t)__popc(idle & lanemask_lt());
-                const uint32_t i = rank < rem ? chunk_next + rank : base + (rank - rem);
-                if (i < n && (rank < rem || base < n)) {
-                    item = i;
-                    CoopScene own = uniform;
-                    const bool loaded = load(i, r, own);
-                    if (MIXED) sc = own;
-                    const bool traced = loaded && (MIXED ? own.node_count : uniform.node_count) != 0;
-                    if (traced) {
-                        has = true;
-                        group = make_uint2(0u, 0x80000000u);
-                        sp = 0;
-                        steps = 0;
-                        best_t = r.tmax;
-                        S.ray_a[lane] = make_float4(r.ox, r.oy, r.oz, r.tmin);
-                        S.ray_b[lane] = make_float4(r.sx, r.sy, r.sz,
-                                                    __uint_as_float((uint32_t)r.kx | ((uint32_t)r.ky << 2) | ((uint32_t)r.kz << 4)));
-                        S.best[lane] = ((unsigned long long)coop_ordered(r.tmax) << 32) | 0xFFFFFFFFull;
-                        if (MIXED) S.tris[lane] = reinterpret_cast<const float4*>(sc.tris);
-                    } else {
-                        empty_item = true;   // no ray: stored as a miss
+        // refill idle lanes from the staged rays, staging the next chunk when they run out
+        const uint32_t active = __ballot_sync(kAll, has);
+        if ((uint32_t)__popc(active) <= refill_at && !(exhausted && st_next >= st_count)) {
+            uint32_t idle = ~active;
+            while (idle) {
+                if (st_next >= st_count) {
+                    if (exhausted) break;
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(next, kCoopChunk);
+                    base = __shfl_sync(kAll, base, 0);
+                    st_next = 0;
+                    st_count = base < n ? min(kCoopChunk, n - base) : 0u;
+                    st_base = base;
+                    if (st_count < kCoopChunk) exhausted = true;
+                    if (st_count == 0) break;
+                    if (lane < st_count) {
+                        float4 o, d;
+                        if constexpr (MIXED) S.stage_scene[lane] = load(base + lane, o, d);
+                        else load(base + lane, o, d);
+                        S.stage_o[lane] = o;
+                        S.stage_d[lane] = d;
                     }
+                    __syncwarp();
                 }
-            }
-            if (rem < n_idle) {
-                chunk_next = base + (n_idle - rem);
-                chunk_end = base + CHUNK;
-                if (base >= n) exhausted = true;
-                if (chunk_end > n) chunk_end = n > chunk_next ? n : chunk_next;
-            } else {
-                chunk_next += n_idle;
-            }
-            // items without a ray go straight to the finished list
-            const uint32_t em = __ballot_sync(0xFFFFFFFFu, empty_item);
-            if (em) {
-                if (n_fin + (uint32_t)__popc(em) > 32u) {
-                    coop_store_finished<REFINE, MIXED>(S, lane, n_fin, utris, store);
-                    n_fin = 0;
+                const uint32_t take = min((uint32_t)__popc(idle), st_count - st_next);
+                const uint32_t rank = (uint32_t)__popc(idle & lanemask_lt());
+                const bool mine = ((idle >> lane) & 1u) && rank < take;
+                if (mine) {
+                    const uint32_t e = st_next + rank;
+                    const float4 o = S.stage_o[e], d = S.stage_d[e];
+                    item = st_base + e;
+                    r = make_trace_ray(o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w);
+                    octant_weights(r.oct_inv, wlo, whi);
+                    uint32_t node_count = uniform.node_count;
+                    bool two = TWO;
+                    if constexpr (MIXED) {
+                        const DeviceScene* sc = S.stage_scene[e];
+                        S.scene[lane] = sc;
+                        nodes = reinterpret_cast<const uint4*>(sc->nodes);
+                        node_count = sc->node_count;
+                        if (TWO) two = sc->inst_trav != nullptr;
+                    }
+                    if constexpr (TWO) {
+                        S.world_o[lane] = o;
+                        S.first[lane] = 0;
+                        S.inst[lane] = 0;
+                        S.best_inst[lane] = 0;
+                        in_blas = !two;
+                        at_marker = false;
+                        entry.y = 0u;
+                    }
+                    has = true;
+                    group = make_uint2(0u, node_count ? 0x80000000u : 0u);
+                    sp = 0;
+                    steps = 0;
+                    best_t = d.w;
+                    S.ray_o[lane] = o;
+                    S.ray_s[lane] = make_float4(r.sx, r.sy, r.sz,
+                                                __uint_as_float((uint32_t)r.kx | ((uint32_t)r.ky << 2) | ((uint32_t)r.kz << 4)));
+                    S.ray_d[lane] = d;
+                    S.best[lane] = ((unsigned long long)coop_ordered(d.w) << 32) | 0xFFFFFFFFull;
                 }
-                if (empty_item) {
-                    const uint32_t pos = n_fin + (uint32_t)__popc(em & lanemask_lt());
-                    S.fin_o[pos] = make_float4(0.0f, 0.0f, 0.0f, r.tmax);
-                    S.fin_d[pos] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    S.fin_i[pos] = make_uint4(item, kMiss, 0u, 0u);
-                    if (MIXED) S.fin_tris[pos] = nullptr;
-                }
-                n_fin += (uint32_t)__popc(em);
+                idle &= ~__ballot_sync(kAll, mine);
+                st_next += take;
             }
         }
-        if (!__any_sync(0xFFFFFFFFu, has)) {
-            if (exhausted) break;
-            continue;
-        }
+        if (!__any_sync(kAll, has)) break;   // nothing staged is left either
         // watchdog: a ray's traversal ends with kErrStepLimit after kMaxTraversalSteps visit slots
         if (has) {
             steps += VISITS;
@@ -304,82 +405,157 @@ __device__ __forceinline__ uint32_t coop_trace(const CoopScene& uniform, uint32_
                 err |= kErrStepLimit;
                 group = make_uint2(0u, 0u);
                 sp = 0;
+                if (TWO) { entry.y = 0u; at_marker = false; }
             }
         }
         // VISITS node visits per tracing lane, each followed by its stack pop; every visit's leaf triangles
-        // join the warp's list (tested before the list could overflow, between visits if need be)
+        // join the warp's list (tested when a further visit's could overflow it)
 #pragma unroll
         for (int v = 0; v < VISITS; ++v) {
-            uint32_t tbase = 0, tmask = 0;
-            if (has && group.y > 0x00FFFFFFu) {
+            uint32_t tbase = 0;
+            uint2 leaf = make_uint2(0u, 0u);   // meta bytes of the hit leaf children
+            if (has && group.y > 0x00FFFFFFu && (!TWO || entry.y == 0u)) {
                 const uint32_t slot_bit = 31u - __clz(group.y);
                 const uint32_t slot = (slot_bit - 24u) ^ r.oct_inv;
                 const uint32_t child = group.x + (uint32_t)__popc(group.y & ((1u << slot) - 1u));
                 group.y &= ~(1u << slot_bit);
-                if (group.y > 0x00FFFFFFu) {
-                    if (sp < SS) {
-                        stack[sp * stride] = group;
-                        ++sp;
-                    } else if (sp < kTotalStack) {
-                        spill[sp - SS] = group;
-                        ++sp;
-                    } else {
-                        err |= kErrStackOverflow;
-                    }
-                }
-                const uint4* np = reinterpret_cast<const uint4*>(MIXED ? sc.nodes : uniform.nodes) + 5ull * child;
+                if (group.y > 0x00FFFFFFu) push(group);
+                const uint4* np = nodes + 5ull * child;
                 const uint4 w0 = __ldg(np + 0), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
                             w4 = __ldg(np + 4);
                 if (COUNT) cnt.nodes++;
-                const uint32_t hm = intersect_children(r, w0, w1, w2, w3, w4, best_t);
-                group = make_uint2(w1.x, (hm & 0xFF000000u) | (w0.w >> 24));
+                uint32_t ordered;
+                child_hits(r, wlo, whi, w0, w1, w2, w3, w4, best_t, ordered, leaf);
+                group = make_uint2(w1.x, ordered << 24 | (w0.w >> 24));
                 tbase = w1.y;
-                tmask = hm & 0x00FFFFFFu;
             }
-            if (has && group.y <= 0x00FFFFFFu && sp > 0) {
-                --sp;
-                group = sp < SS ? stack[sp * stride] : spill[sp - SS];
-            }
-            const uint32_t app = __ballot_sync(0xFFFFFFFFu, tmask != 0u);
-            if (app) {
-                if (tmask) {
-                    const uint32_t pos = n_groups + (uint32_t)__popc(app & lanemask_lt());
-                    S.gbase[pos] = tbase;
-                    S.gmo[pos] = (lane << 24) | tmask;
-                    ++my_groups;
+            if constexpr (TWO) {
+                if (!in_blas && (leaf.x | leaf.y)) {   // top-level leaves: the lane's instances to enter
+                    entry.x = tbase;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t m = ((i < 4 ? leaf.x : leaf.y) >> (8 * (i & 3))) & 0xFFu;
+                        entry.y |= (m >> 5) << (m & 31u);
+                    }
+                    leaf = make_uint2(0u, 0u);
                 }
-                n_groups += (uint32_t)__popc(app);
-                n_tris += __reduce_add_sync(0xFFFFFFFFu, (uint32_t)__popc(tmask));
+                if (has && !at_marker && entry.y == 0u && group.y <= 0x00FFFFFFu && sp > 0) {
+                    pop();
+                    if (group.x == kLevelMarker && group.y == 0u) {
+                        at_marker = true;
+                    } else if (group.y <= 0x00FFFFFFu) {   // instances left of an earlier top-level leaf
+                        entry = group;
+                        group = make_uint2(0u, 0u);
+                    }
+                }
+            } else {
+                if (has && group.y <= 0x00FFFFFFu && sp > 0) pop();
             }
+            const bool found = (leaf.x | leaf.y) != 0u;
+            const uint32_t app = __ballot_sync(kAll, found);
+            if (found) {
+                const uint32_t pos = n_groups + (uint32_t)__popc(app & lanemask_lt());
+                S.g_base[pos] = tbase;
+                S.g_meta[0][pos] = leaf.x;
+                S.g_meta[1][pos] = leaf.y;
+                S.g_own[pos] = (uint8_t)lane;
+                pending = true;
+            }
+            n_groups += (uint32_t)__popc(app);
             if (v + 1 < VISITS && n_groups > 32u) flush();
         }
-        // test the list when it is full enough, could overflow next step, or holds groups of a finished lane
-        const bool waiting = has && group.y <= 0x00FFFFFFu && sp == 0 && my_groups > 0;
-        if (n_groups && (__any_sync(0xFFFFFFFFu, waiting) || n_tris >= FLUSH || n_groups > 32u)) flush();
+        // test the list when it is full enough, could overflow next step, or lanes with groups in it have nothing
+        // else to do
+        const bool idle_pending = has && pending && group.y <= 0x00FFFFFFu && (TWO ? (at_marker || (sp == 0 && entry.y == 0u)) : sp == 0);
+        const bool waiting = __any_sync(kAll, idle_pending);
+        if (n_groups && (waiting || n_groups >= FLUSH || n_groups > 32u)) flush();
+        if constexpr (TWO) {
+            // leave instances: back to the world ray and the entries below the marker
+            if (at_marker && !pending) {
+                at_marker = false;
+                in_blas = false;
+                const float4 o = S.world_o[lane], d = S.ray_d[lane];
+                r.ox = o.x; r.oy = o.y; r.oz = o.z;
+                r.idx = safe_rcp(d.x); r.idy = safe_rcp(d.y); r.idz = safe_rcp(d.z);
+                r.oct_inv = 7u - ((d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u));
+                octant_weights(r.oct_inv, wlo, whi);
+                group = make_uint2(0u, 0u);
+                if (sp > 0) {
+                    pop();
+                    if (group.y <= 0x00FFFFFFu) {
+                        entry = group;
+                        group = make_uint2(0u, 0u);
+                    }
+                }
+            }
+            // enter the next instance; the rest of the top level waits below a marker
+            if (entry.y) {
+                const DeviceScene* sc = &uniform;
+                if constexpr (MIXED) sc = S.scene[lane];
+                const uint32_t k = (uint32_t)__ffs(entry.y) - 1u;
+                entry.y &= entry.y - 1u;
+                const uint32_t ii = __ldg(sc->tlas_refs + entry.x + k);
+                const uint4 tail = __ldg(reinterpret_cast<const uint4*>(sc->inst_trav + ii) + 3);
+                if (tail.x != 0xFFFFFFFFu) {   // (a model without triangles has no bottom level)
+                    if (group.y > 0x00FFFFFFu) push(group);
+                    if (entry.y) push(entry);
+                    entry.y = 0u;
+                    push(make_uint2(kLevelMarker, 0u));
+                    const float4 o = S.world_o[lane], d = S.ray_d[lane];
+                    TraceRay w;
+                    w.ox = o.x; w.oy = o.y; w.oz = o.z;
+                    w.dx = d.x; w.dy = d.y; w.dz = d.z;
+                    w.tmin = o.w; w.tmax = d.w;
+                    r = instance_ray(w, sc->inst_trav + ii);
+                    octant_weights(r.oct_inv, wlo, whi);
+                    S.ray_o[lane] = make_float4(r.ox, r.oy, r.oz, r.tmin);
+                    S.ray_s[lane] = make_float4(r.sx, r.sy, r.sz,
+                                                __uint_as_float((uint32_t)r.kx | ((uint32_t)r.ky << 2) | ((uint32_t)r.kz << 4)));
+                    S.inst[lane] = ii;
+                    S.first[lane] = tail.y;
+                    in_blas = true;
+                    group = make_uint2(tail.x, 0x80000000u);
+                } else if (entry.y == 0u && group.y <= 0x00FFFFFFu && sp > 0) {
+                    pop();   // at the top level: nodes or instances, never a marker
+                    if (group.y <= 0x00FFFFFFu) {
+                        entry = group;
+                        group = make_uint2(0u, 0u);
+                    }
+                }
+            }
+        }
         // finished rays join the warp's finished list
-        const bool done = has && group.y <= 0x00FFFFFFu && sp == 0 && my_groups == 0;
-        const uint32_t dm = __ballot_sync(0xFFFFFFFFu, done);
+        const bool done = has && group.y <= 0x00FFFFFFu && sp == 0 && !pending && (!TWO || (entry.y == 0u && !at_marker));
+        const uint32_t dm = __ballot_sync(kAll, done);
         if (dm) {
             if (n_fin + (uint32_t)__popc(dm) > 32u) {
-                coop_store_finished<REFINE, MIXED>(S, lane, n_fin, utris, store);
+                coop_store_finished<REFINE, MIXED, TWO>(n_fin, uniform, store);
                 n_fin = 0;
             }
             if (done) {
                 const uint32_t pos = n_fin + (uint32_t)__popc(dm & lanemask_lt());
                 const unsigned long long key = S.best[lane];
-                const float4 bh = S.best_hit[lane];
                 const bool miss = (uint32_t)key == 0xFFFFFFFFu;
-                S.fin_o[pos] = make_float4(r.ox, r.oy, r.oz, miss ? r.tmax : bh.y);
-                S.fin_d[pos] = make_float4(r.dx, r.dy, r.dz, miss ? 0.0f : bh.z);
-                S.fin_i[pos] = make_uint4(item, miss ? kMiss : (uint32_t)key, miss ? 0u : __float_as_uint(bh.x),
-                                          miss ? 0u : __float_as_uint(bh.w));
-                if (MIXED) S.fin_tris[pos] = S.tris[lane];
+                float4 o;
+                uint32_t inst = 0;
+                if constexpr (TWO) {
+                    o = S.world_o[lane];
+                    inst = S.best_inst[lane];
+                } else {
+                    o = S.ray_o[lane];
+                }
+                const float4 d = S.ray_d[lane];
+                const uint2 rec = S.best_rec[lane];
+                S.fin_o[pos] = make_float4(o.x, o.y, o.z, miss ? d.w : __uint_as_float(rec.y));
+                S.fin_d[pos] = d;
+                S.fin_i[pos] = make_uint4(item, (uint32_t)key, rec.x, inst);
+                if constexpr (MIXED) S.fin_scene[pos] = S.scene[lane];
                 has = false;
             }
             n_fin += (uint32_t)__popc(dm);
         }
     }
-    if (n_fin) coop_store_finished<REFINE, MIXED>(S, lane, n_fin, utris, store);
+    if (n_fin) coop_store_finished<REFINE, MIXED, TWO>(n_fin, uniform, store);
     return err;
 }
 

@@ -13,9 +13,9 @@ namespace rt {
 
 constexpr int kTraceBlock = 128;
 // Traversal launch form: 0 = one thread per ray (grid); 1..32 = the warp-cooperative persistent form
-// (coop_trace.cuh), whose warps fetch new rays once this many of their 32 lanes are idle.  The
-// cooperative form is the default for flat scenes (two-level scenes always run the grid form): on the
-// 1.3M-triangle ray cast, closest hit 0.58 ms against 0.82 ms for the grid form, any hit 0.36 / 0.51 ms.
+// (coop_trace.cuh), whose warps take new rays once this many of their 32 lanes are idle.  The cooperative form
+// is the default: on the 1.3M-triangle ray cast closest hit 0.42 ms against 0.80 ms for the grid form, on 256
+// instances of a 20,480-triangle model (two-level) 0.93 against 1.48 ms.
 constexpr int kDefaultRefill = 8;
 // Launch form of the wavefront extension and shadow kernels (renders, batches, the server): the grid
 // form.  The cooperative form's refill costs more than it saves there, where a wave's queue holds many

@@ -103,20 +103,18 @@ __global__ void __launch_bounds__(BLOCK) k_extend_grid(RenderLaunch L, int cur) 
 
 // Cooperative persistent form (coop_trace.cuh): warps refill idle lanes from the queue; triangle tests
 // and hit refinement are spread over the warp.  Flat scenes.
-__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_extend(RenderLaunch L, int cur) {
-    __shared__ CoopWarp warps[kBlock / 32];
-    __shared__ uint2 stack[kSmemStack * kBlock];
+__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_extend(const __grid_constant__ RenderLaunch L, int cur) {
     const PathState& ps = L.ps;
     const uint32_t n = ps.counters[kCntActive + cur];
     const uint32_t* q = ps.q_active[cur];
     TraceCounters c{0u, 0u};
-    auto load = [&](uint32_t i, TraceRay& r, CoopScene& sc) {
+    auto load = [&](uint32_t i, float4& o, float4& d) {
         const uint32_t p = checked_index(q[i], L.P, ps.counters + kCntError);
-        r = make_trace_ray(ps.ox[p], ps.oy[p], ps.oz[p], ps.dx[p], ps.dy[p], ps.dz[p], 0.0f, 10000.0f);
-        (void)sc;
-        return true;
+        o = make_float4(ps.ox[p], ps.oy[p], ps.oz[p], 0.0f);
+        d = make_float4(ps.dx[p], ps.dy[p], ps.dz[p], 10000.0f);
     };
-    auto store = [&](uint32_t i, const Hit& h, bool valid) {   // called by all 32 lanes
+    auto store = [&](uint32_t i, const CoopHit& c, bool valid) {   // called by all 32 lanes
+        const Hit& h = c.h;
         int m = -1;
         uint32_t p = 0;
         if (valid) {
@@ -135,10 +133,8 @@ __global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_extend(RenderLaunch 
             if (mine) ps.q_shade[(size_t)k * L.P + checked_index(pos, L.P, ps.counters + kCntError)] = p;
         }
     };
-    const uint32_t e = coop_trace<false, true, true, false, kSmemStack>(CoopScene{L.s.nodes, L.s.tris, L.s.node_count}, n,
-                                                                        ps.counters + kCntFetchExtend, (uint32_t)(32 - L.refill),
-                                                                 warps[threadIdx.x >> 5], stack + threadIdx.x, kBlock,
-                                                                 load, store, c);
+    const uint32_t e = coop_trace<false, true, true, false, false>(L.s, n, ps.counters + kCntFetchExtend,
+                                                                   (uint32_t)(32 - L.refill), load, store, c);
     if (e) atomicOr(ps.counters + kCntError, e);
     coop_add_counts(c, ps.counters, kCntNodes, kCntTris);
 }
@@ -262,28 +258,23 @@ __global__ void __launch_bounds__(BLOCK) k_shadow_grid(RenderLaunch L) {
 }
 
 // Cooperative persistent form of the shadow kernel (flat scenes).
-__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_shadow(RenderLaunch L) {
-    __shared__ CoopWarp warps[kBlock / 32];
-    __shared__ uint2 stack[kSmemStack * kBlock];
+__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_shadow(const __grid_constant__ RenderLaunch L) {
     const PathState& ps = L.ps;
     const uint32_t n = ps.counters[kCntShadow];
     TraceCounters c{0u, 0u};
-    auto load = [&](uint32_t i, TraceRay& r, CoopScene& sc) {
-        r = make_trace_ray(ps.s_ox[i], ps.s_oy[i], ps.s_oz[i], ps.s_dx[i], ps.s_dy[i], ps.s_dz[i], 0.0f, ps.s_tmax[i]);
-        (void)sc;
-        return true;
+    auto load = [&](uint32_t i, float4& o, float4& d) {
+        o = make_float4(ps.s_ox[i], ps.s_oy[i], ps.s_oz[i], 0.0f);
+        d = make_float4(ps.s_dx[i], ps.s_dy[i], ps.s_dz[i], ps.s_tmax[i]);
     };
-    auto store = [&](uint32_t i, const Hit& h, bool valid) {   // called by all 32 lanes
-        if (valid && h.prim == kMiss) {
+    auto store = [&](uint32_t i, const CoopHit& c, bool valid) {   // called by all 32 lanes
+        if (valid && c.h.prim == kMiss) {
             const uint32_t p = checked_index(ps.q_shadow[i], L.P, ps.counters + kCntError);
             store_rad(ps, p, load_rad(ps, p) + V3{ps.s_cr[i], ps.s_cg[i], ps.s_cb[i]});
         }
         warp_count64(reinterpret_cast<unsigned long long*>(ps.counters + kCntShadowRays), valid);
     };
-    const uint32_t e = coop_trace<true, true, false, false, kSmemStack>(CoopScene{L.s.nodes, L.s.tris, L.s.node_count}, n,
-                                                                        ps.counters + kCntFetchShadow, (uint32_t)(32 - L.refill),
-                                                                 warps[threadIdx.x >> 5], stack + threadIdx.x, kBlock,
-                                                                 load, store, c);
+    const uint32_t e = coop_trace<true, true, false, false, false>(L.s, n, ps.counters + kCntFetchShadow,
+                                                                   (uint32_t)(32 - L.refill), load, store, c);
     if (e) atomicOr(ps.counters + kCntError, e);
     coop_add_counts(c, ps.counters, kCntShadowNodes, kCntShadowTris);
 }
@@ -486,7 +477,7 @@ void RenderWorkspace::ensure(uint32_t paths) {
 
 // Resident grid (blocks per SM x SMs) of a kernel at a block size, computed once per (kernel, block size,
 // SM count) and kept in a table that any thread rendering may read or fill (under a lock).
-static int cached_grid(const void* fn, int block, int sm_count) {
+static int cached_grid(const void* fn, int block, int sm_count, size_t shared = 0) {
     static std::mutex mu;
     static std::map<std::tuple<const void*, int, int>, int> table;
     const auto key = std::make_tuple(fn, block, sm_count);
@@ -495,7 +486,7 @@ static int cached_grid(const void* fn, int block, int sm_count) {
         const auto it = table.find(key);
         if (it != table.end()) return it->second;
     }
-    const int g = resident_grid(fn, block, sm_count);
+    const int g = resident_grid(fn, block, sm_count, shared);
     std::lock_guard<std::mutex> lock(mu);
     table[key] = g;
     return g;
@@ -522,8 +513,8 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
     L.samples = d_samples;
     L.refill = opt.trace.refill;
 
-    const int g_ext = occupancy_blocks((const void*)k_extend, sm_count);
-    const int g_sh = occupancy_blocks((const void*)k_shadow, sm_count);
+    const int g_ext = cached_grid((const void*)k_extend, kBlock, sm_count, coop_shared_bytes<false, false>());
+    const int g_sh = cached_grid((const void*)k_shadow, kBlock, sm_count, coop_shared_bytes<false, false>());
     const int g_shade[5] = {0, occupancy_blocks((const void*)k_shade<1>, sm_count),
                             occupancy_blocks((const void*)k_shade<2>, sm_count),
                             occupancy_blocks((const void*)k_shade<3>, sm_count),
@@ -553,7 +544,7 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
                 const int grid = cached_grid((const void*)k_extend_grid<kTraceBlock, kDefaultTraceStack, true>, kTraceBlock, sm_count);
                 k_extend_grid<kTraceBlock, kDefaultTraceStack, true><<<grid, kTraceBlock, 0, st>>>(L, cur);
             } else if (opt.trace.refill > 0) {
-                k_extend<<<g_ext, kBlock, 0, st>>>(L, cur);
+                k_extend<<<g_ext, kBlock, coop_shared_bytes<false, false>(), st>>>(L, cur);
             } else {
                 with_trace_variant(opt.trace, [&](auto B, auto S) {
                     const int grid = cached_grid((const void*)k_extend_grid<B.value, S.value, false>, B.value, sm_count);
@@ -570,7 +561,7 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
                     const int grid = cached_grid((const void*)k_shadow_grid<kTraceBlock, kDefaultTraceStack, true>, kTraceBlock, sm_count);
                     k_shadow_grid<kTraceBlock, kDefaultTraceStack, true><<<grid, kTraceBlock, 0, st>>>(L);
                 } else if (opt.trace.refill > 0) {
-                    k_shadow<<<g_sh, kBlock, 0, st>>>(L);
+                    k_shadow<<<g_sh, kBlock, coop_shared_bytes<false, false>(), st>>>(L);
                 } else {
                     with_trace_variant(opt.trace, [&](auto B, auto S) {
                         const int grid = cached_grid((const void*)k_shadow_grid<B.value, S.value, false>, B.value, sm_count);

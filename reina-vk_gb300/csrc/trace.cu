@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "coop_trace.cuh"
 #include "kernels.h"
@@ -37,28 +38,21 @@ __device__ __forceinline__ void reduce_counters(const TraceCounters& c, unsigned
 
 // Warp-cooperative persistent form (coop_trace.cuh): warps refill idle lanes once at most `refill_at` of
 // their lanes still trace; triangle tests and hit refinement are spread over the warp.
-template <bool ANY, bool COUNT>
-__global__ void __launch_bounds__(kTraceBlock, kCoopMinBlocks) raycast_kernel(const Bvh8Node* __restrict__ nodes,
-                                                              const TriRecord* __restrict__ tris, uint32_t node_count,
-                                                              const Ray* __restrict__ rays, uint32_t n,
-                                                              Hit* __restrict__ hits, unsigned long long* counters,
-                                                              uint32_t* err_flag, uint32_t* next, uint32_t refill_at) {
-    __shared__ CoopWarp warps[kTraceBlock / 32];
-    __shared__ uint2 stack[kSmemStack * kTraceBlock];
+template <bool ANY, bool COUNT, bool TWO>
+__global__ void __launch_bounds__(kTraceBlock, TWO ? kCoopMinBlocksTwo : kCoopMinBlocks)
+    raycast_kernel(const __grid_constant__ DeviceScene scene, const Ray* __restrict__ rays, uint32_t n, Hit* __restrict__ hits,
+                   unsigned long long* counters, uint32_t* err_flag, uint32_t* next, uint32_t refill_at) {
     TraceCounters c{0u, 0u};
-    auto load = [&](uint32_t i, TraceRay& r, CoopScene& sc) {
+    auto load = [&](uint32_t i, float4& o, float4& d) {
         const float4* rp = reinterpret_cast<const float4*>(rays) + 2ull * i;
-        const float4 a = __ldcs(rp), b = __ldcs(rp + 1);
-        r = make_trace_ray(a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w);
-        (void)sc;
-        return true;
+        o = __ldcs(rp);
+        d = __ldcs(rp + 1);
     };
-    auto store = [&](uint32_t i, const Hit& h, bool valid) {
+    auto store = [&](uint32_t i, const CoopHit& c, bool valid) {
+        const Hit& h = c.h;
         if (valid && hits) __stcs(reinterpret_cast<float4*>(hits) + i, make_float4(__uint_as_float(h.prim), h.t, h.u, h.v));
     };
-    const uint32_t e = coop_trace<ANY, COUNT, true, false, kSmemStack>(CoopScene{nodes, tris, node_count}, n, next, refill_at,
-                                                                       warps[threadIdx.x >> 5], stack + threadIdx.x,
-                                                                       kTraceBlock, load, store, c);
+    const uint32_t e = coop_trace<ANY, COUNT, true, false, TWO>(scene, n, next, refill_at, load, store, c);
     if (e) atomicOr(err_flag, e);
     reduce_counters<COUNT>(c, counters);
 }
@@ -248,14 +242,25 @@ static void ray_order(const Ray* d_rays, uint64_t n, uint32_t* bin_of, uint32_t*
     k_ray_scatter<<<grid * 4, kBinBlock, 0, st>>>(bin_of, (uint32_t)n, hist, order);
 }
 
-template <bool ANY, bool COUNT>
+template <bool ANY, bool COUNT, bool TWO>
 static int persistent_grid(int sm_count) {
     static const int per_sm = [] {   // initialised once, thread-safely (a function-local static)
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, raycast_kernel<ANY, COUNT>, kTraceBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, raycast_kernel<ANY, COUNT, TWO>, kTraceBlock,
+                                                      coop_shared_bytes<false, TWO>());
         return std::max(1, b);
     }();
     return per_sm * std::max(1, sm_count);
+}
+
+template <bool ANY, bool COUNT, bool TWO>
+static void launch_coop(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_hits, unsigned long long* d_counters,
+                        uint32_t* d_err, uint32_t* d_next, int sm_count, int refill, cudaStream_t st) {
+    const uint64_t needed = (n + kTraceBlock - 1) / kTraceBlock;
+    check_cuda(cudaMemsetAsync(d_next, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
+    const int grid = (int)std::min<uint64_t>(needed, (uint64_t)persistent_grid<ANY, COUNT, TWO>(sm_count));
+    raycast_kernel<ANY, COUNT, TWO><<<grid, kTraceBlock, coop_shared_bytes<false, TWO>(), st>>>(
+        s, d_rays, (uint32_t)n, d_hits, d_counters, d_err, d_next, (uint32_t)(32 - refill));
 }
 
 // Two-level scenes always run the default block size and stack depth.
@@ -284,9 +289,8 @@ static void launch_grid_stack(int stack, const DeviceScene& s, const Ray* d_rays
 template <bool ANY>
 static void launch(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_hits, uint32_t* d_err, uint32_t* d_next,
                    int sm_count, const TraceConfig& cfg, cudaStream_t st) {
-    // grid form (also for more than 2^31 rays, where the persistent form's fetch counter could wrap, and
-    // for two-level scenes)
-    if (cfg.refill <= 0 || n > (1ull << 31) || s.inst_trav) {
+    // grid form (also for more than 2^31 rays, where the persistent form's fetch counter could wrap)
+    if (cfg.refill <= 0 || n > (1ull << 31)) {
         uint32_t* scratch = nullptr;
         const uint32_t* order = nullptr;
         if (cfg.sort) {   // stream-ordered scratch: concurrent calls on other streams do not share it
@@ -300,11 +304,8 @@ static void launch(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_h
         if (scratch) check_cuda(cudaFreeAsync(scratch, st), "cudaFreeAsync");
         return;
     }
-    const uint64_t needed = (n + kTraceBlock - 1) / kTraceBlock;
-    check_cuda(cudaMemsetAsync(d_next, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
-    const int grid = (int)std::min<uint64_t>(needed, (uint64_t)persistent_grid<ANY, false>(sm_count));
-    raycast_kernel<ANY, false><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, s.node_count, d_rays, (uint32_t)n, d_hits,
-                                                             nullptr, d_err, d_next, (uint32_t)(32 - cfg.refill));
+    if (s.inst_trav) launch_coop<ANY, false, true>(s, d_rays, n, d_hits, nullptr, d_err, d_next, sm_count, cfg.refill, st);
+    else launch_coop<ANY, false, false>(s, d_rays, n, d_hits, nullptr, d_err, d_next, sm_count, cfg.refill, st);
 }
 
 bool valid_trace_config(const TraceConfig& c) {
@@ -325,25 +326,20 @@ void launch_raycast_counters(const DeviceScene& s, const Ray* d_rays, uint64_t n
                              unsigned long long* d_counters, uint32_t* d_err, uint32_t* d_next, int sm_count,
                              cudaStream_t st) {
     if (n == 0) return;
-    // The counting build of the default form: the cooperative form for flat scenes (its deferred triangle
-    // tests cull later, so it may visit a few more nodes than the grid form), the grid form otherwise.
-    if (s.inst_trav || n > (1ull << 31)) {
+    // The counting build of the default form, the cooperative one (its deferred triangle tests cull later, so it
+    // may visit a few more nodes than the grid form); the grid form for more rays than its fetch counter holds.
+    if (n > (1ull << 31)) {
         if (any) launch_grid<true, true, kTraceBlock, kSmemStack>(s, d_rays, n, nullptr, d_counters, d_err, nullptr, st);
         else launch_grid<false, true, kTraceBlock, kSmemStack>(s, d_rays, n, nullptr, d_counters, d_err, nullptr, st);
         return;
     }
-    check_cuda(cudaMemsetAsync(d_next, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
-    const uint64_t needed = (n + kTraceBlock - 1) / kTraceBlock;
-    const uint32_t refill_at = (uint32_t)(32 - kDefaultRefill);
-    if (any) {
-        const int grid = (int)std::min<uint64_t>(needed, (uint64_t)persistent_grid<true, true>(sm_count));
-        raycast_kernel<true, true><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, s.node_count, d_rays, (uint32_t)n,
-                                                                 nullptr, d_counters, d_err, d_next, refill_at);
-    } else {
-        const int grid = (int)std::min<uint64_t>(needed, (uint64_t)persistent_grid<false, true>(sm_count));
-        raycast_kernel<false, true><<<grid, kTraceBlock, 0, st>>>(s.nodes, s.tris, s.node_count, d_rays, (uint32_t)n,
-                                                                  nullptr, d_counters, d_err, d_next, refill_at);
-    }
+    auto go = [&](auto any_c, auto two_c) {
+        launch_coop<any_c.value, true, two_c.value>(s, d_rays, n, nullptr, d_counters, d_err, d_next, sm_count, kDefaultRefill, st);
+    };
+    if (any && s.inst_trav) go(std::true_type{}, std::true_type{});
+    else if (any) go(std::true_type{}, std::false_type{});
+    else if (s.inst_trav) go(std::false_type{}, std::true_type{});
+    else go(std::false_type{}, std::false_type{});
 }
 
 }  // namespace rt

@@ -151,7 +151,8 @@ __device__ __forceinline__ float dot2_f(float x0, float x1, float x2, float y0, 
     return __fadd_rn(p, s);
 }
 
-__device__ __forceinline__ void refine_hit(const TraceRay& r, const float4& a4, const float4& b4, const float4& c4,
+// Returns false, with the hit as it was, where the determinant vanishes.
+__device__ __forceinline__ bool refine_hit(const TraceRay& r, const float4& a4, const float4& b4, const float4& c4,
                                            Hit& h) {
     const float t0 = h.t;
     auto moved = [&](float o, float d, float v0) {   // (o + t0 d) - v0 with the moved origin kept exactly
@@ -166,11 +167,12 @@ __device__ __forceinline__ void refine_hit(const TraceRay& r, const float4& a4, 
     const float p0 = diff_prod_f(r.dy, e22, r.dz, e21), p1 = diff_prod_f(r.dz, e20, r.dx, e22),
                 p2 = diff_prod_f(r.dx, e21, r.dy, e20);
     const float det = dot2_f(e10, e11, e12, p0, p1, p2);
-    if (det == 0.0f) return;
+    if (det == 0.0f) return false;
     const float q0 = diff_prod_f(s1, e12, s2, e11), q1 = diff_prod_f(s2, e10, s0, e12), q2 = diff_prod_f(s0, e11, s1, e10);
     h.u = __fdiv_rn(dot2_f(s0, s1, s2, p0, p1, p2), det);
     h.v = __fdiv_rn(dot2_f(r.dx, r.dy, r.dz, q0, q1, q2), det);
     h.t = __fadd_rn(t0, __fdiv_rn(dot2_f(e20, e21, e22, q0, q1, q2), det));
+    return true;
 }
 
 // The bits of 1.0f, read by the byte permutes of the box test from the constant bank: as an immediate the
@@ -238,6 +240,67 @@ __device__ __forceinline__ uint32_t intersect_children(const TraceRay& r, const 
     }
     return hitmask;
 }
+
+// Weights that put the hit of child slot i at bit i XOR oct_inv: byte i of `lo` (slots 0..3) and `hi` (4..7) is
+// 1 << (i XOR oct_inv).
+__device__ __forceinline__ void octant_weights(uint32_t oct_inv, uint32_t& lo, uint32_t& hi) {
+    const uint32_t sel = 0x3210u ^ ((oct_inv & 3u) * 0x1111u);
+    const uint32_t a = __byte_perm(0x08040201u, 0u, sel), b = __byte_perm(0x80402010u, 0u, sel);
+    lo = (oct_inv & 4u) ? b : a;
+    hi = (oct_inv & 4u) ? a : b;
+}
+
+// The signs of bytes 0 and 1 of a and of b, as four bytes of 0x00 or 0xFF (prmt's sign-replicating selectors,
+// which __byte_perm masks out).
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, 0xDC98;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// The box test of intersect_children with other results: `ordered` gets the mask of the hit internal children in
+// the ray's order, `leaf` the meta bytes of the hit leaf children (zero for the other slots).  A child is missed
+// where far - near is negative; the eight signs are gathered by byte permutes and weighted by byte dot
+// products, about half of the instructions that eight compares and meta-byte shifts take.
+__device__ __forceinline__ void child_hits(const TraceRay& r, uint32_t wlo, uint32_t whi, const uint4& w0, const uint4& w1,
+                                           const uint4& w2, const uint4& w3, const uint4& w4, float tmax, uint32_t& ordered,
+                                           uint2& leaf) {
+    const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
+    const uint32_t ex = w0.w & 0xFFu, ey = (w0.w >> 8) & 0xFFu, ez = (w0.w >> 16) & 0xFFu;
+    const float sx = __uint_as_float((ex + 15u) << 23) * r.idx;
+    const float sy = __uint_as_float((ey + 15u) << 23) * r.idy;
+    const float sz = __uint_as_float((ez + 15u) << 23) * r.idz;
+    const float ox = (px - r.ox) * r.idx - sx;
+    const float oy = (py - r.oy) * r.idy - sy;
+    const float oz = (pz - r.oz) * r.idz - sz;
+    const bool nx = r.idx < 0.0f, ny = r.idy < 0.0f, nz = r.idz < 0.0f;
+    const uint32_t nearx[2] = {nx ? w3.z : w2.x, nx ? w3.w : w2.y}, farx[2] = {nx ? w2.x : w3.z, nx ? w2.y : w3.w};
+    const uint32_t neary[2] = {ny ? w4.x : w2.z, ny ? w4.y : w2.w}, fary[2] = {ny ? w2.z : w4.x, ny ? w2.w : w4.y};
+    const uint32_t nearz[2] = {nz ? w4.z : w3.x, nz ? w4.w : w3.y}, farz[2] = {nz ? w3.x : w4.z, nz ? w3.y : w4.w};
+    uint32_t miss[2];   // a byte per slot: 0xFF where its box is missed
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t d[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float tnx = fmaf(q15(nearx[h], b), sx, ox), tfx = fmaf(q15(farx[h], b), sx, ox);
+            const float tny = fmaf(q15(neary[h], b), sy, oy), tfy = fmaf(q15(fary[h], b), sy, oy);
+            const float tnz = fmaf(q15(nearz[h], b), sz, oz), tfz = fmaf(q15(farz[h], b), sz, oz);
+            const float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, r.tmin));
+            const float tf = fminf(fminf(tfx, tfy), fminf(tfz, tmax));
+            d[b] = __float_as_uint(tf - tn);
+        }
+        miss[h] = sign_bytes(__byte_perm(d[0], d[1], 0x0073), __byte_perm(d[2], d[3], 0x0073));
+    }
+    // internal children have meta bits 3 and 4 both set
+    const uint32_t i0 = w1.z & (w1.z << 1) & 0x10101010u, i1 = w1.w & (w1.w << 1) & 0x10101010u;
+    ordered = __dp4a(i0 & ~miss[0], wlo, __dp4a(i1 & ~miss[1], whi, 0u)) >> 4;
+    leaf.x = w1.z & ~miss[0] & ~((i0 >> 4) * 0xFFu);
+    leaf.y = w1.w & ~miss[1] & ~((i1 >> 4) * 0xFFu);
+}
+
+// Triangle bits of the meta bytes of leaf children: bits 0..2 of each byte, one per triangle.
+__device__ __forceinline__ uint32_t leaf_bits(uint32_t meta) { return (meta >> 5) & 0x07070707u; }
 
 struct TraceCounters {
     uint32_t nodes;

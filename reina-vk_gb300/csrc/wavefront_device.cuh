@@ -375,10 +375,11 @@ inline void with_trace_variant(const TraceConfig& c, F&& f) {
     else by_stack(std::integral_constant<int, 128>{});
 }
 
-// Host: resident blocks of `kernel` at `block` threads, times the SM count (grid of a grid-stride kernel).
-inline int resident_grid(const void* kernel, int block, int sm_count) {
+// Host: resident blocks of `kernel` at `block` threads and `shared` dynamic shared bytes, times the SM count
+// (grid of a grid-stride kernel).
+inline int resident_grid(const void* kernel, int block, int sm_count, size_t shared = 0) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, shared);
     return (per_sm > 0 ? per_sm : 1) * (sm_count > 0 ? sm_count : 1);
 }
 
