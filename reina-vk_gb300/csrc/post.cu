@@ -5,8 +5,8 @@
 // The reference's kernel has kernelSize = int(radiusPx * 3 + 0.5) taps on each side.  Its sums run over the taps
 // in order (so do these), a NaN or infinite pixel spreads over the whole kernel as it does there, and the
 // sum of the weights counts out-of-image and thresholded taps (blurCommon.h.glsl:24-31).
-// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.156 ms, against 1.558 ms with a thread
-// per pixel that summed every tap.
+// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.144 ms, against 1.558 ms with a thread
+// per pixel that summed every tap; 671x296, radius 0.86: 21 us against 36 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,13 +31,37 @@ static int near_taps(int K, float sigma) {
 // in registers takes 4 new ones per 4 taps; Y, a window of kYOut weights takes one new one per row.
 constexpr int kXOut = 9, kXStep = kXOut + 3;
 constexpr int kYOut = 12;
-constexpr int kXThreads = 128;                 // an X block's outputs: kXSeg consecutive pixels of a row
-constexpr int kXSeg = kXThreads * kXOut;
+constexpr int kXChunk = 32 * kXOut;             // outputs of one warp in one channel
+constexpr int kXSeg = 4 * kXChunk;              // an X block's outputs: consecutive pixels of a row
+constexpr int kXThreads = 3 * 4 * 32;           // a warp per chunk and channel
 constexpr int kYWarps = 4;    // a Y block's outputs: 48 consecutive rows of 32 columns
 constexpr int kYRows = 24;    // rows of the input a Y block holds per stage of its ring
 constexpr int kYStages = 3;
 static_assert(kXSeg % 32 == 0, "a Y block's columns lie in one X segment");
+constexpr int kWeightPart = 1024;   // weights summed from shared memory at a time
 constexpr size_t kXMaxShared = 200 * 1024;
+
+// The three kernels of a call are chained by programmatic launches, which take a launch's latency out of each gap
+// (671x296, radius 2: 27.8 us without, 22.8 us with): a kernel waits (wait_for_previous) before it reads what
+// the one before it wrote.  The first is launched plainly, so nothing of a call starts before the work ahead of it
+// on the stream is done, and it lets blurX start at once, whose blocks load their pixels meanwhile.  blurX does
+// not: blurY's blocks would fill the slots that blurX leaves on some SMs and crowd there (35 us).
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+static void launch_after(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t shared, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "postprocess launch");
+}
 
 struct BloomTaps {
     int K, near;      // kernel half-width, and the half-width of its non-zero taps
@@ -50,6 +74,7 @@ static size_t y_words(int near) { return (size_t)(2 * near + 1 + 3 * kYOut + 3) 
 // Both passes' weights, one block each: the exponentials in parallel, their sum by one thread in order (the
 // zero taps leave it as it is).  One thread for all of it took 47 us at 1920x1080 and radius 5.
 __global__ void __launch_bounds__(kPostBlock) k_bloom_weights(BloomTaps tx, BloomTaps ty, int x_total, int y_total, float sigma) {
+    let_next_start();
     const bool X = blockIdx.x == 0;
     const BloomTaps t = X ? tx : ty;
     const int total = X ? x_total : y_total, pad = X ? 0 : kYOut, n = 2 * t.near + 1;
@@ -62,16 +87,29 @@ __global__ void __launch_bounds__(kPostBlock) k_bloom_weights(BloomTaps tx, Bloo
         }
         t.w[k] = g;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = 0.0f;
+    __shared__ float part[kWeightPart];
+    float sum = 0.0f;
+    for (int base = 0; base < n; base += kWeightPart) {
+        const int m = min(kWeightPart, n - base);
+        __syncthreads();
+        for (int k = threadIdx.x; k < m; k += blockDim.x) part[k] = t.w[pad + base + k];
+        __syncthreads();
+        if (threadIdx.x == 0) {
 #pragma unroll 8
-        for (int i = 0; i < n; ++i) sum += t.w[pad + i];
-        *t.sum = sum;
+            for (int i = 0; i < m; ++i) sum += part[i];
+        }
     }
+    if (threadIdx.x == 0) *t.sum = sum;
 }
 
-__device__ __forceinline__ float blur_mean(float c, float wsum) { return wsum < 0.0001f ? 0.0f : c / wsum; }
+// c / wsum.  A quotient of a tiny c would take the division's slow path, and where little passes the threshold
+// most sums are zeros or the Gaussian's tails: those are divided at 2^64 times their size.
+__device__ __forceinline__ float blur_mean(float c, float wsum) {
+    if (wsum < 0.0001f) return 0.0f;
+    const bool tiny = fabsf(c) < 0x1p-60f, zero = c == 0.0f;
+    const float q = (zero ? wsum : (tiny ? c * 0x1p64f : c)) / wsum;
+    return zero ? c : (tiny ? q * 0x1p-64f : q);
+}
 __device__ __forceinline__ bool not_finite(float a, float b, float c) {
     return !(fabsf(a) < INFINITY && fabsf(b) < INFINITY && fabsf(c) < INFINITY);
 }
@@ -118,14 +156,15 @@ __device__ __noinline__ bool blur_x_all_taps(const float4* __restrict__ src, flo
 
 // blurX of one segment (kXSeg pixels) of a row per block, into one plane per channel.  The thresholded pixels of
 // the segment and its `near` neighbours lie in shared memory, a plane per channel (zeros stand for taps
-// outside the image and below the threshold); a thread sums kXOut neighbouring outputs of a channel from a
-// register window, so a tap costs kXOut FMAs, one shared load and a quarter of a weight load (kXOut is
+// outside the image and below the threshold); a warp has a channel of a quarter of the segment (four warps that
+// took the channels in turn left a small image's few blocks waiting: 671x296 at radius 0.86, 43 us a call, 34 us
+// so), and a thread sums kXOut neighbouring outputs from a register window, so a tap costs kXOut FMAs, one shared load and a quarter of a weight load (kXOut is
 // odd: the threads' windows start in different banks).  A warp's outputs go through shared memory to leave
 // in full lines.  The pixels that only taps of weight zero reach are read for values that are not finite.
 // SHARED false: a kernel too wide for a block's shared memory, every tap read from memory.  Bound by the FP32
 // issue rate.
 template <bool SHARED>
-__global__ void __launch_bounds__(kXThreads, 8) k_blur_x(const float4* __restrict__ in, float* __restrict__ out, int W, int H, int pitch,
+__global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restrict__ in, float* __restrict__ out, int W, int H, int pitch,
                                                          size_t plane, BloomTaps t, float threshold, int* __restrict__ flags) {
     extern __shared__ float row[];
     const int y = (int)(blockIdx.x % (unsigned)H), seg = (int)(blockIdx.x / (unsigned)H);
@@ -133,17 +172,15 @@ __global__ void __launch_bounds__(kXThreads, 8) k_blur_x(const float4* __restric
     const int stride = xe - xs + 2 * t.near + 2 * kXStep;   // plane length: from pixel xs - near, and zeros behind
     const float4* src = in + (size_t)y * W;
     float* dst = out + (size_t)y * pitch;
-    const float wsum = *t.sum;
     bool bad = !SHARED;
     if (SHARED) {
-        for (int j = threadIdx.x; j < stride; j += blockDim.x) {
+#pragma unroll 4
+        for (int j = threadIdx.x; j < stride; j += kXThreads) {
             const int x = xs + j - t.near;
             float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (x >= 0 && x < W) {
-                p = __ldg(src + x);
-                if (below(p, threshold)) p.x = p.y = p.z = 0.0f;
-                bad = bad || not_finite(p.x, p.y, p.z);
-            }
+            if (x >= 0 && x < W) p = __ldg(src + x);
+            if (below(p, threshold)) p.x = p.y = p.z = 0.0f;
+            bad = bad || not_finite(p.x, p.y, p.z);
             row[j] = p.x;
             row[stride + j] = p.y;
             row[2 * stride + j] = p.z;
@@ -156,22 +193,23 @@ __global__ void __launch_bounds__(kXThreads, 8) k_blur_x(const float4* __restric
             bad = bad || (!below(p, threshold) && not_finite(p.x, p.y, p.z));
         }
     }
+    wait_for_previous();   // the weights; the pixels above were there before the call's first kernel began
+    const float wsum = *t.sum;
     const int any_bad = __syncthreads_or(bad ? 1 : 0);
     bool flag = false;
     if (any_bad) {
         flag = blur_x_all_taps(src, dst, plane, W, xs, xe, t, threshold, wsum);
     } else {
         const int steps = (2 * t.near + 1 + kXStep - 1) / kXStep;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        float* stage = row + 3 * stride + warp * (32 * kXOut);
-        const int xw = xs + warp * (32 * kXOut);   // the warp's first output
-#pragma unroll 1
-        for (int ch = 0; ch < 3; ++ch) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = warp / 4;
+        float* stage = row + 3 * stride + warp * kXChunk;
+        const int x0 = (warp % 4) * kXChunk, xw = xs + x0;   // the warp's first output
+        if (xw < xe) {
             float acc[kXOut], win[kXStep];   // win[k % kXStep] holds v[k]
 #pragma unroll
             for (int r = 0; r < kXOut; ++r) acc[r] = 0.0f;
             if (xw + lane * kXOut < xe) {
-                const float* v = row + ch * stride + (int)threadIdx.x * kXOut;   // output r sums v[r + i] w[i], i in order
+                const float* v = row + ch * stride + x0 + lane * kXOut;   // output r sums v[r + i] w[i], i in order
                 const float4* w4 = reinterpret_cast<const float4*>(t.w);
 #pragma unroll
                 for (int r = 0; r < kXOut; ++r) win[r] = v[r];
@@ -256,6 +294,7 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
     const int x = (int)(blockIdx.x % cols) * 32 + lane;
     const int yb = (int)(blockIdx.x / cols) * (kYOut * kYWarps);
     const int y0 = yb + warp * kYOut;
+    wait_for_previous();
     const float wsum = *t.sum;
     // rows that a tap of this block reaches and that hold a value that is not finite
     bool bad = false;
@@ -263,23 +302,29 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
     for (int y = f0 + (int)threadIdx.x; y <= f1; y += blockDim.x)
         bad = bad || __ldg(flags + (size_t)((x - lane) / kXSeg) * H + y) != 0;
     const int any_bad = __syncthreads_or(bad ? 1 : 0);
-    float cr[kYOut], cg[kYOut], cb[kYOut];
-#pragma unroll
-    for (int r = 0; r < kYOut; ++r) cr[r] = cg[r] = cb[r] = 0.0f;
+    // the sums of a thread's outputs, [output][channel][thread] over the ring once it is read: the epilogue then loops
+    // (unrolled over the outputs with their divisions it had a small image wait on instruction fetches)
+    float* sums = &ring[0][0] + threadIdx.x;
+    constexpr int kSumCh = 32 * kYWarps;
+    static_assert(sizeof(ring) >= sizeof(float) * kYOut * 3 * kSumCh);
     if (any_bad) {
         if (x < W) {
-#pragma unroll
-            for (int r = 0; r < kYOut; ++r) {
-                if (y0 + r >= H) break;
+#pragma unroll 1
+            for (int r = 0; r < kYOut && y0 + r < H; ++r) {
                 const float3 c = blur_all_taps(y0 + r, H, t, t.w + kYOut + t.near, [&](int i, float3& v) {
                     const float* p = blurred_x + (size_t)(y0 + r + i) * pitch + x;
                     v = make_float3(__ldg(p), __ldg(p + plane), __ldg(p + 2 * plane));
                     return true;
                 });
-                cr[r] = c.x; cg[r] = c.y; cb[r] = c.z;
+                sums[(3 * r + 0) * kSumCh] = c.x;
+                sums[(3 * r + 1) * kSumCh] = c.y;
+                sums[(3 * r + 2) * kSumCh] = c.z;
             }
         }
     } else {
+        float cr[kYOut], cg[kYOut], cb[kYOut];
+#pragma unroll
+        for (int r = 0; r < kYOut; ++r) cr[r] = cg[r] = cb[r] = 0.0f;
         // chunk c: rows [yb - near + kYRows c, + kYRows); those with a row of the image only
         const int base = yb - t.near;
         const int c0 = base < 0 ? -base / kYRows : 0;
@@ -333,15 +378,22 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
             }
             __syncthreads();
         }
+#pragma unroll
+        for (int r = 0; r < kYOut; ++r) {
+            sums[(3 * r + 0) * kSumCh] = cr[r];
+            sums[(3 * r + 1) * kSumCh] = cg[r];
+            sums[(3 * r + 2) * kSumCh] = cb[r];
+        }
     }
     if (x >= W) return;
-#pragma unroll
-    for (int r = 0; r < kYOut; ++r) {
-        if (y0 + r >= H) break;
+    const int rows = min(kYOut, H - y0);
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
         const size_t i = (size_t)(y0 + r) * W + x;
-        const float4 o = orig[i];
-        const float3 c = make_float3(o.x + blur_mean(cr[r], wsum) * intensity, o.y + blur_mean(cg[r], wsum) * intensity,
-                                     o.z + blur_mean(cb[r], wsum) * intensity);
+        const float4 o = __ldg(orig + i);
+        const float3 c = make_float3(o.x + blur_mean(sums[(3 * r + 0) * kSumCh], wsum) * intensity,
+                                     o.y + blur_mean(sums[(3 * r + 1) * kSumCh], wsum) * intensity,
+                                     o.z + blur_mean(sums[(3 * r + 2) * kSumCh], wsum) * intensity);
         if (combined) combined[i] = make_float4(c.x, c.y, c.z, 1.0f);
         const float3 m = aces_fitted(make_float3(c.x * exposure_scale, c.y * exposure_scale, c.z * exposure_scale));
         out[i] = make_uchar4(to_unorm8(m.x), to_unorm8(m.y), to_unorm8(m.z), 255);
@@ -388,22 +440,21 @@ void postprocess(PostWorkspace& ws, const float* d_accum, int W, int H, const Bl
     int* flags = reinterpret_cast<int*>(ty.w + yw);
     const float4* accum = reinterpret_cast<const float4*>(d_accum);
     k_bloom_weights<<<2, kPostBlock, 0, st>>>(tx, ty, (int)xw, (int)yw, bloom.radius);
+    check_cuda(cudaGetLastError(), "postprocess launch");
     float* ping = ws.ping.as<float>();
-    const size_t shared = sizeof(float) * (3 * ((size_t)std::min(W, kXSeg) + 2 * (size_t)tx.near + 2 * kXStep) + kXSeg);
+    const size_t shared = sizeof(float) * (3 * ((size_t)std::min(W, kXSeg) + 2 * (size_t)tx.near + 2 * kXStep) + 3 * kXSeg);
     const unsigned xblocks = (unsigned)segs * (unsigned)H;
     if (shared <= kXMaxShared) {
         if (shared > 48 * 1024)
             check_cuda(cudaFuncSetAttribute(k_blur_x<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXMaxShared),
                        "cudaFuncSetAttribute");
-        k_blur_x<true><<<xblocks, kXThreads, shared, st>>>(accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
+        launch_after(k_blur_x<true>, xblocks, kXThreads, shared, st, accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
     } else {
-        k_blur_x<false><<<xblocks, kXThreads, 0, st>>>(accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
+        launch_after(k_blur_x<false>, xblocks, kXThreads, 0, st, accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
     }
     const unsigned blocks = (unsigned)((W + 31) / 32) * (unsigned)((H + kYOut * kYWarps - 1) / (kYOut * kYWarps));
-    k_blur_y_tonemap<<<blocks, 32 * kYWarps, 0, st>>>(ping, pitch, plane, accum, reinterpret_cast<float4*>(d_combined),
-                                                      reinterpret_cast<uchar4*>(d_rgba8), W, H, ty, flags, bloom.intensity,
-                                                      exp2f(tm.exposure));
-    check_cuda(cudaGetLastError(), "postprocess launch");
+    launch_after(k_blur_y_tonemap, blocks, 32 * kYWarps, 0, st, ping, pitch, plane, accum, reinterpret_cast<float4*>(d_combined),
+                 reinterpret_cast<uchar4*>(d_rgba8), W, H, ty, flags, bloom.intensity, exp2f(tm.exposure));
 }
 
 }  // namespace rt
