@@ -73,8 +73,10 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
  *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
  *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and
- *            batches take wave_refill, whose default is the grid form (a 1920x1080 64-spp frame of that
- *            scene 318 ms grid against 352 ms cooperative, a 256x256 Cornell room 2.48 against 3.79 ms).
+ *            batches take wave_refill, where 0 and REINA_REFILL_GRID leave the form to the engine: cooperative
+ *            for flat scenes of 512 or more BVH nodes and for two-level calls of 2^20 or more paths, else the
+ *            grid form (1920x1080, 16 spp of that scene 75.3 ms grid, 48.8 ms cooperative; a 256x256 Cornell
+ *            room 1.36 against 1.85 ms); calls that return work counters run the grid form.
  *   trace_block: threads per block of the grid-form traversal kernels (ray cast, wavefront extend and
  *            shadow): 64, 128 or 256 (default 128).  Grid form only.
  *   trace_stack: shared-memory traversal stack entries per thread, 8, 12 or 16 (default 12); deeper
@@ -83,7 +85,8 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *   wave_paths: path slots of one wave of a batched render or frame (0 = REINA_DEFAULT_WAVE_PATHS);
  *            the path state costs 164 bytes per slot and wave in flight (wave_lanes): the waves run on
  *            streams of their own, so that one wave's last bounces (few long paths) overlap the next
- *            waves' first ones.  A wave holds any number of samples of a pixel of a NEE+MIS job and at
+ *            waves' first ones.  Cooperative waves (wave_refill) take the slots of all lanes and run one
+ *            after the other, since each fills the GPU by itself.  A wave holds any number of samples of a pixel of a NEE+MIS job and at
  *            most one of a job in the reference's mode; a batch gets no more slots than one wave can
  *            hold of it, rounded up to a power of two (at least 2^16); an engine already built with
  *            more slots than that (up to wave_paths) is reused.
@@ -105,7 +108,8 @@ typedef struct reina_tuning {
     uint32_t wave_lanes;         /* waves in flight in batched renders and frames, 1..16
                                   * (0 = REINA_DEFAULT_WAVE_LANES) */
     uint32_t wave_refill;        /* launch form of the wavefront extension and shadow kernels (frames,
-                                  * batches): like `refill`, but 0 = the default REINA_REFILL_GRID */
+                                  * batches): like `refill`, but 0 = the default REINA_REFILL_GRID, with which
+                                  * the engine chooses */
 } reina_tuning;
 /* REINA_ORDER_INPUT traces ray i on thread i.  REINA_ORDER_COHERENT first bins the rays by direction
  * octant and origin cell (Morton order on an 8^3 grid over the origins' bounds) and traces them in that
@@ -360,12 +364,12 @@ enum {
                                     * engine of the batched renders with the frame as its one job */
 };
 /* Without a flag a frame runs on the context's wave engine (reina_render_batch with one job): waves
- * of its samples (several per pixel in REINA_MODE_NEE_MIS, one per pixel in REINA_MODE_REINA), eight in
- * flight on their own streams (tuning.wave_lanes), each replayed from a CUDA graph — on the 1920x1080,
- * 64 spp, 12-bounce frame 0.32 s against 0.59 s pass by pass.  The three forms give the same images. */
+ * of its samples (several per pixel in REINA_MODE_NEE_MIS, one per pixel in REINA_MODE_REINA), each
+ * replayed from a CUDA graph and, in the grid form, overlapping on their own streams (tuning.wave_lanes).
+ * The three forms give the same images. */
 /* The grid-form traversal variant of a frame comes from the render autotune cache (REINA_AUTOTUNE_CACHED)
- * or the context's tuning; the cooperative form (the default) runs the extension and shadow kernels of
- * both the wave engine and the pass-by-pass form for flat scenes. */
+ * or the context's tuning; tuning.wave_refill says when the wave engine's extension and shadow kernels run
+ * cooperatively.  Pass by pass they do for flat scenes where it asks for that. */
 
 typedef struct reina_render_stats {
     uint64_t rays;               /* closest-hit rays traced (path segments) */

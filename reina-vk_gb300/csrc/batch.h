@@ -17,6 +17,8 @@
 namespace rt {
 
 constexpr uint32_t kMaxWaveSegments = 1024;
+constexpr size_t kBatchPathBytes = 164;   // path state and queues of a wave slot
+struct BatchLaunch;                       // the kernels' view of a wave (batch.cu)
 
 // Per-job data the kernels read (one table per wave, holding the jobs present in that wave).
 struct JobGpu {
@@ -103,17 +105,14 @@ public:
     // receive the jobs in the wave and the jobs whose last samples it holds.
     bool submit_wave(const std::vector<BatchJob*>& jobs, bool fifo, std::vector<BatchJob*>* members = nullptr,
                      std::vector<BatchJob*>* completed = nullptr);
-    bool lane_free() const { return !lanes_[submitted_ % lanes_.size()].pending; }
+    bool lane_free() const { return !lanes_[lane_index(submitted_)].pending; }
     bool pending() const { return retired_ < submitted_; }
     // Waits for the oldest wave in flight and adds its ray counts; throws on a device error flag.
     void wait_oldest();
     // Waits for every wave in flight without reading their results (error and shutdown paths).
     void drain();
-    // The lanes' next work waits for the work queued on `st` so far.
-    void order_after(cudaStream_t st);
-    // The work queued on `st` from now on waits for every wave submitted so far.
-    void order_before(cudaStream_t st);
-    // Runs waves until every job is resolved, as many in flight as the engine has lanes.  Ordered
+    // Runs waves until every job is resolved: waves of the lanes' slots, as many in flight as the engine has
+    // lanes, or (cooperative traversal, choose_form) waves of all lanes' slots one after the other.  Ordered
     // after the work queued on `st` before the call; returns with every wave complete and the work
     // queued on `st` afterwards ordered after them.
     void run_all(const std::vector<BatchJob*>& jobs, cudaStream_t st, bool fifo = false);
@@ -131,33 +130,58 @@ public:
     uint32_t waves() const { return waves_; }
 
 private:
-    struct GraphSlot {
+    // What the kernel sequence of a wave depends on.
+    struct Shape {
         uint32_t bounces = 0;
-        bool nee = false;
-        bool two = false;   // the wave holds a two-level scene
-        bool count = false; // counting kernels (traversal work)
+        uint32_t materials = 0;  // bit m: a scene of the wave has material m
+        bool nee = false;        // shadow rays may be cast
+        bool two = false;        // the wave holds a two-level scene
+        bool mixed = false;      // several jobs (cooperative form: each ray looks up its scene)
+        bool count = false;      // counting kernels (traversal work)
+        bool coop = false;       // cooperative traversal
+        uint32_t nodes = 0;      // most BVH8 nodes of a scene of the wave (not part of the sequence)
+        bool operator==(const Shape& o) const {
+            return bounces == o.bounces && materials == o.materials && nee == o.nee && two == o.two && mixed == o.mixed &&
+                   count == o.count && coop == o.coop;
+        }
+    };
+    struct GraphSlot {
+        Shape shape;
         cudaGraphExec_t exec = nullptr;
     };
     struct Lane {
-        DeviceBuffer paths;             // path state for the capacity's slots (+ job, pixel, sample, depth)
+        size_t index = 0;
         DeviceBuffer desc;              // header + segments + job table
         void* host_desc = nullptr;      // pinned staging of the descriptor
         uint32_t* host_counters = nullptr;   // pinned copy of the wave's counters
         cudaStream_t stream = nullptr;  // run_all's stream for this lane
         cudaEvent_t finished = nullptr; // after the lane's last finish kernel and resolves
         cudaEvent_t done = nullptr;     // after the lane's last counter copy
+        bool ordered = true;            // ordered after the caller's stream (run_all)
         bool pending = false;           // a wave whose counters are not collected yet
         std::vector<GraphSlot> graphs;  // captured wave bodies (pointers into this lane's buffers)
     };
     struct Packed {
         WaveHeader hdr;
-        bool any_nee = false, two = false, carries = false;
+        Shape shape;
+        bool carries = false;
         std::vector<BatchJob*> members, completed;
     };
     // Packs the next wave into the lane's host descriptor; hdr.count == 0 when nothing is left.
     Packed pack(const std::vector<BatchJob*>& jobs, bool fifo, Lane& L);
     // Descriptor upload + wave body (init and the bounce kernels) on `s`.
     void launch_body(Lane& L, const Packed& pk, cudaStream_t s);
+    void launch_sequence(const BatchLaunch& B, const Shape& w, cudaStream_t main, bool fork);
+    void launch_trace(const BatchLaunch& B, const Shape& w, bool extend, int cur, uint32_t* bounce, cudaStream_t st);
+    template <bool MIXED, bool TWO, bool COUNT>
+    void launch_coop(const BatchLaunch& B, bool extend, int cur, uint32_t* bounce, cudaStream_t st);
+    void choose_form(const std::vector<BatchJob*>& jobs);
+    size_t lane_index(uint64_t wave) const { return coop_ ? 0 : wave % lanes_.size(); }
+    Lane& lane_of(uint64_t wave) { return lanes_[lane_index(wave)]; }
+    size_t lane_bytes() const;
+    // Slots of one wave: a lane's, or all lanes' in the cooperative form.
+    uint32_t wave_slots() const { return coop_ ? capacity_ * (uint32_t)lanes_.size() : capacity_; }
+    BatchLaunch wave_view(const Lane& L) const;
     // Finish kernel, resolves of the completed jobs, counter copy on `s`.
     void launch_finish(Lane& L, const Packed& pk, cudaStream_t s);
     // Adds a synchronized lane's counters to the totals; throws on a device error flag.
@@ -175,9 +199,13 @@ private:
     uint32_t waves_ = 0;
     uint64_t submitted_ = 0, retired_ = 0;   // waves launched / waited for
     int blocks_ext_ = 0, blocks_shade_[5] = {0, 0, 0, 0, 0}, blocks_sh_ = 0, blocks_simple_ = 0;
-    int blocks_ext_two_ = 0, blocks_sh_two_ = 0;
-    int blocks_ext_cnt_ = 0, blocks_sh_cnt_ = 0, blocks_ext_two_cnt_ = 0, blocks_sh_two_cnt_ = 0;
+    int blocks_plain_[2][2][2] = {};       // grids of the default grid-form variant: [extend][two][count]
+    int blocks_coop_[2][2][2][2] = {};     // of the cooperative form: [extend][mixed][two][count]
     bool count_ = false;
+    DeviceBuffer paths_;                   // path state of all lanes
+    cudaEvent_t caller_ = nullptr;         // the caller's stream at run_all
+    bool coop_ = false;                    // form of the waves in flight (chosen while none is)
+    uint32_t wave_limit_ = UINT32_MAX;     // paths of one wave, where fewer than its slots are wanted
 };
 
 }  // namespace rt

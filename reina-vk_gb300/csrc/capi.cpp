@@ -746,11 +746,15 @@ static void render_batch(reina_ctx* ctx, const reina_render_job* jobs, uint32_t 
         acc[k] = count > 1 ? &acc_own[k] : &ctx->accum;
         smp[k] = count > 1 ? &smp_own[k] : &ctx->samples;
     }
+    // the jobs' pixel state is stream-ordered on the caller's stream: a cudaMalloc and cudaFree per job and call
+    // cost more than a small frame's launches
+    cudaMemPool_t pool;
+    check_cuda(cudaDeviceGetDefaultMemPool(&pool, ctx->device), "cudaDeviceGetDefaultMemPool");
     std::vector<rt::BatchJob*> ptrs(count);
     for (uint32_t k = 0; k < count; ++k) {
         const reina_render_job& j = jobs[k];
         const size_t px = (size_t)j.options.width * j.options.height;
-        rt::BatchEngine::prepare(bj[k]);
+        rt::BatchEngine::prepare(bj[k], pool, st);
         if (host) {
             acc[k]->reserve(px * 4 * sizeof(float));
             if (j.push_consts.sampleBatch > 0)

@@ -39,12 +39,16 @@ constexpr uint32_t kCoopChunk = 32;
 #ifndef RT_COOP_MINB
 #define RT_COOP_MINB 7
 #endif
-constexpr int kCoopMinBlocks = RT_COOP_MINB;
+#ifndef RT_COOP_BLOCK
+#define RT_COOP_BLOCK 128
+#endif
+constexpr int kCoopBlock = RT_COOP_BLOCK;   // threads per block; warps share nothing
+constexpr int kCoopMinBlocks = RT_COOP_MINB * 128 / kCoopBlock;
 // Blocks per SM of the two-level form, which keeps more state (5 blocks: 5 % slower; 7: the same, with spills).
 #ifndef RT_COOP_MINB_TWO
 #define RT_COOP_MINB_TWO 6
 #endif
-constexpr int kCoopMinBlocksTwo = RT_COOP_MINB_TWO;
+constexpr int kCoopMinBlocksTwo = RT_COOP_MINB_TWO * 128 / kCoopBlock;
 #ifndef RT_COOP_FLUSH
 #define RT_COOP_FLUSH 12
 #endif
@@ -55,6 +59,10 @@ constexpr uint32_t kFlushGroups = RT_COOP_FLUSH;   // groups (two triangles on a
 #define RT_COOP_VISITS 2
 #endif
 constexpr int kCoopVisits = RT_COOP_VISITS;
+#ifndef RT_COOP_VISITS_TWO
+#define RT_COOP_VISITS_TWO 1
+#endif
+constexpr int kCoopVisitsTwo = RT_COOP_VISITS_TWO;
 // Shared-memory stack entries per thread (deeper levels spill to local memory): what fits beside the lists.
 #ifndef RT_COOP_STACK
 #define RT_COOP_STACK 8
@@ -105,7 +113,7 @@ __device__ __forceinline__ CoopWarp<MIXED, TWO>& coop_warp() {
 }
 template <bool MIXED, bool TWO>
 constexpr size_t coop_shared_bytes() {
-    return (kTraceBlock / 32) * sizeof(CoopWarp<MIXED, TWO>) + kTraceBlock * kCoopStack * sizeof(uint2);
+    return (kCoopBlock / 32) * sizeof(CoopWarp<MIXED, TWO>) + kCoopBlock * kCoopStack * sizeof(uint2);
 }
 
 __device__ __forceinline__ uint32_t coop_ordered(float f) {
@@ -262,18 +270,18 @@ __device__ __noinline__ void coop_store_finished(uint32_t n_fin, const DeviceSce
 // tmax); with MIXED it also returns the item's scene (batched waves mix scenes), otherwise every item uses
 // `uniform`.  store(i, hit, valid) is called by all 32 lanes together with up to 32 finished items (valid
 // marks the lanes holding one).  `next` is the global fetch counter (zero at launch); a warp refills its idle
-// lanes once at most `refill_at` lanes still trace.  Requires blocks of kTraceBlock threads and
+// lanes once at most `refill_at` lanes still trace.  Requires blocks of kCoopBlock threads and
 // coop_shared_bytes() of dynamic shared memory.  Returns the device error bits of the warp's rays.  TWO: scenes may be two-level.  VISITS: node visits per lane between two rounds of the
 // warp's bookkeeping (the triangles found meanwhile are tested at the next flush, so the closest distance a
 // visit culls with may lag by up to VISITS - 1 visits: a few more nodes, same hits).
 template <bool ANY, bool COUNT, bool REFINE, bool MIXED, bool TWO, int SS = kCoopStack, uint32_t FLUSH = kFlushGroups,
-          int VISITS = kCoopVisits, class Load, class Store>
+          int VISITS = TWO ? kCoopVisitsTwo : kCoopVisits, class Load, class Store>
 __device__ __forceinline__ uint32_t coop_trace(const DeviceScene& uniform, uint32_t n, uint32_t* next, uint32_t refill_at,
                                                Load load, Store store, TraceCounters& cnt) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
-    constexpr int stride = kTraceBlock;
+    constexpr int stride = kCoopBlock;
     CoopWarp<MIXED, TWO>& S = coop_warp<MIXED, TWO>();
-    uint2* stack = reinterpret_cast<uint2*>(coop_shared + (kTraceBlock / 32) * sizeof(CoopWarp<MIXED, TWO>)) + threadIdx.x;
+    uint2* stack = reinterpret_cast<uint2*>(coop_shared + (kCoopBlock / 32) * sizeof(CoopWarp<MIXED, TWO>)) + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     uint2 spill[kTotalStack - SS];
     uint32_t err = 0;

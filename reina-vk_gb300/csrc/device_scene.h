@@ -46,6 +46,7 @@ struct DeviceScene {
     const uint8_t* has_tbn = nullptr;         // per object: 1 if the model supplied TBN data
     uint32_t instance_count = 0;
     uint32_t props_count = 0;
+    uint32_t material_mask = 0;               // bit m: an InstanceProperties record has material m
     // emissive sampling data (src/scene/Instances.cpp:129-191, packed as in :197-232)
     const EmissiveInstanceData* emissive = nullptr;
     const float* cdf_triangles = nullptr;
@@ -65,6 +66,11 @@ struct DeviceScene {
 };
 
 #if defined(__CUDACC__)
+// InstanceProperties index of triangle `prim` of instance `inst` of a two-level scene.
+__device__ __forceinline__ uint32_t instance_props(const DeviceScene& s, uint32_t inst, uint32_t prim) {
+    const InstanceGpu& g = s.instances[inst];
+    return g.face_base == 0xFFFFFFFFu ? g.props : s.face_props[g.face_base + (prim - g.first_prim)];
+}
 // Instance and InstanceProperties index of global triangle `prim`: the per-triangle tables of a flat
 // scene, or (two-level scenes, which keep no per-triangle tables) a binary search over the instances'
 // first triangles and the instance's material or per-face table.
@@ -81,8 +87,7 @@ __device__ __forceinline__ void prim_lookup(const DeviceScene& s, uint32_t prim,
         else hi = mid - 1;
     }
     inst = lo;
-    const InstanceGpu& g = s.instances[lo];
-    props = g.face_base == 0xFFFFFFFFu ? g.props : s.face_props[g.face_base + (prim - g.first_prim)];
+    props = instance_props(s, lo, prim);
 }
 __device__ __forceinline__ uint32_t prim_props_of(const DeviceScene& s, uint32_t prim) {
     uint32_t inst, props;

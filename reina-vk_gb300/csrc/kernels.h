@@ -17,10 +17,9 @@ constexpr int kTraceBlock = 128;
 // is the default: on the 1.3M-triangle ray cast closest hit 0.42 ms against 0.80 ms for the grid form, on 256
 // instances of a 20,480-triangle model (two-level) 0.93 against 1.48 ms.
 constexpr int kDefaultRefill = 8;
-// Launch form of the wavefront extension and shadow kernels (renders, batches, the server): the grid
-// form.  The cooperative form's refill costs more than it saves there, where a wave's queue holds many
-// paths per scene and rays of one bounce are coherent: 1920x1080 64-spp frame of the 1.3M-triangle scene
-// 318 ms grid against 352 ms cooperative (refill 8), 256x256 Cornell room 2.48 against 3.79 ms.
+// Launch form of the wavefront extension and shadow kernels (renders, batches, the server): 0, the pass-by-pass
+// engine's and the server's grid form, and the batch engine's own choice by scene and paths
+// (BatchEngine::choose_form, which holds the measurements).
 constexpr int kDefaultWaveRefill = 0;
 
 // Launch configuration of the traversal kernels: block size (64, 128, 256) and shared-memory stack
@@ -41,5 +40,8 @@ void launch_raycast(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_
 void launch_raycast_counters(const DeviceScene& s, const Ray* d_rays, uint64_t n, bool any,
                              unsigned long long* d_counters, uint32_t* d_err, uint32_t* d_next, int sm_count,
                              cudaStream_t st);
+
+// Writes a flat scene's per-triangle indices into the padding of its n triangle records (TriRecord).
+void tag_triangles(TriRecord* d_tris, uint32_t n, const uint32_t* d_prim_props, const uint32_t* d_prim_instance, cudaStream_t st);
 
 }  // namespace rt

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(BLOCK) k_extend_grid(RenderLaunch L, int cur) 
 
 // Cooperative persistent form (coop_trace.cuh): warps refill idle lanes from the queue; triangle tests
 // and hit refinement are spread over the warp.  Flat scenes.
-__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_extend(const __grid_constant__ RenderLaunch L, int cur) {
+__global__ void __launch_bounds__(kCoopBlock, kCoopMinBlocks) k_extend(const __grid_constant__ RenderLaunch L, int cur) {
     const PathState& ps = L.ps;
     const uint32_t n = ps.counters[kCntActive + cur];
     const uint32_t* q = ps.q_active[cur];
@@ -158,17 +158,19 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderLaunch 
             const V3 ro{ps.ox[p], ps.oy[p], ps.oz[p]};
             const V3 rd{ps.dx[p], ps.dy[p], ps.dz[p]};
             const uint32_t prim = ps.hprim[p];
-            const HitInfo h = hit_info(L.s, prim, ps.hu[p], ps.hv[p], rd);
+            const HitInfo h = hit_info<MAT == 4>(L.s, prim, ps.hu[p], ps.hv[p], rd);
             const InstanceProperties& pr = L.s.props[h.props];
             uint32_t rng = ps.rng[p];
             uint32_t flags = ps.flags[p];
             float acc = ps.acc[p];
             const bool inside = (flags & kFlagInside) != 0;
+            M3 tbn{};
+            if (MAT == 4) tbn = h.tbn;
             Vertex vx;
             if (MAT == 1) vx = shade_lambert(L.s, h, pr, rd, rng, inside, acc);
             else if (MAT == 2) vx = shade_metal(L.s, h, pr, rd, rng, inside, acc);
             else if (MAT == 3) vx = shade_dielectric(L.s, h, pr, ro, rd, rng, inside, acc);
-            else vx = shade_disney(L.s, h, pr, ro, rd, rng, inside, acc);
+            else vx = shade_disney(L.s, h, tbn, pr, ro, rd, rng, inside, acc);
             if (vx.skip) {
                 flags &= ~kFlagPrevNee;
             } else {
@@ -178,9 +180,9 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderLaunch 
                     V3 contrib = vx.emission;
                     if (nee) {
                         if ((flags & kFlagPrevNee) && (vx.emission.x != 0.0f || vx.emission.y != 0.0f || vx.emission.z != 0.0f))
-                            contrib = contrib * power_heuristic(ps.ppdf[p], light_pdf_sa(L.s, L.pc.totalEmissiveWeight, prim, ro, vx.newO));
+                            contrib = contrib * power_heuristic(ps.ppdf[p], light_pdf_sa(L.s, L.pc.totalEmissiveWeight, prim, h.inst, h.props, ro, vx.newO));
                         const bool do_nee = (MAT == 1 || MAT == 4) && L.s.emissive_count > 0;
-                        if (do_nee) emit = next_event(L.s, L.pc.totalEmissiveWeight, rng, MAT == 4, vx.newO, vx.n, vx.albedo, pr, h.tbn, rd, thr, sh);
+                        if (do_nee) emit = next_event(L.s, L.pc.totalEmissiveWeight, rng, MAT == 4, vx.newO, vx.n, vx.albedo, pr, tbn, rd, thr, sh);
                         flags = do_nee ? (flags | kFlagPrevNee) : (flags & ~kFlagPrevNee);
                         ps.ppdf[p] = vx.pdf;
                     }
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(BLOCK) k_shadow_grid(RenderLaunch L) {
 }
 
 // Cooperative persistent form of the shadow kernel (flat scenes).
-__global__ void __launch_bounds__(kBlock, kCoopMinBlocks) k_shadow(const __grid_constant__ RenderLaunch L) {
+__global__ void __launch_bounds__(kCoopBlock, kCoopMinBlocks) k_shadow(const __grid_constant__ RenderLaunch L) {
     const PathState& ps = L.ps;
     const uint32_t n = ps.counters[kCntShadow];
     TraceCounters c{0u, 0u};
@@ -364,14 +366,14 @@ __global__ void __launch_bounds__(kBlock) k_megakernel(RenderLaunch L) {
                     rad = rad + sky * thr;
                     break;
                 }
-                const HitInfo hi = hit_info(L.s, h.prim, h.u, h.v, rd);
+                const HitInfo hi = hit_info<true>(L.s, h.prim, h.u, h.v, rd);
                 const InstanceProperties& pr = L.s.props[hi.props];
                 const uint32_t mat = L.s.props_material[hi.props];
                 Vertex vx;
                 if (mat == 0) vx = shade_lambert(L.s, hi, pr, rd, rng, inside, acc);
                 else if (mat == 1) vx = shade_metal(L.s, hi, pr, rd, rng, inside, acc);
                 else if (mat == 2) vx = shade_dielectric(L.s, hi, pr, ro, rd, rng, inside, acc);
-                else vx = shade_disney(L.s, hi, pr, ro, rd, rng, inside, acc);
+                else vx = shade_disney(L.s, hi, hi.tbn, pr, ro, rd, rng, inside, acc);
                 const V3 ray_org = ro, ray_in = rd;
                 ro = vx.newO;
                 rd = vx.newD;
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(kBlock) k_megakernel(RenderLaunch L) {
                     V3 contrib = vx.emission;
                     if (nee) {
                         if (prev_nee && (vx.emission.x != 0.0f || vx.emission.y != 0.0f || vx.emission.z != 0.0f))
-                            contrib = contrib * power_heuristic(ppdf, light_pdf_sa(L.s, L.pc.totalEmissiveWeight, h.prim, ray_org, vx.newO));
+                            contrib = contrib * power_heuristic(ppdf, light_pdf_sa(L.s, L.pc.totalEmissiveWeight, h.prim, hi.inst, hi.props, ray_org, vx.newO));
                         const bool do_nee = (mat == 0 || mat == 3) && L.s.emissive_count > 0;
                         if (do_nee) {
                             ShadowRec sh;
@@ -513,8 +515,8 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
     L.samples = d_samples;
     L.refill = opt.trace.refill;
 
-    const int g_ext = cached_grid((const void*)k_extend, kBlock, sm_count, coop_shared_bytes<false, false>());
-    const int g_sh = cached_grid((const void*)k_shadow, kBlock, sm_count, coop_shared_bytes<false, false>());
+    const int g_ext = cached_grid((const void*)k_extend, kCoopBlock, sm_count, coop_shared_bytes<false, false>());
+    const int g_sh = cached_grid((const void*)k_shadow, kCoopBlock, sm_count, coop_shared_bytes<false, false>());
     const int g_shade[5] = {0, occupancy_blocks((const void*)k_shade<1>, sm_count),
                             occupancy_blocks((const void*)k_shade<2>, sm_count),
                             occupancy_blocks((const void*)k_shade<3>, sm_count),
@@ -544,7 +546,7 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
                 const int grid = cached_grid((const void*)k_extend_grid<kTraceBlock, kDefaultTraceStack, true>, kTraceBlock, sm_count);
                 k_extend_grid<kTraceBlock, kDefaultTraceStack, true><<<grid, kTraceBlock, 0, st>>>(L, cur);
             } else if (opt.trace.refill > 0) {
-                k_extend<<<g_ext, kBlock, coop_shared_bytes<false, false>(), st>>>(L, cur);
+                k_extend<<<g_ext, kCoopBlock, coop_shared_bytes<false, false>(), st>>>(L, cur);
             } else {
                 with_trace_variant(opt.trace, [&](auto B, auto S) {
                     const int grid = cached_grid((const void*)k_extend_grid<B.value, S.value, false>, B.value, sm_count);
@@ -561,7 +563,7 @@ static void launch_frame(const PathState& ps, const DeviceScene& s, const RtPush
                     const int grid = cached_grid((const void*)k_shadow_grid<kTraceBlock, kDefaultTraceStack, true>, kTraceBlock, sm_count);
                     k_shadow_grid<kTraceBlock, kDefaultTraceStack, true><<<grid, kTraceBlock, 0, st>>>(L);
                 } else if (opt.trace.refill > 0) {
-                    k_shadow<<<g_sh, kBlock, coop_shared_bytes<false, false>(), st>>>(L);
+                    k_shadow<<<g_sh, kCoopBlock, coop_shared_bytes<false, false>(), st>>>(L);
                 } else {
                     with_trace_variant(opt.trace, [&](auto B, auto S) {
                         const int grid = cached_grid((const void*)k_shadow_grid<B.value, S.value, false>, B.value, sm_count);

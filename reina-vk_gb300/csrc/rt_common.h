@@ -51,7 +51,9 @@ struct alignas(16) Bvh8Node {
 static_assert(sizeof(Bvh8Node) == 80, "BVH8 node must be 80 bytes");
 
 // Traversal triangle record, 48 bytes: world-space vertices and the global triangle id in v0.w (in a
-// two-level scene: the model's object-space vertices and the triangle's index within the model).
+// two-level scene: the model's object-space vertices and the triangle's index within the model).  The device copy
+// of a flat scene carries the triangle's InstanceProperties index in pad1 and its instance in pad2 (bits), so
+// that a hit is classified and shaded without two more table reads; they are 0 in the host copy.
 struct alignas(16) TriRecord {
     float v0x, v0y, v0z;
     uint32_t prim;

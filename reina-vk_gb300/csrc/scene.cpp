@@ -3,6 +3,7 @@
 #include "scene.h"
 
 #include "emissive.h"
+#include "kernels.h"
 
 #include <array>
 #include <chrono>
@@ -721,7 +722,13 @@ void Scene::upload() {
     up(d_tex_texels_, tex_texels_.data(), tex_texels_.size() * sizeof(uint32_t));
     up(d_tex_info_, tex_info_.data(), tex_info_.size() * sizeof(uint32_t));
 
+    if (!two_level_)
+        tag_triangles(d_tris_.as<TriRecord>(), (uint32_t)bvh_.tris.size(), d_prim_props_.as<uint32_t>(),
+                      d_prim_instance_.as<uint32_t>(), nullptr);
+    check_cuda(cudaStreamSynchronize(nullptr), "scene upload");   // before any other stream reads the records
+
     dev_ = DeviceScene{};
+    for (uint32_t m : props_material_) dev_.material_mask |= 1u << (m & 31u);
     dev_.nodes = d_nodes_.as<Bvh8Node>();
     dev_.tris = d_tris_.as<TriRecord>();
     dev_.node_count = (uint32_t)bvh_.nodes.size();

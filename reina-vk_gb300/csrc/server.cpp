@@ -13,7 +13,7 @@ namespace rt {
 namespace {
 constexpr size_t kPixelStateBytes = 24;   // per pixel: carried RNG, accumulatedDistance, sums, count
 constexpr size_t kImageBytes = 16;        // per pixel: RGBA32F
-constexpr size_t kPathBytes = 164;        // per wave slot of the batch engine
+constexpr size_t kPathBytes = kBatchPathBytes;   // per wave slot of the batch engine
 }  // namespace
 
 double Server::now() const {

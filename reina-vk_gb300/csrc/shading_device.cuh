@@ -57,7 +57,8 @@ __device__ __forceinline__ float rng_next(uint32_t& s) {
     s = s * 747796405u + 1u;
     uint32_t w = ((s >> ((s >> 28) + 4u)) ^ s) * 277803737u;
     w = (w >> 22) ^ w;
-    return __fdiv_rn(__uint2float_rn(w), 4294967295.0f);
+    // 4294967295.0f is 2^32 in float, so the reference's division is an exact scaling
+    return __fmul_rn(__uint2float_rn(w), 1.0f / 4294967296.0f);
 }
 
 // Per-path seed of the nee_mis mode: a murmur3-style finalizer over (pixel, sample, seed).
@@ -112,8 +113,8 @@ __device__ __forceinline__ float power_heuristic(float a, float b) { return a * 
 
 struct HitInfo {
     V3 pos, n, ng;
+    M3 tbn;           // tangent frame (hit_info<true> only)
     bool front;
-    M3 tbn;
     uint32_t props;
     uint32_t inst;
     uint32_t lp;      // triangle index within its model
@@ -123,10 +124,15 @@ struct HitInfo {
 // getObjectHitInfo (closestHitCommon.h.glsl:52-148).  The UV is reconstructed on demand by surface_uv()
 // (only textured materials read it).  Models without TBN data use the tangent frame (1,0,0), (0,1,0) and
 // the geometric normal at every vertex (the reference reads its TBN buffer unconditionally).
-__device__ __forceinline__ HitInfo hit_info(const DeviceScene& s, uint32_t prim, float bu, float bv, V3 rayDir) {
+// FRAME forms the tangent frame, which the Disney shader and the normal and bump maps use; the other hits do
+// without it (about 400 of the Lambertian kernel's 2,600 instructions a warp and 27 floats a hit).  One
+// function, because the frame has to keep the rounding it has beside the hit's other vectors: formed in a
+// function of its own its products contract into FMAs differently, and paths part from those bits.
+// `ii` and `pid` are the triangle's instance and InstanceProperties index (prim_lookup).
+template <bool FRAME>
+__device__ __forceinline__ HitInfo hit_info(const DeviceScene& s, uint32_t prim, uint32_t ii, uint32_t pid, float bu, float bv,
+                                            V3 rayDir) {
     HitInfo h;
-    uint32_t ii, pid;
-    prim_lookup(s, prim, ii, pid);
     const InstanceGpu& inst = s.instances[ii];
     h.inst = ii;
     h.props = pid;
@@ -149,43 +155,57 @@ __device__ __forceinline__ HitInfo hit_info(const DeviceScene& s, uint32_t prim,
                   m[8] * v.x + m[9] * v.y + m[10] * v.z};
     };
     const V3 ngo = norm3(cross3(v1 - v0, v2 - v0));
+    const bool have_tbn = s.tbn_indices != nullptr && s.has_tbn != nullptr && s.has_tbn[inst.object];
     V3 no = ngo;
     M3 t0, t1, t2;
-    const bool have_tbn = s.tbn_indices != nullptr && s.has_tbn != nullptr && s.has_tbn[inst.object];
-    if (have_tbn) {
-        auto ldm = [&](uint32_t k) {
-            const float* q = s.tbns + 9ull * s.tbn_indices[3 * lp + pr.tbnsIndicesOffset + k];
-            return M3{ld3(q), ld3(q + 3), ld3(q + 6)};
-        };
-        t0 = ldm(0);
-        t1 = ldm(1);
-        t2 = ldm(2);
-        if (pr.interpNormals) no = norm3(norm3(t0.c2) * b0 + norm3(t1.c2) * bu + norm3(t2.c2) * bv);
-    } else {
-        t0.c0 = t1.c0 = t2.c0 = V3{1.0f, 0.0f, 0.0f};
-        t0.c1 = t1.c1 = t2.c1 = V3{0.0f, 1.0f, 0.0f};
-        t0.c2 = t1.c2 = t2.c2 = ngo;
+    if (FRAME) {
+        if (have_tbn) {
+            auto ldm = [&](uint32_t k) {
+                const float* q = s.tbns + 9ull * s.tbn_indices[3 * lp + pr.tbnsIndicesOffset + k];
+                return M3{ld3(q), ld3(q + 3), ld3(q + 6)};
+            };
+            t0 = ldm(0);
+            t1 = ldm(1);
+            t2 = ldm(2);
+            if (pr.interpNormals) no = norm3(norm3(t0.c2) * b0 + norm3(t1.c2) * bu + norm3(t2.c2) * bv);
+        } else {
+            t0.c0 = t1.c0 = t2.c0 = V3{1.0f, 0.0f, 0.0f};
+            t0.c1 = t1.c1 = t2.c1 = V3{0.0f, 1.0f, 0.0f};
+            t0.c2 = t1.c2 = t2.c2 = ngo;
+        }
+    } else if (pr.interpNormals && have_tbn) {
+        auto normal_of = [&](uint32_t k) { return norm3(ld3(s.tbns + 9ull * s.tbn_indices[3 * lp + pr.tbnsIndicesOffset + k] + 6)); };
+        no = norm3(normal_of(0) * b0 + normal_of(1) * bu + normal_of(2) * bv);
     }
     h.n = norm3(m3(no));
     h.ng = norm3(m3(ngo));
     h.front = dot3(rayDir, h.ng) < 0.0f;
     h.n = faceforward3(h.n, rayDir, h.ng);
     h.ng = faceforward3(h.ng, rayDir, h.ng);
-    const V3 tangent = norm3(t0.c0 * b0 + t1.c0 * bu + t2.c0 * bv);
-    const V3 bitangent = norm3(t0.c1 * b0 + t1.c1 * bu + t2.c1 * bv);
-    const V3 normal = norm3(t0.c2 * b0 + t1.c2 * bu + t2.c2 * bv);
-    const float* nm = inst.nrm;
-    const V3 nN{nm[0] * normal.x + nm[1] * normal.y + nm[2] * normal.z, nm[3] * normal.x + nm[4] * normal.y + nm[5] * normal.z,
-                nm[6] * normal.x + nm[7] * normal.y + nm[8] * normal.z};
-    V3 wT = norm3(m3(tangent));
-    V3 wB = norm3(m3(bitangent));
-    V3 wN = norm3(nN);
-    wT = norm3(wT - wN * dot3(wN, wT));
-    wB = norm3(wB - wN * dot3(wN, wB));
-    wB = wB * -1.0f;
-    wN = wN * (h.front ? 1.0f : -1.0f);
-    h.tbn = M3{wT, wB, wN};
+    if (FRAME) {
+        const V3 tangent = norm3(t0.c0 * b0 + t1.c0 * bu + t2.c0 * bv);
+        const V3 bitangent = norm3(t0.c1 * b0 + t1.c1 * bu + t2.c1 * bv);
+        const V3 normal = norm3(t0.c2 * b0 + t1.c2 * bu + t2.c2 * bv);
+        const float* nm = inst.nrm;
+        const V3 nN{nm[0] * normal.x + nm[1] * normal.y + nm[2] * normal.z, nm[3] * normal.x + nm[4] * normal.y + nm[5] * normal.z,
+                    nm[6] * normal.x + nm[7] * normal.y + nm[8] * normal.z};
+        V3 wT = norm3(m3(tangent));
+        V3 wB = norm3(m3(bitangent));
+        V3 wN = norm3(nN);
+        wT = norm3(wT - wN * dot3(wN, wT));
+        wB = norm3(wB - wN * dot3(wN, wB));
+        wB = wB * -1.0f;
+        wN = wN * (h.front ? 1.0f : -1.0f);
+        h.tbn = M3{wT, wB, wN};
+    }
     return h;
+}
+
+template <bool FRAME>
+__device__ __forceinline__ HitInfo hit_info(const DeviceScene& s, uint32_t prim, float bu, float bv, V3 rayDir) {
+    uint32_t ii, pid;
+    prim_lookup(s, prim, ii, pid);
+    return hit_info<FRAME>(s, prim, ii, pid, bu, bv, rayDir);
 }
 
 // ---- textures ---------------------------------------------------------------------------------------
@@ -280,22 +300,26 @@ __device__ __forceinline__ float2 bump_mapping(const DeviceScene& s, int id, flo
 // out-of-[0,1] skip (UVCHECK: Lambertian, Disney), the normal map (tangent normal rgb * 2 - 1 with y
 // negated, through the hit's TBN) and the albedo texture with its alpha test (ALPHA: a < 0.999 and a
 // uniform draw above a skips the hit; dielectrics only tint).  Returns false when the hit is skipped;
-// `n` and `albedo` receive the shading normal and the albedo.
+// `n` and `albedo` receive the shading normal and the albedo.  `frame` is the hit's tangent frame, or null to
+// form it where a map needs it.
 template <bool UVCHECK, bool ALPHA>
 __device__ __forceinline__ bool apply_textures(const DeviceScene& s, const HitInfo& h, const InstanceProperties& pr, V3 rd,
-                                               uint32_t& rng, V3& n, V3& albedo) {
+                                               uint32_t& rng, V3& n, V3& albedo, const M3* frame = nullptr) {
     n = h.n;
     albedo = ld3(pr.albedo);
     if ((pr.textureID & pr.normalMapTexID & pr.bumpMapTexID) < 0) return true;   // all three unset
     float2 uv = surface_uv(s, pr, h);
     uv.x = uv.x - floorf(uv.x);
     uv.y = uv.y - floorf(uv.y);
-    if (pr.bumpMapTexID >= 0) uv = bump_mapping(s, pr.bumpMapTexID, uv, norm3(rd), h.tbn);
+    M3 tbn;
+    if (frame) tbn = *frame;
+    else if (pr.bumpMapTexID >= 0 || pr.normalMapTexID >= 0) tbn = hit_info<true>(s, s.instances[h.inst].first_prim + h.lp, h.inst, h.props, h.bu, h.bv, rd).tbn;
+    if (pr.bumpMapTexID >= 0) uv = bump_mapping(s, pr.bumpMapTexID, uv, norm3(rd), tbn);
     if (UVCHECK && (uv.x < 0.0f || uv.x > 1.0f || uv.y < 0.0f || uv.y > 1.0f)) return false;
     if (pr.normalMapTexID >= 0) {
         const float4 t = tex_sample<3>(s, pr.normalMapTexID, uv.x, uv.y);
         const V3 tn{t.x * 2.0f - 1.0f, -(t.y * 2.0f - 1.0f), t.z * 2.0f - 1.0f};
-        n = norm3(mul(h.tbn, tn));
+        n = norm3(mul(tbn, tn));
     }
     if (pr.textureID >= 0) {
         const float4 t = tex_sample<4>(s, pr.textureID, uv.x, uv.y);

@@ -39,7 +39,7 @@ __device__ __forceinline__ void reduce_counters(const TraceCounters& c, unsigned
 // Warp-cooperative persistent form (coop_trace.cuh): warps refill idle lanes once at most `refill_at` of
 // their lanes still trace; triangle tests and hit refinement are spread over the warp.
 template <bool ANY, bool COUNT, bool TWO>
-__global__ void __launch_bounds__(kTraceBlock, TWO ? kCoopMinBlocksTwo : kCoopMinBlocks)
+__global__ void __launch_bounds__(kCoopBlock, TWO ? kCoopMinBlocksTwo : kCoopMinBlocks)
     raycast_kernel(const __grid_constant__ DeviceScene scene, const Ray* __restrict__ rays, uint32_t n, Hit* __restrict__ hits,
                    unsigned long long* counters, uint32_t* err_flag, uint32_t* next, uint32_t refill_at) {
     TraceCounters c{0u, 0u};
@@ -73,9 +73,10 @@ __global__ void RT_TRACE_BOUNDS(BLOCK) raycast_kernel_grid(const Bvh8Node* __res
         const float4 a = __ldcs(rp), b = __ldcs(rp + 1);
         const TraceRay r = make_trace_ray(a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w);
         Hit h;
+        HitTail tail;
         uint32_t e = 0;
         if (node_count) {
-            e = traverse<ANY, COUNT, true, SS>(nodes, tris, r, stack + threadIdx.x, BLOCK, h, c);
+            e = traverse<ANY, COUNT, true, SS>(nodes, tris, r, stack + threadIdx.x, BLOCK, h, c, tail);
         } else {
             h.prim = kMiss; h.t = r.tmax; h.u = 0.0f; h.v = 0.0f;
         }
@@ -102,9 +103,10 @@ __global__ void __launch_bounds__(kTraceBlock, ANY ? 1 : 8) raycast_kernel_two_l
         const float4 a = __ldcs(rp), b = __ldcs(rp + 1);
         const TraceRay r = make_trace_ray(a.x, a.y, a.z, b.x, b.y, b.z, a.w, b.w);
         Hit h;
+        HitTail tail;
         uint32_t e = 0;
         if (sc.node_count) {
-            e = traverse_two_level<ANY, COUNT, true, kSmemStack>(sc, r, stack + threadIdx.x, kTraceBlock, h, c);
+            e = traverse_two_level<ANY, COUNT, true, kSmemStack>(sc, r, stack + threadIdx.x, kTraceBlock, h, c, tail);
         } else {
             h.prim = kMiss; h.t = r.tmax; h.u = 0.0f; h.v = 0.0f;
         }
@@ -246,7 +248,7 @@ template <bool ANY, bool COUNT, bool TWO>
 static int persistent_grid(int sm_count) {
     static const int per_sm = [] {   // initialised once, thread-safely (a function-local static)
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, raycast_kernel<ANY, COUNT, TWO>, kTraceBlock,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, raycast_kernel<ANY, COUNT, TWO>, kCoopBlock,
                                                       coop_shared_bytes<false, TWO>());
         return std::max(1, b);
     }();
@@ -256,10 +258,10 @@ static int persistent_grid(int sm_count) {
 template <bool ANY, bool COUNT, bool TWO>
 static void launch_coop(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_hits, unsigned long long* d_counters,
                         uint32_t* d_err, uint32_t* d_next, int sm_count, int refill, cudaStream_t st) {
-    const uint64_t needed = (n + kTraceBlock - 1) / kTraceBlock;
+    const uint64_t needed = (n + kCoopBlock - 1) / kCoopBlock;
     check_cuda(cudaMemsetAsync(d_next, 0, sizeof(uint32_t), st), "cudaMemsetAsync");
     const int grid = (int)std::min<uint64_t>(needed, (uint64_t)persistent_grid<ANY, COUNT, TWO>(sm_count));
-    raycast_kernel<ANY, COUNT, TWO><<<grid, kTraceBlock, coop_shared_bytes<false, TWO>(), st>>>(
+    raycast_kernel<ANY, COUNT, TWO><<<grid, kCoopBlock, coop_shared_bytes<false, TWO>(), st>>>(
         s, d_rays, (uint32_t)n, d_hits, d_counters, d_err, d_next, (uint32_t)(32 - refill));
 }
 
@@ -306,6 +308,23 @@ static void launch(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_h
     }
     if (s.inst_trav) launch_coop<ANY, false, true>(s, d_rays, n, d_hits, nullptr, d_err, d_next, sm_count, cfg.refill, st);
     else launch_coop<ANY, false, false>(s, d_rays, n, d_hits, nullptr, d_err, d_next, sm_count, cfg.refill, st);
+}
+
+// Writes a flat scene's per-triangle InstanceProperties and instance indices into its triangle records.
+__global__ void __launch_bounds__(256) k_tag_triangles(TriRecord* tris, uint32_t n, const uint32_t* __restrict__ prim_props,
+                                                       const uint32_t* __restrict__ prim_instance) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t prim = tris[i].prim;
+    if (prim >= n) return;
+    tris[i].pad1 = __uint_as_float(prim_props[prim]);
+    tris[i].pad2 = __uint_as_float(prim_instance[prim]);
+}
+
+void tag_triangles(TriRecord* d_tris, uint32_t n, const uint32_t* d_prim_props, const uint32_t* d_prim_instance, cudaStream_t st) {
+    if (n == 0) return;
+    k_tag_triangles<<<(n + 255u) / 256u, 256, 0, st>>>(d_tris, n, d_prim_props, d_prim_instance);
+    check_cuda(cudaGetLastError(), "triangle tagging");
 }
 
 bool valid_trace_config(const TraceConfig& c) {

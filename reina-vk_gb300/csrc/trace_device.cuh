@@ -417,16 +417,24 @@ __device__ __forceinline__ bool trav_step(const Bvh8Node* __restrict__ nodes, co
     return false;
 }
 
+// What a hit carries beside t, u and v: its instance (two-level scenes) and the two words that a flat scene's
+// triangle record keeps beside its vertices (TriRecord).
+struct HitTail {
+    uint32_t inst = 0, pad1 = 0, pad2 = 0;
+};
+
 // After the last step: a miss reports t = tmax; a hit gets its reported t, u, v refined (refine_hit).
 template <bool REFINE>
-__device__ __forceinline__ void trav_finish(const Bvh8Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
-                                            const TraceRay& r, const TravState& s, Hit& hit) {
-    (void)nodes;
+__device__ __forceinline__ void trav_finish(const TriRecord* __restrict__ tris, const TraceRay& r, const TravState& s, Hit& hit,
+                                            HitTail& tail) {
     if (hit.prim == kMiss) {
         hit.t = r.tmax;
     } else if (REFINE) {
         const float4* tp = reinterpret_cast<const float4*>(tris) + 3ull * s.best_rec;
-        refine_hit(r, __ldg(tp + 0), __ldg(tp + 1), __ldg(tp + 2), hit);
+        const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), c = __ldg(tp + 2);
+        refine_hit(r, a, b, c, hit);
+        tail.pad1 = __float_as_uint(b.w);
+        tail.pad2 = __float_as_uint(c.w);
     }
 }
 
@@ -435,14 +443,14 @@ __device__ __forceinline__ void trav_finish(const Bvh8Node* __restrict__ nodes, 
 template <bool ANY, bool COUNT, bool REFINE = true, int SS = kSmemStack>
 __device__ __forceinline__ uint32_t traverse(const Bvh8Node* __restrict__ nodes, const TriRecord* __restrict__ tris,
                                              const TraceRay& r, uint2* stack, int stride, Hit& hit,
-                                             TraceCounters& cnt) {
+                                             TraceCounters& cnt, HitTail& tail) {
     TravState s;
     trav_init(r, s, hit);
     uint2 spill[kTotalStack - SS];
     uint32_t err = 0;
     while (!trav_step<ANY, COUNT, SS>(nodes, tris, r, s, hit, stack, stride, spill, cnt, err)) {
     }
-    trav_finish<REFINE>(nodes, tris, r, s, hit);
+    trav_finish<REFINE>(tris, r, s, hit, tail);
     return err;
 }
 
@@ -475,7 +483,7 @@ __device__ __forceinline__ TraceRay instance_ray(const TraceRay& w, const Instan
 // Triangles are tested as soon as they are reached (no postponing).
 template <bool ANY, bool COUNT, bool REFINE = true, int SS = kSmemStack>
 __device__ __forceinline__ uint32_t traverse_two_level(const DeviceScene& sc, const TraceRay& wr, uint2* stack, int stride,
-                                                       Hit& hit, TraceCounters& cnt) {
+                                                       Hit& hit, TraceCounters& cnt, HitTail& tail) {
     const uint4* nptr = reinterpret_cast<const uint4*>(sc.nodes);
     const float4* tptr = reinterpret_cast<const float4*>(sc.tris);
     uint2 spill[kTotalStack - SS];
@@ -578,6 +586,7 @@ __device__ __forceinline__ uint32_t traverse_two_level(const DeviceScene& sc, co
         const TraceRay ri = instance_ray(wr, sc.inst_trav + best_inst);
         const float4* tp = tptr + 3ull * best_rec;
         refine_hit(ri, __ldg(tp + 0), __ldg(tp + 1), __ldg(tp + 2), hit);
+        tail.inst = best_inst;
     }
     return err;
 }
@@ -587,11 +596,17 @@ __device__ __forceinline__ uint32_t traverse_two_level(const DeviceScene& sc, co
 // launchers pick TWO = true when a scene of the launch is two-level.
 template <bool ANY, bool COUNT, bool REFINE = true, int SS = kSmemStack, bool TWO = false>
 __device__ __forceinline__ uint32_t trace_scene(const DeviceScene& sc, const TraceRay& r, uint2* stack, int stride, Hit& hit,
-                                                TraceCounters& cnt) {
+                                                TraceCounters& cnt, HitTail& tail) {
     if constexpr (TWO) {
-        if (sc.inst_trav) return traverse_two_level<ANY, COUNT, REFINE, SS>(sc, r, stack, stride, hit, cnt);
+        if (sc.inst_trav) return traverse_two_level<ANY, COUNT, REFINE, SS>(sc, r, stack, stride, hit, cnt, tail);
     }
-    return traverse<ANY, COUNT, REFINE, SS>(sc.nodes, sc.tris, r, stack, stride, hit, cnt);
+    return traverse<ANY, COUNT, REFINE, SS>(sc.nodes, sc.tris, r, stack, stride, hit, cnt, tail);
+}
+template <bool ANY, bool COUNT, bool REFINE = true, int SS = kSmemStack, bool TWO = false>
+__device__ __forceinline__ uint32_t trace_scene(const DeviceScene& sc, const TraceRay& r, uint2* stack, int stride, Hit& hit,
+                                                TraceCounters& cnt) {
+    HitTail tail;
+    return trace_scene<ANY, COUNT, REFINE, SS, TWO>(sc, r, stack, stride, hit, cnt, tail);
 }
 
 }  // namespace rt

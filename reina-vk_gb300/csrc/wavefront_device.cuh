@@ -24,6 +24,12 @@ namespace rt {
 #define RT_SHADE_MINB 4
 #endif
 constexpr int kShadeMinBlocks = RT_SHADE_MINB;
+// Lambertian, metal and dielectric, which do without a tangent frame: 6 blocks (84 registers) 1.53 ms for a
+// 256x256 room frame, 4 blocks 1.58 ms, 8 blocks 1.53 ms.
+#ifndef RT_SHADE_MINB_LIGHT
+#define RT_SHADE_MINB_LIGHT 6
+#endif
+constexpr int kShadeMinBlocksLight = RT_SHADE_MINB_LIGHT;
 
 
 // Checked build (compiled with -DRT_CHECKED): every queue position and path index the wavefront kernels
@@ -82,9 +88,9 @@ __device__ __forceinline__ void store_ray(const PathState& ps, uint32_t p, V3 o,
 // Shared pieces of the shade kernels.
 
 // Light pdf (solid angle) of reaching `p` on emissive triangle `prim` from `from` (emission MIS).
-__device__ __forceinline__ float light_pdf_sa(const DeviceScene& s, float total_w, uint32_t prim, V3 from, V3 p) {
-    uint32_t ii, pid;
-    prim_lookup(s, prim, ii, pid);
+// `ii` and `pid`: the triangle's instance and InstanceProperties index.
+__device__ __forceinline__ float light_pdf_sa(const DeviceScene& s, float total_w, uint32_t prim, uint32_t ii, uint32_t pid, V3 from,
+                                              V3 p) {
     const InstanceGpu& inst = s.instances[ii];
     if (!(inst.light_weight > 0.0f)) return 0.0f;
     const InstanceProperties& pr = s.props[pid];
@@ -289,22 +295,22 @@ __device__ __forceinline__ Vertex shade_dielectric(const DeviceScene& s, const H
 }
 
 // disney.rchit.glsl:36-198
-__device__ __forceinline__ Vertex shade_disney(const DeviceScene& s, const HitInfo& h, const InstanceProperties& pr,
+__device__ __forceinline__ Vertex shade_disney(const DeviceScene& s, const HitInfo& h, const M3& tbn, const InstanceProperties& pr,
                                                V3 ro, V3 rd, uint32_t& rng, bool inside, float& acc) {
     Vertex v;
     v.skip = false;
     v.inside = inside;
     if (pr.cullBackface != 0u && !h.front) { skip_vertex(h, rd, v); return v; }
     V3 n, albedo;
-    if (!apply_textures<true, true>(s, h, pr, rd, rng, n, albedo)) { skip_vertex(h, rd, v); return v; }
+    if (!apply_textures<true, true>(s, h, pr, rd, rng, n, albedo, &tbn)) { skip_vertex(h, rd, v); return v; }
     const float eta = h.front ? 1.0f / pr.ior : pr.ior;
     const DisneyParams dp = disney_params(pr, albedo);
     bool didRefract = false, choseGlass = false;
     const V3 wi = -rd;
-    const V3 dir = sample_disney(h.tbn, dp, eta, n, wi, didRefract, choseGlass, rng);
+    const V3 dir = sample_disney(tbn, dp, eta, n, wi, didRefract, choseGlass, rng);
     const V3 hv = norm3(dir + wi);
     float pdf;
-    const V3 f = eval_disney(h.tbn, dp, eta, didRefract, n, wi, dir, hv, pdf);
+    const V3 f = eval_disney(tbn, dp, eta, didRefract, n, wi, dir, hv, pdf);
     const float cosI = fmaxf(dot3(n, dir), 0.0f);
     v.color = div3(f * cosI, pdf);
     v.albedo = albedo;
