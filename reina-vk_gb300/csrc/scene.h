@@ -126,7 +126,7 @@ private:
     std::vector<ModelData> models_;
     std::vector<ModelRange> ranges_;
     std::vector<float> all_vertices_, all_tbns_, all_tex_coords_;
-    std::vector<uint32_t> all_indices_offset_, all_tex_indices_offset_, all_tbns_indices_offset_, all_indices_non_offset_;
+    std::vector<uint32_t> all_indices_offset_, all_tex_indices_offset_, all_tbns_indices_offset_;
     // Instances
     std::vector<InstanceProperties> props_;
     std::vector<uint32_t> props_material_;
