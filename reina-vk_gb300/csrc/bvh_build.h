@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "bvh_sah.h"
+#include "errors.h"
 #include "rt_common.h"
 
 namespace rt {
@@ -50,11 +51,20 @@ constexpr uint32_t kMaxBvhDepth = 64;
 // Largest quantization exponent of a node (scale 2^e): the traversal forms 2^(e+15) in single precision.
 constexpr int kMaxQuantExponent = sah::kMaxQuantExponent;
 
+// What a device build reads and leaves on the device besides its host result.
+struct DeviceScene;
+struct DeviceBuild {
+    // in: a flat scene's uploaded tables; the triangles are its instances' in world space (`verts` is not read)
+    const DeviceScene* world = nullptr;
+    // out: bounds of the world-space triangles, and the nodes and triangle records as the traversal reads them
+    float lo[3], hi[3];
+    DeviceBuffer nodes, tris;
+    double kernel_seconds = 0.0;   // device time of the build kernels
+};
+
 // The same BVH8 built on the GPU `device` (bvh_gpu.cu): byte-identical nodes and triangle records for the
-// same input and options (SAH collapse only, at most 64 bins).  `kernel_seconds` receives the device
-// time of the build kernels.  Synchronous.
-Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const BvhBuildOptions& opt = BvhBuildOptions(),
-                       double* kernel_seconds = nullptr);
+// same input and options (SAH collapse only, at most 64 bins).  Synchronous.
+Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const BvhBuildOptions& opt, DeviceBuild& dev);
 constexpr int kMaxDeviceSahBins = 64;
 
 }  // namespace rt

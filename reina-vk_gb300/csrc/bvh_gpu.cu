@@ -31,6 +31,7 @@
 
 #include "bvh_build.h"
 #include "bvh_sah.h"
+#include "device_scene.h"
 #include "errors.h"
 
 namespace rt {
@@ -59,7 +60,8 @@ enum : uint32_t {
     kCtrWide = 5,        // wide nodes allocated
     kCtrMag = 6,         // largest |coordinate| (float bits)
     kCtrSite = 7,        // first failed access check: site << 24 | low 24 bits of the index
-    kCtrWords = 8
+    kCtrBox = 8,         // bounds of the triangles, order-preserving encodings: lo x, y, z, hi x, y, z
+    kCtrWords = 14
 };
 enum : uint32_t { kErrNonFinite = 1, kErrRange = 2, kErrInternal = 4 };
 enum : uint32_t { kModeLeaf = 0, kModeSplit = 1, kModeMedian = 2 };
@@ -126,8 +128,11 @@ __device__ __forceinline__ uint32_t ord(float f) {
     const uint32_t u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__device__ __forceinline__ float unord(uint32_t u) {
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
+__host__ __device__ __forceinline__ float unord(uint32_t u) {
+    u = (u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u;
+    float f;
+    memcpy(&f, &u, sizeof(f));
+    return f;
 }
 __device__ __forceinline__ float fmin_h(float acc, float v) { return v < acc ? v : acc; }   // std::min(acc, v)
 __device__ __forceinline__ float fmax_h(float acc, float v) { return acc < v ? v : acc; }   // std::max(acc, v)
@@ -356,6 +361,7 @@ __global__ void k_init(uint32_t* ctr, BNodeD* root, uint32_t n) {
     if (threadIdx.x != 0) return;
     for (int k = 0; k < (int)kCtrWords; ++k) ctr[k] = 0u;
     ctr[kCtrNodes] = 1u;
+    for (int k = 0; k < 3; ++k) ctr[kCtrBox + k] = 0xFFFFFFFFu;
     for (int k = 0; k < 3; ++k) {
         root->lo[k] = 0.0f;
         root->hi[k] = 0.0f;
@@ -365,31 +371,70 @@ __global__ void k_init(uint32_t* ctr, BNodeD* root, uint32_t n) {
     root->left = 0u;
 }
 
-// Primitive boxes, the identity permutation, the coordinate magnitude and the finiteness check.
-__global__ void __launch_bounds__(kBT) k_prims(const float* __restrict__ verts, uint32_t n, float4* plo, float4* phi,
+// Primitive boxes, the identity permutation, the coordinate magnitude and the finiteness check.  WORLD also
+// forms the triangles: those of a flat scene's instances in world space, with the host assembly's order of
+// roundings (scene.cpp, build_flat), and their bounds.  (On the host that loop took 3.7 of the 8.6 ms in which
+// a 327,680-triangle scene was built; here 12 us, the gathers and the records' stores.)
+template <bool WORLD>
+__global__ void __launch_bounds__(kBT) k_prims(DeviceScene sc, float* __restrict__ verts, uint32_t n, float4* plo, float4* phi,
                                                uint32_t* idx, uint32_t* ctr) {
+    __shared__ uint32_t block_box[7];   // bounds, magnitude
+    if (threadIdx.x < 7) block_box[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
     const uint32_t i = blockIdx.x * kBT + threadIdx.x;
-    if (i >= n) return;
-    const float* v = verts + 9ull * i;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     float mag = 0.0f;
     bool finite = true;
-    for (int j = 0; j < 3; ++j)
-        for (int k = 0; k < 3; ++k) {
-            const float x = v[3 * j + k];
-            finite = finite && isfinite(x);
-            lo[k] = fmin_h(lo[k], x);
-            hi[k] = fmax_h(hi[k], x);
-            mag = fmaxf(mag, fabsf(x));
+    if (i < n) {
+        float v[9];
+        if (WORLD) {
+            const InstanceGpu& inst = sc.instances[sc.prim_instance[i]];
+            const uint32_t* tri = sc.indices + 3ull * (i - inst.first_prim) + sc.props[sc.prim_props[i]].indicesOffset;
+            for (int j = 0; j < 3; ++j) {
+                const float4 p = *reinterpret_cast<const float4*>(sc.vertices + 4ull * tri[j]);
+                for (int r = 0; r < 3; ++r) {
+                    float s = __fmul_rn(inst.m[4 * r + 0], p.x);
+                    s = __fadd_rn(s, __fmul_rn(inst.m[4 * r + 1], p.y));
+                    s = __fadd_rn(s, __fmul_rn(inst.m[4 * r + 2], p.z));
+                    v[3 * j + r] = __fadd_rn(s, inst.m[4 * r + 3]);
+                }
+            }
+            for (int k = 0; k < 9; ++k) verts[9ull * i + k] = v[k];
+        } else {
+            for (int k = 0; k < 9; ++k) v[k] = verts[9ull * i + k];
         }
-    idx[i] = i;
-    plo[i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-    phi[i] = make_float4(hi[0], hi[1], hi[2], 0.0f);
-    if (!finite) {
-        atomicOr(&ctr[kCtrErr], kErrNonFinite);
-        return;
+        for (int j = 0; j < 3; ++j)
+            for (int k = 0; k < 3; ++k) {
+                const float x = v[3 * j + k];
+                finite = finite && isfinite(x);
+                lo[k] = fmin_h(lo[k], x);
+                hi[k] = fmax_h(hi[k], x);
+                mag = fmaxf(mag, fabsf(x));
+            }
+        idx[i] = i;
+        plo[i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+        phi[i] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        if (!finite) {
+            atomicOr(&ctr[kCtrErr], kErrNonFinite);
+            mag = 0.0f;
+        }
     }
-    atomicMax(&ctr[kCtrMag], __float_as_uint(mag));
+    // one atomic per block and word (one per thread on the same word took 30 us)
+    const uint32_t warp_mag = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(mag));
+    if (threadIdx.x % 32 == 0) atomicMax(&block_box[6], warp_mag);
+    if (WORLD) {
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, ord(lo[k])), h = __reduce_max_sync(0xFFFFFFFFu, ord(hi[k]));
+            if (threadIdx.x % 32 == 0) {
+                atomicMin(&block_box[k], l);
+                atomicMax(&block_box[3 + k], h);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 6) atomicMax(&ctr[kCtrMag], block_box[6]);
+    if (WORLD && threadIdx.x < 3) atomicMin(&ctr[kCtrBox + threadIdx.x], block_box[threadIdx.x]);
+    if (WORLD && threadIdx.x >= 3 && threadIdx.x < 6) atomicMax(&ctr[kCtrBox + threadIdx.x], block_box[threadIdx.x]);
 }
 
 // The per-level counters (large tasks, their items, large tasks of the next level).
@@ -1163,10 +1208,9 @@ inline uint32_t blocks_for(uint64_t n, int per_block) { return (uint32_t)((n + p
 
 }  // namespace
 
-Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const BvhBuildOptions& opt,
-                       double* kernel_seconds) {
+Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const BvhBuildOptions& opt, DeviceBuild& dev) {
     const auto t0 = std::chrono::steady_clock::now();
-    if (kernel_seconds) *kernel_seconds = 0.0;
+    dev.kernel_seconds = 0.0;
     if (tri_count == 0) return Bvh8{};
     if (tri_count >= 0x7FFFFFFFull) throw std::runtime_error("BVH build: too many triangles");
     if (opt.collapse != kCollapseSahDp) fail(REINA_ERR_INVALID, "device BVH build: only the SAH collapse is implemented");
@@ -1200,32 +1244,49 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     const uint32_t max_large = n / kSmall + 2;
     const uint32_t item = item_size(n);
     const uint32_t max_items = n / item + max_large + 2;
-    DeviceBuffer d_verts(9ull * n * sizeof(float)), d_plo(16ull * n), d_phi(16ull * n), d_idx(4ull * n), d_tmp(4ull * n),
-        d_nodes((size_t)max_nodes * sizeof(BNodeD)), d_ctr(kCtrWords * sizeof(uint32_t)),
-        d_large((size_t)max_large * sizeof(LargeTask)), d_items((size_t)max_items * sizeof(Item)),
-        d_lbins((size_t)max_large * 3 * kMaxBins * 7 * sizeof(uint32_t));
+    // one allocation for the build's tables (14 of them and their releases took 0.5 of the build's 4 ms)
+    const uint32_t wcap = n + 1;
+    size_t bytes = 0;
+    auto place = [&](size_t size) {
+        const size_t at = bytes;
+        bytes += (size + 255) / 256 * 256;
+        return at;
+    };
+    const size_t at_verts = place(9ull * n * sizeof(float)), at_plo = place(16ull * n), at_phi = place(16ull * n),
+                 at_idx = place(4ull * n), at_tmp = place(4ull * n), at_nodes = place((size_t)max_nodes * sizeof(BNodeD)),
+                 at_ctr = place(kCtrWords * sizeof(uint32_t)), at_large = place((size_t)max_large * sizeof(LargeTask)),
+                 at_items = place((size_t)max_items * sizeof(Item)),
+                 at_lbins = place((size_t)max_large * 3 * kMaxBins * 7 * sizeof(uint32_t)),
+                 at_dp = place((size_t)max_nodes * sizeof(sah::Dp)), at_w = place((size_t)wcap * sizeof(WideRec));
+    DeviceBuffer tables(bytes);
+    auto table = [&](size_t at) { return static_cast<void*>(tables.as<uint8_t>() + at); };
+    float* d_verts = static_cast<float*>(table(at_verts));
+    sah::Dp* d_dp = static_cast<sah::Dp*>(table(at_dp));
+    WideRec* d_w = static_cast<WideRec*>(table(at_w));
     // The vertices are the stream's first work; every later piece of state is written by kernels on the
     // stream, and counters are read back only after a stream synchronization, so that no copy from or to
     // pageable host memory is ever ordered against queued device work.
-    check_cuda(cudaMemcpyAsync(d_verts.get(), verts, 9ull * n * sizeof(float), cudaMemcpyHostToDevice, st), "H2D vertices");
+    if (!dev.world)
+        check_cuda(cudaMemcpyAsync(d_verts, verts, 9ull * n * sizeof(float), cudaMemcpyHostToDevice, st), "H2D vertices");
     check_cuda(cudaEventRecord(e0, st), "cudaEventRecord");
 
-    uint32_t* ctr = d_ctr.as<uint32_t>();
-    k_init<<<1, 32, 0, st>>>(ctr, d_nodes.as<BNodeD>(), n);
-    k_prims<<<blocks_for(n, kBT), kBT, 0, st>>>(d_verts.as<float>(), n, d_plo.as<float4>(), d_phi.as<float4>(),
-                                                d_idx.as<uint32_t>(), ctr);
+    Ctx c{};
+    float4 *plo = static_cast<float4*>(table(at_plo)), *phi = static_cast<float4*>(table(at_phi));
+    c.plo = plo;
+    c.phi = phi;
+    c.idx = static_cast<uint32_t*>(table(at_idx));
+    c.tmp = static_cast<uint32_t*>(table(at_tmp));
+    c.nodes = static_cast<BNodeD*>(table(at_nodes));
+    c.ctr = static_cast<uint32_t*>(table(at_ctr));
+    c.large = static_cast<LargeTask*>(table(at_large));
+    c.items = static_cast<Item*>(table(at_items));
+    c.lbins = static_cast<uint32_t*>(table(at_lbins));
+    uint32_t* ctr = c.ctr;
+    k_init<<<1, 32, 0, st>>>(ctr, c.nodes, n);
+    if (dev.world) k_prims<true><<<blocks_for(n, kBT), kBT, 0, st>>>(*dev.world, d_verts, n, plo, phi, c.idx, ctr);
+    else k_prims<false><<<blocks_for(n, kBT), kBT, 0, st>>>(DeviceScene{}, d_verts, n, plo, phi, c.idx, ctr);
     check_cuda(cudaGetLastError(), "BVH build: primitive boxes");
 
-    Ctx c{};
-    c.plo = d_plo.as<float4>();
-    c.phi = d_phi.as<float4>();
-    c.idx = d_idx.as<uint32_t>();
-    c.tmp = d_tmp.as<uint32_t>();
-    c.nodes = d_nodes.as<BNodeD>();
-    c.ctr = ctr;
-    c.large = d_large.as<LargeTask>();
-    c.items = d_items.as<Item>();
-    c.lbins = d_lbins.as<uint32_t>();
     c.max_large = max_large;
     c.max_items = max_items;
     c.max_nodes = max_nodes;
@@ -1247,6 +1308,10 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     read_ctr();
     float mag = 0.0f;
     std::memcpy(&mag, &h_ctr[kCtrMag], sizeof(float));
+    for (int k = 0; k < 3; ++k) {
+        dev.lo[k] = unord(h_ctr[kCtrBox + k]);
+        dev.hi[k] = unord(h_ctr[kCtrBox + 3 + k]);
+    }
 
     // Binary build, one level per iteration.
     std::vector<uint32_t> level_begin{0u, 1u};   // level L = nodes [level_begin[L], level_begin[L + 1])
@@ -1280,21 +1345,18 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     const uint32_t nb = le;
 
     // Collapse: dynamic programme bottom-up.
-    DeviceBuffer d_dp((size_t)nb * sizeof(sah::Dp));
     for (size_t L = level_begin.size() - 1; L-- > 0;) {
         const uint32_t a = level_begin[L], b = level_begin[L + 1];
-        if (b > a) k_dp<<<blocks_for(b - a, kBT), kBT, 0, st>>>(c.nodes, d_dp.as<sah::Dp>(), a, b, nb, ctr);
+        if (b > a) k_dp<<<blocks_for(b - a, kBT), kBT, 0, st>>>(c.nodes, d_dp, a, b, nb, ctr);
     }
     check_cuda(cudaGetLastError(), "BVH build: collapse");
 
     // Wide tree: records level by level from the root.
-    const uint32_t wcap = n + 1;
-    DeviceBuffer d_w((size_t)wcap * sizeof(WideRec));
-    k_init_wide<<<1, 32, 0, st>>>(d_w.as<WideRec>(), ctr);
+    k_init_wide<<<1, 32, 0, st>>>(d_w, ctr);
     std::vector<uint32_t> wlevel{0u, 1u};   // wide level L = records [wlevel[L], wlevel[L + 1])
     uint32_t wb = 0, we = 1;
     while (wb < we) {
-        k_wide_expand<<<blocks_for(we - wb, kBT), kBT, 0, st>>>(c.nodes, d_dp.as<sah::Dp>(), nb, d_w.as<WideRec>(), wb, we,
+        k_wide_expand<<<blocks_for(we - wb, kBT), kBT, 0, st>>>(c.nodes, d_dp, nb, d_w, wb, we,
                                                                ctr, wcap);
         check_cuda(cudaGetLastError(), "BVH build: wide level");
         read_ctr();
@@ -1307,16 +1369,17 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     if (depth > kMaxBvhDepth) throw std::runtime_error("BVH build: tree deeper than the traversal stack");
     for (size_t L = wlevel.size() - 1; L-- > 0;)
         if (wlevel[L + 1] > wlevel[L])
-            k_wide_sums<<<blocks_for(wlevel[L + 1] - wlevel[L], kBT), kBT, 0, st>>>(d_w.as<WideRec>(), wlevel[L],
+            k_wide_sums<<<blocks_for(wlevel[L + 1] - wlevel[L], kBT), kBT, 0, st>>>(d_w, wlevel[L],
                                                                                   wlevel[L + 1]);
     for (size_t L = 0; L + 1 < wlevel.size(); ++L)
         if (wlevel[L + 1] > wlevel[L])
-            k_wide_offsets<<<blocks_for(wlevel[L + 1] - wlevel[L], kBT), kBT, 0, st>>>(d_w.as<WideRec>(), wlevel[L],
+            k_wide_offsets<<<blocks_for(wlevel[L + 1] - wlevel[L], kBT), kBT, 0, st>>>(d_w, wlevel[L],
                                                                                      wlevel[L + 1]);
-    DeviceBuffer d_out_nodes((size_t)nw * sizeof(Bvh8Node)), d_out_tris((size_t)n * sizeof(TriRecord));
-    k_wide_emit<<<blocks_for(nw, kBT), kBT, 0, st>>>(c.nodes, d_dp.as<sah::Dp>(), nb, d_w.as<WideRec>(), nw, c.idx,
-                                                     d_verts.as<float>(), sah::quant_delta(mag), d_out_nodes.as<Bvh8Node>(),
-                                                     d_out_tris.as<TriRecord>(), n, ctr);
+    dev.nodes.alloc((size_t)nw * sizeof(Bvh8Node));
+    dev.tris.alloc((size_t)n * sizeof(TriRecord));
+    k_wide_emit<<<blocks_for(nw, kBT), kBT, 0, st>>>(c.nodes, d_dp, nb, d_w, nw, c.idx,
+                                                     d_verts, sah::quant_delta(mag), dev.nodes.as<Bvh8Node>(),
+                                                     dev.tris.as<TriRecord>(), n, ctr);
     check_cuda(cudaGetLastError(), "BVH build: emit");
     check_cuda(cudaEventRecord(e1, st), "cudaEventRecord");
     read_ctr();
@@ -1324,13 +1387,13 @@ Bvh8 build_bvh8_device(int device, const float* verts, uint64_t tri_count, const
     Bvh8 out;
     out.nodes.resize(nw);
     out.tris.resize(n);
-    check_cuda(cudaMemcpy(out.nodes.data(), d_out_nodes.get(), (size_t)nw * sizeof(Bvh8Node), cudaMemcpyDeviceToHost),
+    check_cuda(cudaMemcpy(out.nodes.data(), dev.nodes.get(), (size_t)nw * sizeof(Bvh8Node), cudaMemcpyDeviceToHost),
                "D2H nodes");
-    check_cuda(cudaMemcpy(out.tris.data(), d_out_tris.get(), (size_t)n * sizeof(TriRecord), cudaMemcpyDeviceToHost),
+    check_cuda(cudaMemcpy(out.tris.data(), dev.tris.get(), (size_t)n * sizeof(TriRecord), cudaMemcpyDeviceToHost),
                "D2H triangles");
     float ms = 0.0f;
     check_cuda(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
-    if (kernel_seconds) *kernel_seconds = ms * 1e-3;
+    dev.kernel_seconds = ms * 1e-3;
     out.depth = depth;
     out.binary_nodes = nb;
     out.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -414,14 +414,31 @@ bool Scene::use_two_level() const {
 // A triangle BVH on the host or on the scene's GPU (same bytes either way).
 Bvh8 Scene::build_triangles(const float* verts, uint64_t tri_count) {
     if (!bvh_device_) return build_bvh8(verts, tri_count, bvh_opt_);
-    double k = 0.0;
-    Bvh8 b = build_bvh8_device(device_, verts, tri_count, bvh_opt_, &k);
-    bvh_kernel_seconds_ += k;
+    DeviceBuild dev;
+    Bvh8 b = build_bvh8_device(device_, verts, tri_count, bvh_opt_, dev);
+    bvh_kernel_seconds_ += dev.kernel_seconds;
     return b;
 }
 
 // One BVH over all instances' world-space triangles.
 void Scene::build_flat() {
+    inst_trav_.clear();
+    tlas_refs_.clear();
+    blas_count_ = 0;
+    if (bvh_device_ && tri_total_ > 0) {   // from the uploaded tables, and the result stays on the device
+        upload_tables();
+        DeviceBuild dev;
+        dev.world = &dev_;
+        bvh_ = build_bvh8_device(device_, nullptr, tri_total_, bvh_opt_, dev);
+        bvh_kernel_seconds_ += dev.kernel_seconds;
+        for (int k = 0; k < 3; ++k) {
+            bounds_lo_[k] = dev.lo[k];
+            bounds_hi_[k] = dev.hi[k];
+        }
+        d_nodes_ = std::move(dev.nodes);
+        d_tris_ = std::move(dev.tris);
+        return;
+    }
     std::vector<float> world(9 * tri_total_);
     for (int k = 0; k < 3; ++k) { bounds_lo_[k] = INFINITY; bounds_hi_[k] = -INFINITY; }
     for (size_t ii = 0; ii < instances_.size(); ++ii) {
@@ -447,9 +464,6 @@ void Scene::build_flat() {
         }
     }
     bvh_ = build_triangles(world.data(), tri_total_);
-    inst_trav_.clear();
-    tlas_refs_.clear();
-    blas_count_ = 0;
 }
 
 // The reference's structure (src/scene/Scene.cpp:93-116; BLAS per model, src/graphics/Blas.cpp; TLAS
@@ -635,15 +649,6 @@ void Scene::build(bool require_emissive) {
             prim_props_[inst.first_prim + t] = inst.per_face ? inst.face_props[t] : inst.props_id;
         }
     }
-    try {
-        if (two_level_) build_two_level();
-        else build_flat();
-    } catch (const Error&) {
-        throw;
-    } catch (const std::exception& e) {
-        fail(REINA_ERR_INVALID, e.what());
-    }
-
     inst_gpu_.assign(instances_.size(), InstanceGpu{});
     uint32_t face_base = 0;
     for (size_t ii = 0; ii < instances_.size(); ++ii) {
@@ -667,6 +672,17 @@ void Scene::build(bool require_emissive) {
 
     has_tbn_.resize(models_.size());
     for (size_t o = 0; o < models_.size(); ++o) has_tbn_[o] = models_[o].tbn_indices.empty() ? 0 : 1;
+    try {
+        if (two_level_) build_two_level();
+        else build_flat();
+    } catch (const Error&) {
+        release_device();
+        throw;
+    } catch (const std::exception& e) {
+        release_device();
+        fail(REINA_ERR_INVALID, e.what());
+    }
+
     built_ = true;
     if (host_only) {   // host-only scenes keep the assembled buffers and the BVH, nothing is uploaded
         dev_ = DeviceScene{};
@@ -674,7 +690,8 @@ void Scene::build(bool require_emissive) {
         dev_.tri_count = (uint32_t)bvh_.tris.size();
         return;
     }
-    upload();
+    if (d_nodes_.bytes() != 0) finish_upload();   // a flat scene's device build left everything there
+    else upload();
 }
 
 size_t Scene::upload_bytes() const {
@@ -702,16 +719,11 @@ void Scene::release_device() {
     resident_ = false;
 }
 
-void Scene::upload() {
-    if (!built_) fail(REINA_ERR_STATE, "scene is not built");
-    if (device_ < 0) fail(REINA_ERR_STATE, "host-only scene cannot be uploaded");
-    if (resident_) return;
-    check_cuda(cudaSetDevice(device_), "cudaSetDevice");
+// The assembled buffers but for the BVH, and dev_'s view of them.
+void Scene::upload_tables() {
     // Upload (src/scene/Models.cpp:94-115 uploads the same arrays; an empty texcoord buffer gets one
     // float there and here so that the pointer stays valid).
     auto up = [](DeviceBuffer& b, const void* p, size_t bytes) { b.upload(p, bytes); };
-    up(d_nodes_, bvh_.nodes.data(), bvh_.nodes.size() * sizeof(Bvh8Node));
-    up(d_tris_, bvh_.tris.data(), bvh_.tris.size() * sizeof(TriRecord));
     up(d_vertices_, all_vertices_.data(), all_vertices_.size() * sizeof(float));
     up(d_indices_, all_indices_offset_.data(), all_indices_offset_.size() * sizeof(uint32_t));
     up(d_tbns_, all_tbns_.data(), all_tbns_.size() * sizeof(float));
@@ -735,17 +747,8 @@ void Scene::upload() {
     up(d_tex_texels_, tex_texels_.data(), tex_texels_.size() * sizeof(uint32_t));
     up(d_tex_info_, tex_info_.data(), tex_info_.size() * sizeof(uint32_t));
 
-    if (!two_level_)
-        tag_triangles(d_tris_.as<TriRecord>(), (uint32_t)bvh_.tris.size(), d_prim_props_.as<uint32_t>(),
-                      d_prim_instance_.as<uint32_t>(), nullptr);
-    check_cuda(cudaStreamSynchronize(nullptr), "scene upload");   // before any other stream reads the records
-
     dev_ = DeviceScene{};
     for (uint32_t m : props_material_) dev_.material_mask |= 1u << (m & 31u);
-    dev_.nodes = d_nodes_.as<Bvh8Node>();
-    dev_.tris = d_tris_.as<TriRecord>();
-    dev_.node_count = (uint32_t)bvh_.nodes.size();
-    dev_.tri_count = (uint32_t)bvh_.tris.size();
     dev_.vertices = d_vertices_.as<float>();
     dev_.indices = d_indices_.as<uint32_t>();
     dev_.tbns = d_tbns_.as<float>();
@@ -771,6 +774,30 @@ void Scene::upload() {
     dev_.tex_texels = d_tex_texels_.as<uint32_t>();
     dev_.tex_info = d_tex_info_.as<uint4>();
     dev_.tex_count = (uint32_t)textures_.size();
+    check_cuda(cudaStreamSynchronize(nullptr), "scene upload");   // before any other stream reads the tables
+}
+
+void Scene::upload() {
+    if (!built_) fail(REINA_ERR_STATE, "scene is not built");
+    if (device_ < 0) fail(REINA_ERR_STATE, "host-only scene cannot be uploaded");
+    if (resident_) return;
+    check_cuda(cudaSetDevice(device_), "cudaSetDevice");
+    upload_tables();
+    d_nodes_.upload(bvh_.nodes.data(), bvh_.nodes.size() * sizeof(Bvh8Node));
+    d_tris_.upload(bvh_.tris.data(), bvh_.tris.size() * sizeof(TriRecord));
+    finish_upload();
+}
+
+// The BVH (d_nodes_, d_tris_) joins the tables.
+void Scene::finish_upload() {
+    if (!two_level_)
+        tag_triangles(d_tris_.as<TriRecord>(), (uint32_t)bvh_.tris.size(), d_prim_props_.as<uint32_t>(),
+                      d_prim_instance_.as<uint32_t>(), nullptr);
+    check_cuda(cudaStreamSynchronize(nullptr), "scene upload");   // before any other stream reads the records
+    dev_.nodes = d_nodes_.as<Bvh8Node>();
+    dev_.tris = d_tris_.as<TriRecord>();
+    dev_.node_count = (uint32_t)bvh_.nodes.size();
+    dev_.tri_count = (uint32_t)bvh_.tris.size();
     for (int k = 0; k < 3; ++k) {
         dev_.bounds_lo[k] = bounds_lo_[k];
         dev_.bounds_hi[k] = bounds_hi_[k];

@@ -117,6 +117,8 @@ private:
     void pack_emissives(const std::vector<uint8_t>* same = nullptr);
     bool use_two_level() const;
     void build_flat();
+    void upload_tables();
+    void finish_upload();
     void build_two_level();
 
     int device_;
