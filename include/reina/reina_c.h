@@ -70,8 +70,8 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *   refill: the traversal launch form.  1..32 (0 = the default, 8): the warp-cooperative persistent form
  *            (block 128): warps keep 32 rays in flight, take new rays once `refill` of their lanes are idle,
  *            and share each step's triangle tests and the finished rays' hit refinement over all 32 lanes (at
- *            the default, casts of at most 224 rays per SM run eight lanes per ray instead: 1,000 rays of an
- *            81,920-triangle scene 26.6 us a call against 37.7 us);
+ *            the default, casts of at most 352 rays per SM run eight lanes per ray instead: 1,000 rays of an
+ *            81,920-triangle scene 25 us a call against 35 us);
  *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
  *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
  *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and

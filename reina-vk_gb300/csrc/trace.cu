@@ -87,11 +87,12 @@ __global__ void RT_TRACE_BOUNDS(BLOCK) raycast_kernel_grid(const Bvh8Node* __res
 }
 
 // Eight lanes per ray, for casts of few rays: what such a cast takes is the longest ray's chain of node visits (66 of
-// them among 128 rays of the 1.3M-triangle scene, about 0.6 us each), and a visit is shorter when a lane tests one
-// child box and then one of the node's triangles instead of eight boxes.  Up to four rays per warp, each group of eight
-// lanes holding its ray's state; the next node is on its way before the current one's triangles are tested.  (A
-// prefetch of the other hit children changed nothing; a lane testing its own child's triangles one after the other
-// was 5 to 10 % slower.)  No fetch counter, so no memset before the launch.  Same hits as the other forms: the
+// them among 128 rays of the 1.3M-triangle scene: 52 us cooperative, 40 us here), and a visit is shorter when a lane
+// tests one child box and then one of the node's triangles instead of eight boxes.  Up to four rays per warp, each
+// group of eight lanes holding its ray's state; the next node is on its way before the current one's triangles are
+// tested.  Bound by the visits' dependent instructions (about 180 of a warp, 4 to 5 cycles each) and a load's latency;
+// a prefetch of the other hit children changed nothing, a lane testing its own child's triangles one after the
+// other was 5 to 10 % slower.  No fetch counter, so no memset before the launch.  Same hits as the other forms: the
 // lowest (t, prim) among the triangles hit.
 constexpr int kWideBlock = 128;
 template <bool ANY, bool TWO>
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
                                                                  uint32_t n, Hit* __restrict__ hits, uint32_t* err_flag, uint32_t per_warp) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
     __shared__ uint2 stacks[kWideBlock / 8][kTotalStack];
-    const uint32_t lane = threadIdx.x & 31u, j = lane & 7u, shift = lane & 24u, group_lanes = 0xFFu << shift;
+    const uint32_t lane = threadIdx.x & 31u, j = lane & 7u, shift = lane & 24u;
     uint2* stack = stacks[threadIdx.x >> 3];
     const uint32_t in_warp = lane >> 3, i = ((blockIdx.x * kWideBlock + threadIdx.x) >> 5) * per_warp + in_warp;
     const bool valid = in_warp < per_warp && i < n;
@@ -120,6 +121,8 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
     uint32_t nx = 0, ny = 0, nz = 0, fx = 0, fy = 0, fz = 0, slot = 0;
     bool live = false;
 
+    // (The warp's lanes pop together, with full-mask barriers around the read: with a group's own mask each barrier
+    // costs a dozen instructions and a branch, 26.8 us against 24.7 for 1,000 rays.)
     auto push = [&](uint2 g) {
         if (sp < kTotalStack) {
             if (j == 0) stack[sp] = g;
@@ -130,44 +133,50 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
     };
     // The ray's next node, if it has one, on its way to the registers.
     auto advance = [&]() {
-        live = false;
-        for (;;) {
-            if (err) return;
-            if (group.y > 0x00FFFFFFu) break;
-            if (TWO && group.y != 0u) {   // enter the nearest pending instance
-                const uint32_t k = (uint32_t)__ffs(group.y) - 1u, ii = __ldg(sc.tlas_refs + group.x + k);
-                group.y &= group.y - 1u;
-                if (group.y) push(group);
-                group = make_uint2(0u, 0u);
-                const uint4 tail = __ldg(reinterpret_cast<const uint4*>(sc.inst_trav + ii) + 3);
-                if (tail.x != 0xFFFFFFFFu) {   // (a model without triangles has no bottom level)
-                    push(make_uint2(kLevelMarker, 0u));
-                    r = instance_ray(make_trace_ray(wo.x, wo.y, wo.z, wd.x, wd.y, wd.z, wo.w, wd.w), sc.inst_trav + ii);
-                    in_blas = true;
-                    inst = ii;
-                    first = tail.y;
-                    group = make_uint2(tail.x, 0x80000000u);
+        if (TWO) {   // up to a node group, through the ends of instances and into the next ones
+            for (;;) {
+                const bool enters = group.y != 0u && group.y <= 0x00FFFFFFu && !err, pops = group.y == 0u && sp != 0 && !err;
+                if (!__any_sync(kAll, enters || pops)) break;
+                if (pops) --sp;
+                __syncwarp();
+                if (pops) group = stack[sp];
+                __syncwarp();
+                if (pops && group.x == kLevelMarker && group.y == 0u) {   // back to the top level
+                    r = make_trace_ray(wo.x, wo.y, wo.z, wd.x, wd.y, wd.z, wo.w, wd.w);
+                    in_blas = false;
                 }
-                continue;
+                if (enters) {   // the nearest pending instance
+                    const uint32_t k = (uint32_t)__ffs(group.y) - 1u, ii = __ldg(sc.tlas_refs + group.x + k);
+                    group.y &= group.y - 1u;
+                    if (group.y) push(group);
+                    group = make_uint2(0u, 0u);
+                    const uint4 tail = __ldg(reinterpret_cast<const uint4*>(sc.inst_trav + ii) + 3);
+                    if (tail.x != 0xFFFFFFFFu) {   // (a model without triangles has no bottom level)
+                        push(make_uint2(kLevelMarker, 0u));
+                        r = instance_ray(make_trace_ray(wo.x, wo.y, wo.z, wd.x, wd.y, wd.z, wo.w, wd.w), sc.inst_trav + ii);
+                        in_blas = true;
+                        inst = ii;
+                        first = tail.y;
+                        group = make_uint2(tail.x, 0x80000000u);
+                    }
+                }
             }
-            if (sp == 0) return;
-            --sp;
-            __syncwarp(group_lanes);
-            group = stack[sp];
-            __syncwarp(group_lanes);
-            if (TWO && group.x == kLevelMarker && group.y == 0u) {   // back to the top level
-                r = make_trace_ray(wo.x, wo.y, wo.z, wd.x, wd.y, wd.z, wo.w, wd.w);
-                in_blas = false;
-            }
+        } else {
+            const bool pops = group.y == 0u && sp != 0;
+            if (pops) --sp;
+            __syncwarp();
+            if (pops) group = stack[sp];
+            __syncwarp();
         }
-        if (++steps > kMaxTraversalSteps) {
+        live = group.y > 0x00FFFFFFu && !err;
+        if (live && ++steps > kMaxTraversalSteps) {
             err |= kErrStepLimit;
-            return;
+            live = false;
         }
-        const uint32_t bit = 31u - __clz(group.y), child_slot = (bit - 24u) ^ r.oct_inv;
-        const uint32_t child = group.x + __popc(group.y & ((1u << child_slot) - 1u));
+        const uint32_t bit = 31u - __clz(group.y | 1u), child_slot = (bit - 24u) ^ r.oct_inv;
+        const uint32_t child = live ? group.x + __popc(group.y & ((1u << (child_slot & 31u)) - 1u)) : 0u;
         group.y &= ~(1u << bit);
-        if (group.y > 0x00FFFFFFu) push(group);
+        if (live && group.y > 0x00FFFFFFu) push(group);
         slot = j ^ r.oct_inv;   // lane j has the j-th child in the ray's order
         const uint8_t* p = nodes + 80ull * child;
         w0 = __ldg(reinterpret_cast<const uint4*>(p));
@@ -180,10 +189,10 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
         fy = __ldg(q + (by ? 8 : 32));
         nz = __ldg(q + (bz ? 40 : 16));
         fz = __ldg(q + (bz ? 16 : 40));
-        live = true;
     };
 
-    advance();
+    const bool empty = sc.node_count == 0;
+    if (!empty) advance();
     while (__any_sync(kAll, live)) {
         // this lane's child box, with the arithmetic of intersect_children
         const float sx = __uint_as_float(((w0.w & 0xFFu) + 15u) << 23) * r.idx, sy = __uint_as_float((((w0.w >> 8) & 0xFFu) + 15u) << 23) * r.idy,
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
         entries |= __shfl_xor_sync(kAll, entries, 2);
         entries |= __shfl_xor_sync(kAll, entries, 4);
         const uint32_t rec = w1.y + j;   // lane j tests entries j, j + 8 and j + 16
-        if (live) group = inner_mask ? make_uint2(w1.x, inner_mask << 24 | w0.w >> 24) : make_uint2(0u, 0u);
+        group = inner_mask ? make_uint2(w1.x, inner_mask << 24 | w0.w >> 24) : make_uint2(0u, 0u);
         if (TWO && live && !in_blas && entries) {   // instances first, the rest of the top level below them
             if (group.y > 0x00FFFFFFu) push(group);
             group = make_uint2(w1.y, entries);
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
         const TraceRay rt = r;
         const uint32_t tri_inst = inst, tri_first = first;
         const bool was_live = live;
-        if (live) advance();
+        advance();
         if (tests) {
             uint32_t key = ~0u, prim_mine = 0, rec_mine = 0;   // this lane's closest: ordered t, triangle
             float t_mine = 0.0f;
@@ -253,7 +262,10 @@ __global__ void __launch_bounds__(kWideBlock) raycast_kernel_wide(const __grid_c
                     best_prim = prim_low;
                     best_rec = rec_low;
                     best_inst = tri_inst;
-                    if (ANY) live = false;
+                    if (ANY) {
+                        live = false;
+                        sp = 0;
+                    }
                 }
             }
         }
@@ -498,14 +510,16 @@ static void launch(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_h
         if (scratch) check_cuda(cudaFreeAsync(scratch, st), "cudaFreeAsync");
         return;
     }
-    // The default form of few rays: eight lanes per ray as long as the chip is not full of them, two rays per warp while
-    // that leaves SMs with free slots (a warp takes as long as the longest of its rays).  Cooperative / wide, closest
-    // hit in us, 1,280 / 81,920 / 1,310,720 triangles / 64 instances of a 5,120-triangle model: 1,000 rays 22.7 / 35.0
-    // / 60.6 / 63.0 against 12.5 / 28.9 / 47.3 / 33.0 (four per warp 14.5 / 28.8 / 54.5 / 45.3); 10,000 rays four per warp
-    // 16.5 / 43.1 / 65.7 / 55.5, two 18.6 / 41.1 / 67.7 / 45.4; 34,400 rays 30.9 / 73.6 / 99.0 / 85.0 against 29.1 / 50.1
-    // / 67.6 / 66.5; 50,500 rays 33.4 against 41.3 on the small scene.
+    // The default form of few rays: eight lanes per ray until the chip is several times full of them, two rays per warp
+    // while that leaves SMs with free slots (a warp takes as long as the longest of its rays).  Cooperative against
+    // wide with four and with two rays per warp, closest hit, us a call:
+    //                        1,280 triangles   81,920            1,310,720         64 instances of 5,120
+    //     1,000 rays         22.9  12.1  10.5  35.1  24.7  24.8  61.5  43.3  39.1  63.0  39.1  29.9
+    //     10,000 rays        24.2  14.4  16.6  49.4  35.0  34.9  67.8  53.5  56.0  78.0  47.2  39.4
+    //     50,500 rays        33.9  32.1  45.0  73.5  52.1  68.2  86.9  67.1  83.0  90.4  63.8  83.2
+    //     80,000 rays        35.2  43.3  65.4  82.1  65.8  93.1   101  88.8   119   101  92.1   124
     const uint64_t sms = (uint64_t)std::max(1, sm_count);
-    if (cfg.refill == kDefaultRefill && n <= sms * 224) {
+    if (cfg.refill == kDefaultRefill && n <= sms * 352) {
         const uint32_t per_warp = n <= sms * 64 ? 2u : 4u;
         const unsigned blocks = (unsigned)((n + per_warp * (kWideBlock / 32) - 1) / (per_warp * (kWideBlock / 32)));
         if (s.inst_trav) raycast_kernel_wide<ANY, true><<<blocks, kWideBlock, 0, st>>>(s, d_rays, (uint32_t)n, d_hits, d_err, per_warp);
