@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "launch_chain.cuh"
 #include "post.h"
 
 namespace rt {
@@ -40,28 +41,6 @@ constexpr int kYStages = 3;
 static_assert(kXSeg % 32 == 0, "a Y block's columns lie in one X segment");
 constexpr int kWeightPart = 1024;   // weights summed from shared memory at a time
 constexpr size_t kXMaxShared = 200 * 1024;
-
-// The three kernels of a call are chained by programmatic launches, which take a launch's latency out of each gap
-// (671x296, radius 2: 27.8 us without, 22.8 us with): a kernel waits (wait_for_previous) before it reads what
-// the one before it wrote.  The first is launched plainly, so nothing of a call starts before the work ahead of it
-// on the stream is done, and it lets blurX start at once, whose blocks load their pixels meanwhile.  blurX does
-// not: blurY's blocks would fill the slots that blurX leaves on some SMs and crowd there (35 us).
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class... P, class... A>
-static void launch_after(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t shared, cudaStream_t st, A... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = shared;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "postprocess launch");
-}
 
 struct BloomTaps {
     int K, near;      // kernel half-width, and the half-width of its non-zero taps
@@ -439,6 +418,11 @@ void postprocess(PostWorkspace& ws, const float* d_accum, int W, int H, const Bl
     ty.w = tx.w + xw;
     int* flags = reinterpret_cast<int*>(ty.w + yw);
     const float4* accum = reinterpret_cast<const float4*>(d_accum);
+    // The three kernels of a call are chained by programmatic launches, which take a launch's latency out of each gap
+    // (671x296, radius 2: 27.8 us without, 22.8 us with): a kernel waits (wait_for_previous) before it reads what
+    // the one before it wrote.  The first is launched plainly, so nothing of a call starts before the work ahead of it
+    // on the stream is done, and it lets blurX start at once, whose blocks load their pixels meanwhile.  blurX does
+    // not: blurY's blocks would fill the slots that blurX leaves on some SMs and crowd there (35 us).
     k_bloom_weights<<<2, kPostBlock, 0, st>>>(tx, ty, (int)xw, (int)yw, bloom.radius);
     check_cuda(cudaGetLastError(), "postprocess launch");
     float* ping = ws.ping.as<float>();
