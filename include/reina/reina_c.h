@@ -70,15 +70,17 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *   refill: the traversal launch form.  1..32 (0 = the default, 8): the warp-cooperative persistent form
  *            (block 128): warps keep 32 rays in flight, take new rays once `refill` of their lanes are idle,
  *            and share each step's triangle tests and the finished rays' hit refinement over all 32 lanes (at
- *            the default, casts of at most 352 rays per SM run eight lanes per ray instead: 1,000 rays of an
- *            81,920-triangle scene 25 us a call against 35 us);
+ *            the default, casts of at most 192 rays per SM, 256 in scenes of 512 or more nodes and two-level ones, run
+ *            eight lanes per ray instead: 1,000 rays of an 81,920-triangle scene 25 us a call against 35 us);
  *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
  *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
  *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and
- *            batches take wave_refill, where 0 and REINA_REFILL_GRID leave the form to the engine: cooperative
- *            for flat scenes of 512 or more BVH nodes and for two-level calls of 2^20 or more paths, else the
- *            grid form (1920x1080, 16 spp of that scene 75.3 ms grid, 48.8 ms cooperative; a 256x256 Cornell
- *            room 1.36 against 1.85 ms); calls that return work counters run the grid form.
+ *            batches take wave_refill, where 0 and REINA_REFILL_GRID leave the form to the engine: eight
+ *            lanes per ray for calls of few paths (at most 96 per SM, 192 of a two-level scene, 352 of a flat
+ *            one of 512 or more nodes), above that cooperative for flat scenes of 512 or more nodes and for
+ *            two-level calls of 2^20 or more paths, else the grid form (1920x1080, 16 spp of that scene 75.3 ms
+ *            grid, 48.8 ms cooperative; a 256x256 Cornell room 1.36 against 1.85 ms); calls that return work
+ *            counters run the grid form.
  *   trace_block: threads per block of the grid-form traversal kernels (ray cast, wavefront extend and
  *            shadow): 64, 128 or 256 (default 128).  Grid form only.
  *   trace_stack: shared-memory traversal stack entries per thread, 8, 12 or 16 (default 12); deeper

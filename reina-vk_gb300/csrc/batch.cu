@@ -15,6 +15,7 @@
 #include "coop_trace.cuh"
 #include "trace_device.cuh"
 #include "wavefront_device.cuh"
+#include "wide_trace.cuh"
 
 namespace rt {
 
@@ -257,6 +258,35 @@ __global__ void __launch_bounds__(kCoopBlock, TWO ? kCoopMinBlocksTwo : kCoopMin
     if (COUNT) coop_add_counts(c, B.totals, kCntNodes, kCntTris);
 }
 
+// Eight lanes per ray (wide_trace.cuh), for waves of few paths; up to `pairs` rays go two to a warp.
+template <bool TWO>
+__global__ void __launch_bounds__(kWideBlock) kb_extend_wide(BatchLaunch B, const JobGpu* __restrict__ jobs, int cur, uint32_t* bounce,
+                                                            uint32_t pairs) {
+    __shared__ uint2 stacks[kWideBlock / 8 * kTotalStack];
+    const uint32_t n = bounce[kBncActive];
+    const uint32_t* q = B.active[cur];
+    count_rays(B.totals + kCntRays, n);
+    auto load = [&](uint32_t i, float4& o, float4& d) {
+        const uint32_t p = checked_index(q[i], B.P, B.totals + kCntError);
+        const PathRay& w = B.ray[p];
+        o = make_float4(w.ox, w.oy, w.oz, 0.0f);
+        d = make_float4(w.dx, w.dy, w.dz, 10000.0f);
+        return &jobs[w.tag & kJobMask].s;
+    };
+    auto store = [&](uint32_t i, const CoopHit& h, bool valid) {   // called by all 32 lanes
+        int m = -1;
+        uint32_t p = 0;
+        if (valid) {
+            p = checked_index(q[i], B.P, B.totals + kCntError);
+            m = store_hit(B, jobs[B.ray[p].tag & kJobMask].s, p, h.h, h.inst, h.pad1, h.pad2);
+        }
+        const uint32_t pos = append_by_queue(bounce + kBncQueue, m);
+        if (valid) *shade_entry(B, m, pos) = p;
+    };
+    const uint32_t e = wide_trace<false, true, TWO, true>(n, n <= pairs ? 2u : 4u, stacks, load, store);
+    if (e) atomicOr(B.totals + kCntError, e);
+}
+
 // One kernel per material queue (MAT = 1 Lambertian, 2 metal, 3 dielectric, 4 Disney): the closest-hit shader,
 // then the raygen loop body (raytrace.rgen.glsl:124-180).  `seg`: the bounce, which is also every path's depth.
 template <int MAT>
@@ -400,6 +430,26 @@ __global__ void __launch_bounds__(kCoopBlock, TWO ? kCoopMinBlocksTwo : kCoopMin
     const uint32_t e = coop_trace<true, COUNT, false, MIXED, TWO>(jobs[0].s, n, bounce + kBncFetchShadow, refill_at, load, store, c);
     if (e) atomicOr(B.totals + kCntError, e);
     if (COUNT) coop_add_counts(c, B.totals, kCntShadowNodes, kCntShadowTris);
+}
+
+// Eight lanes per shadow ray.
+template <bool TWO>
+__global__ void __launch_bounds__(kWideBlock) kb_shadow_wide(BatchLaunch B, const JobGpu* __restrict__ jobs, uint32_t* bounce,
+                                                            uint32_t pairs) {
+    __shared__ uint2 stacks[kWideBlock / 8 * kTotalStack];
+    const uint32_t n = bounce[kBncShadow];
+    count_rays(B.totals + kCntShadowRays, n);
+    auto load = [&](uint32_t i, float4& o, float4& d) {
+        const ShadowRay& w = B.shadow[i];
+        o = make_float4(w.ox, w.oy, w.oz, 0.0f);
+        d = make_float4(w.dx, w.dy, w.dz, w.tmax);
+        return &jobs[w.job].s;
+    };
+    auto store = [&](uint32_t i, const CoopHit& h, bool valid) {
+        if (valid && h.h.prim == kMiss) add_unoccluded(B, i);
+    };
+    const uint32_t e = wide_trace<true, false, TWO, true>(n, n <= pairs ? 2u : 4u, stacks, load, store);
+    if (e) atomicOr(B.totals + kCntError, e);
 }
 
 // raytrace.rgen.glsl:264-275 per pixel of each job in the wave: clamp (NaN kept), sample output, NaN
@@ -561,6 +611,7 @@ void BatchEngine::prepare(BatchJob& job, cudaMemPool_t pool, cudaStream_t st) {
     job.total = (uint64_t)job.pc.samplesPerPixel * px;
     job.cursor = 0;
     job.resolved = false;
+    job.placed.clear();
     if (pool) job.pixel_state.alloc_async(px * 6 * sizeof(uint32_t), pool, st);
     else job.pixel_state.alloc(px * 6 * sizeof(uint32_t));
 }
@@ -641,7 +692,11 @@ void BatchEngine::launch_coop(const BatchLaunch& B, bool extend, int cur, uint32
 }
 
 // The form of a call's waves: cooperative traversal where it was asked for (reina_tuning.wave_refill), else by
-// the jobs' scenes and paths.  (Counting waves without that request run the grid form, whose counts repeat from
+// the jobs' scenes and paths.  A call of few paths waits for each bounce's longest ray, so it traces with eight
+// lanes per ray (frames of 8 bounces with 4.6k / 12k / 30k / 46k paths, us, grid or cooperative against wide: 3 nodes
+// 268 / 271 / 285 / 303 against 223 / 258 / 322 / 410; zoo of 12 instances 962 / 995 / 1061 / 1096 against 656 / 788 /
+// 1036 / 1409; 64 instances 1275 / 1340 / 1428 / 1503 against 749 / 925 / 1231 / 1692; 82k triangles 743 / 789 / 851 / 894
+// against 492 / 521 / 601 / 703, and 63k paths 934 against 816).  (Counting waves without that request run the grid form, whose counts repeat from
 // run to run.)
 //
 // The cooperative kernels fill every SM until their queue is empty, so waves of that form run one after the other,
@@ -654,7 +709,9 @@ void BatchEngine::launch_coop(const BatchLaunch& B, bool extend, int cur, uint32
 //
 // Grid-form waves overlap: a call of more than a few paths per SM's thread is cut into three waves even where one
 // would hold it (1M paths: 1.54 ms as one wave, 1.36 as two, 1.39 as three; 1.4M of a two-level scene 6.40,
-// 5.91, 5.74; 64k paths: one is best).
+// 5.91, 5.74; 64k paths: one is best; 8 samples of the reference's mode, whose next sample of a pixel waits for
+// its last, over 360k / 491k / 922k pixels of the zoo 10.9 / 19.8 / 22.9 ms with a wave per sample, 10.8 / 17.6 /
+// 19.8 as three).
 void BatchEngine::choose_form(const std::vector<BatchJob*>& jobs) {
     constexpr uint32_t kCoopNodes = 512;
     constexpr uint64_t kCoopTwoLevelPaths = 1ull << 20;
@@ -668,7 +725,9 @@ void BatchEngine::choose_form(const std::vector<BatchJob*>& jobs) {
         nodes = std::max(nodes, j->scene.node_count);
         two = two || j->scene.inst_trav;
     }
-    coop_ = trace_.refill > 0 || (!count_ && (two ? paths >= kCoopTwoLevelPaths : nodes >= kCoopNodes));
+    const uint64_t wide_paths = (two ? 192ull : nodes >= kCoopNodes ? 352ull : 96ull) * sm_count_;
+    wide_ = trace_.refill == 0 && !count_ && paths <= wide_paths;
+    coop_ = trace_.refill > 0 || (!count_ && !wide_ && (two ? paths >= kCoopTwoLevelPaths : nodes >= kCoopNodes));
     wave_limit_ = UINT32_MAX;
     if (!coop_ && paths >= kOverlapPaths) {
         const uint64_t waves = std::max<uint64_t>(std::min<uint64_t>(kOverlapWaves, lanes_.size()), (paths + capacity_ - 1) / capacity_);
@@ -687,6 +746,16 @@ void BatchEngine::launch_trace(const BatchLaunch& B, const Shape& w, bool extend
         else if (w.mixed) by(std::true_type{}, std::false_type{});
         else if (w.two) by(std::false_type{}, std::true_type{});
         else by(std::false_type{}, std::false_type{});
+        return;
+    }
+    if (w.wide) {
+        const uint32_t pairs = wide_pair_limit(sm_count_);
+        auto by = [&](auto two) {
+            if (extend) kb_extend_wide<two.value><<<w.wide, kWideBlock, 0, st>>>(B, B.jobs, cur, bounce, pairs);
+            else kb_shadow_wide<two.value><<<w.wide, kWideBlock, 0, st>>>(B, B.jobs, bounce, pairs);
+        };
+        if (w.two) by(std::true_type{});
+        else by(std::false_type{});
         return;
     }
     // grid form: two-level scenes and counting waves run the default variant
@@ -772,6 +841,10 @@ void BatchEngine::launch_body(Lane& L, const Packed& pk, cudaStream_t st) {
     Shape w = pk.shape;
     w.count = count_;
     w.coop = coop_;
+    if (wide_) {   // blocks for the wave's first bounce, as a power of two (a graph is kept per shape)
+        w.wide = 1;
+        while (w.wide < (uint32_t)wide_blocks(h.count, h.count <= wide_pair_limit(sm_count_) ? 2u : 4u)) w.wide *= 2;
+    }
     if (!w.coop) w.mixed = false;   // (the grid form reads the job's scene per path either way)
     if (!use_graphs_) {
         launch_sequence(B, w, st, false);
@@ -869,8 +942,12 @@ BatchEngine::Packed BatchEngine::pack(const std::vector<BatchJob*>& jobs, bool f
     // A job's samples per pixel in one wave: any number when its samples are independent (NEE+MIS: seeded
     // by (pixel, sample); the finish kernel sums a pixel's samples of the wave in order); one in the
     // reference's mode, where a pixel's next sample starts from the state its previous one left.
-    auto cap = [](const BatchJob* j) -> uint64_t {
-        return j->opt.mode == kModeNeeMis ? UINT64_MAX : (uint64_t)j->opt.width * j->opt.height;
+    // Where waves are cut to overlap, such a job's do not cross from one sample into the next: with 3 waves a sample,
+    // each then waits for the third wave ahead of it, and not for the second.
+    auto cap = [&](const BatchJob* j) -> uint64_t {
+        if (j->opt.mode == kModeNeeMis) return UINT64_MAX;
+        const uint64_t px = (uint64_t)j->opt.width * j->opt.height;
+        return wave_limit_ == UINT32_MAX ? px : px - j->cursor % px;
     };
     std::vector<uint64_t> take(active.size(), 0);
     const uint64_t fair = fifo ? capacity : std::max<uint64_t>(1, capacity / active.size());
@@ -926,8 +1003,18 @@ BatchEngine::Packed BatchEngine::pack(const std::vector<BatchJob*>& jobs, bool f
         jt[ji].take = (uint32_t)placed;
         jt[ji].finish_start = finish;
         finish += (uint32_t)std::min(placed, px);
-        // samples after a pixel's first start from the state its previous sample left (reference mode)
-        pk.carries = pk.carries || (j->opt.mode != kModeNeeMis && c0 + placed > px);
+        // samples after a pixel's first start from the state its previous sample left (reference mode): the wave that
+        // holds the previous sample of the last pixel placed here, and with it those of the pixels before, comes first
+        if (j->opt.mode != kModeNeeMis && j->pc.samplesPerPixel > 1) {
+            const uint64_t end = c0 + placed;
+            if (end > px && !j->placed.empty()) {
+                size_t k = 0;
+                while (k + 1 < j->placed.size() && j->placed[k].first < end - px) ++k;
+                pk.after = std::max(pk.after, j->placed[k].second + 1);
+                j->placed.erase(j->placed.begin(), j->placed.begin() + (std::ptrdiff_t)k);
+            }
+            j->placed.emplace_back(end, submitted_);
+        }
         if (j->cursor == j->total && !j->resolved) {
             pk.completed.push_back(j);
             j->resolved = true;
@@ -956,7 +1043,10 @@ bool BatchEngine::submit_wave(const std::vector<BatchJob*>& jobs, bool fifo, std
     }
     Lane* prev = submitted_ > 0 ? &lane_of(submitted_ - 1) : nullptr;
     if (prev == &L) prev = nullptr;   // one lane: stream order already chains the waves
-    if (prev && pk.carries) check_cuda(cudaStreamWaitEvent(L.stream, prev->finished, 0), "cudaStreamWaitEvent");
+    if (pk.after > 0) {   // (a wave of this lane is ahead of this one on its stream)
+        Lane& D = lane_of(pk.after - 1);
+        if (&D != &L) check_cuda(cudaStreamWaitEvent(L.stream, D.finished, 0), "cudaStreamWaitEvent");
+    }
     launch_body(L, pk, L.stream);
     if (prev) check_cuda(cudaStreamWaitEvent(L.stream, prev->finished, 0), "cudaStreamWaitEvent");
     launch_finish(L, pk, L.stream);
@@ -985,6 +1075,7 @@ void BatchEngine::drain() {
 void BatchEngine::run_all(const std::vector<BatchJob*>& jobs, cudaStream_t st, bool fifo) {
     try {
         choose_form(jobs);
+        if (!pending()) submitted_ = retired_ = 0;   // from lane 0, whose graphs earlier calls have captured
         // each lane's first wave waits for the caller's work, and the caller's next work for the lanes used
         check_cuda(cudaEventRecord(caller_, st), "cudaEventRecord");
         for (Lane& L : lanes_) L.ordered = false;

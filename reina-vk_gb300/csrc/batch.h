@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime_api.h>
@@ -76,6 +77,7 @@ struct BatchJob {
     uint64_t total = 0;      // spp * W*H
     DeviceBuffer pixel_state;
     bool resolved = false;   // every sample is scheduled (set when the job's last wave is packed)
+    std::vector<std::pair<uint64_t, uint64_t>> placed;   // samples that carry state: end cursor and number of recent waves
     void* owner = nullptr;   // the caller's record of the job (the server's request)
 };
 
@@ -95,10 +97,10 @@ public:
     // Waves are packed from `jobs`: an equal share of the capacity per job with samples left, leftovers
     // to the first jobs (or, with `fifo`, each job in list order taking all it can use); a job in the
     // reference's mode places at most one sample of each pixel in a wave, a NEE+MIS job any number (the
-    // finish kernel sums each pixel's samples of the wave in sample order).  Wave k runs on lane k mod lanes, on the lane's own stream.  Each
-    // wave's finish kernel (the per-pixel sums) runs after the previous wave's, so a pixel's samples are
+    // finish kernel sums each pixel's samples of the wave in sample order).  Wave k runs on lane k mod
+    // lanes, on the lane's own stream.  Each wave's finish kernel (the per-pixel sums) runs after the previous wave's, so a pixel's samples are
     // summed in sample order; a wave holding a job whose samples carry state from the pixel's previous
-    // sample (the reference's seeding mode) starts only after the previous wave's finish.
+    // sample (the reference's seeding mode) starts only after the finish of the wave that holds that sample.
     //
     // Packs the next wave into the next lane, which must be free (lane_free()), and launches it.
     // Returns false when no job has samples left to schedule.  `members` and `completed` (optional)
@@ -139,10 +141,11 @@ private:
         bool mixed = false;      // several jobs (cooperative form: each ray looks up its scene)
         bool count = false;      // counting kernels (traversal work)
         bool coop = false;       // cooperative traversal
+        uint32_t wide = 0;       // traversal with eight lanes per ray: its blocks
         uint32_t nodes = 0;      // most BVH8 nodes of a scene of the wave (not part of the sequence)
         bool operator==(const Shape& o) const {
             return bounces == o.bounces && materials == o.materials && nee == o.nee && two == o.two && mixed == o.mixed &&
-                   count == o.count && coop == o.coop;
+                   count == o.count && coop == o.coop && wide == o.wide;
         }
     };
     struct GraphSlot {
@@ -164,7 +167,7 @@ private:
     struct Packed {
         WaveHeader hdr;
         Shape shape;
-        bool carries = false;
+        uint64_t after = 0;      // number + 1 of the wave whose finish the wave has to wait for, 0 for none
         std::vector<BatchJob*> members, completed;
     };
     // Packs the next wave into the lane's host descriptor; hdr.count == 0 when nothing is left.
@@ -205,6 +208,7 @@ private:
     DeviceBuffer paths_;                   // path state of all lanes
     cudaEvent_t caller_ = nullptr;         // the caller's stream at run_all
     bool coop_ = false;                    // form of the waves in flight (chosen while none is)
+    bool wide_ = false;                    // the waves trace with eight lanes per ray
     uint32_t wave_limit_ = UINT32_MAX;     // paths of one wave, where fewer than its slots are wanted
 };
 

@@ -124,3 +124,26 @@ def test_exported_triangles_hold_no_tags(R, ctx, level):
     _, tris = s.export_bvh()
     words = tris.view(np.uint32).reshape(-1, 12)
     assert not words[:, [7, 11]].any()
+
+
+@pytest.mark.parametrize("name,per_sm", [("few_nodes", 96), ("instanced", 192), ("nodes", 352)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_few_paths(R, ctx, built, name, per_sm, extra):
+    """As many paths as are traced with eight lanes per ray, and one column more."""
+    w = per_sm + extra
+    s = built[name]
+    want = samples(R, ctx, [(s, *frame(R, s, w, ctx.sm_count, 1, mode=0, pass_by_pass=True))])
+    for kw, got in forms(R, ctx, [(s, *frame(R, s, w, ctx.sm_count, 1, mode=0))]):
+        same(got, want, kw)
+
+
+@pytest.mark.parametrize("w,h,spp", [(520, 511, 3), (601, 600, 4), (512, 515, 2), (1, 262145, 2)])
+def test_carried_samples_in_cut_waves(R, ctx, built, w, h, spp):
+    """The reference's mode, whose samples of a pixel start from the state the last one left, in waves cut to overlap."""
+    s = built["few_nodes"]
+    want = samples(R, ctx, [(s, *frame(R, s, w, h, spp, 4, mode=0, pass_by_pass=True))])
+    for kw, got in forms(R, ctx, [(s, *frame(R, s, w, h, spp, 4, mode=0))]):
+        same(got, want, kw)
+    jobs = [(s, *frame(R, s, w, h, spp, 4, mode=0)), (built["instanced"], *frame(R, built["instanced"], 40, 30, 7, 3, mode=0))]
+    want += samples(R, ctx, [(jobs[1][0], *frame(R, jobs[1][0], 40, 30, 7, 3, mode=0, pass_by_pass=True))])
+    same(samples(R, ctx, jobs), want, "two jobs")

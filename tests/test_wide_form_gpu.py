@@ -43,8 +43,8 @@ def built(R, gpu_ctx):
     two.close()
 
 
-@pytest.mark.parametrize("per_sm,n", [(0, 1), (0, 2), (0, 3), (0, 7), (0, 8), (0, 9), (64, -1), (64, 0), (64, 1), (64, 3), (352, -1),
-                                      (352, 0), (352, 1)])
+@pytest.mark.parametrize("per_sm,n", [(0, 1), (0, 2), (0, 3), (0, 7), (0, 8), (0, 9), (64, -1), (64, 0), (64, 1), (64, 3), (192, 0),
+                                      (192, 1), (256, 0), (256, 1)])
 def test_counts(R, gpu_ctx, built, per_sm, n):
     n += per_sm * gpu_ctx.sm_count
     for scene in built:
