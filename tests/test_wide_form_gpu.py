@@ -1,6 +1,6 @@
-"""Casts of few rays (eight lanes per ray) against the grid form, bit for bit (any hit: the same hit or miss): ray
+"""Casts of few rays (eight lanes per ray, and above those cooperative with spread chunks) against the grid form, bit for bit (any hit: the same hit or miss): ray
 counts around the ends of a warp's and a block's groups, where two rays per warp become four, and where the
-cooperative form takes over; flat and two-level scenes; rays equal in t to several triangles."""
+cooperative form takes over and stops spreading; flat and two-level scenes; rays equal in t to several triangles."""
 import numpy as np
 import pytest
 
@@ -44,7 +44,7 @@ def built(R, gpu_ctx):
 
 
 @pytest.mark.parametrize("per_sm,n", [(0, 1), (0, 2), (0, 3), (0, 7), (0, 8), (0, 9), (64, -1), (64, 0), (64, 1), (64, 3), (192, 0),
-                                      (192, 1), (256, 0), (256, 1)])
+                                      (192, 1), (256, 0), (256, 1), (600, 0), (600, 1), (1280, -3), (1280, 1)])
 def test_counts(R, gpu_ctx, built, per_sm, n):
     n += per_sm * gpu_ctx.sm_count
     for scene in built:
