@@ -97,10 +97,11 @@ public:
     // Waves are packed from `jobs`: an equal share of the capacity per job with samples left, leftovers
     // to the first jobs (or, with `fifo`, each job in list order taking all it can use); a job in the
     // reference's mode places at most one sample of each pixel in a wave, a NEE+MIS job any number (the
-    // finish kernel sums each pixel's samples of the wave in sample order).  Wave k runs on lane k mod
-    // lanes, on the lane's own stream.  Each wave's finish kernel (the per-pixel sums) runs after the previous wave's, so a pixel's samples are
-    // summed in sample order; a wave holding a job whose samples carry state from the pixel's previous
-    // sample (the reference's seeding mode) starts only after the finish of the wave that holds that sample.
+    // finish kernel sums each pixel's samples of the wave in sample order).  Wave k runs on lane k mod lanes, on
+    // the lane's own stream.  Each wave's finish kernel (the per-pixel sums) runs after the previous wave's, so a
+    // pixel's samples are summed in sample order; a wave holding a job whose samples carry state from the
+    // pixel's previous sample (the reference's seeding mode) starts only after the finish of the wave that
+    // holds that sample.
     //
     // Packs the next wave into the next lane, which must be free (lane_free()), and launches it.
     // Returns false when no job has samples left to schedule.  `members` and `completed` (optional)
