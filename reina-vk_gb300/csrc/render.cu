@@ -370,9 +370,9 @@ __global__ void __launch_bounds__(kBlock) k_megakernel(RenderLaunch L) {
                 const InstanceProperties& pr = L.s.props[hi.props];
                 const uint32_t mat = L.s.props_material[hi.props];
                 Vertex vx;
-                if (mat == 0) vx = shade_lambert(L.s, hi, pr, rd, rng, inside, acc);
-                else if (mat == 1) vx = shade_metal(L.s, hi, pr, rd, rng, inside, acc);
-                else if (mat == 2) vx = shade_dielectric(L.s, hi, pr, ro, rd, rng, inside, acc);
+                if (mat == 0) vx = shade_lambert(L.s, hi, pr, rd, rng, inside, acc, &hi.tbn);
+                else if (mat == 1) vx = shade_metal(L.s, hi, pr, rd, rng, inside, acc, &hi.tbn);
+                else if (mat == 2) vx = shade_dielectric(L.s, hi, pr, ro, rd, rng, inside, acc, &hi.tbn);
                 else vx = shade_disney(L.s, hi, hi.tbn, pr, ro, rd, rng, inside, acc);
                 const V3 ray_org = ro, ray_in = rd;
                 ro = vx.newO;

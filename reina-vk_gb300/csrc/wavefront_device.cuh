@@ -215,13 +215,13 @@ __device__ __forceinline__ void skip_vertex(const HitInfo& h, V3 rd, Vertex& v) 
 
 // lambertian.rchit.glsl:11-78
 __device__ __forceinline__ Vertex shade_lambert(const DeviceScene& s, const HitInfo& h, const InstanceProperties& pr,
-                                                V3 rd, uint32_t& rng, bool inside, float& acc) {
+                                                V3 rd, uint32_t& rng, bool inside, float& acc, const M3* frame = nullptr) {
     Vertex v;
     v.skip = false;
     v.inside = inside;
     if (pr.cullBackface != 0u && !h.front) { skip_vertex(h, rd, v); return v; }
     V3 n, albedo;
-    if (!apply_textures<true, true>(s, h, pr, rd, rng, n, albedo)) { skip_vertex(h, rd, v); return v; }
+    if (!apply_textures<true, true>(s, h, pr, rd, rng, n, albedo, frame)) { skip_vertex(h, rd, v); return v; }
     v.color = albedo;
     v.albedo = v.color;
     v.emission = ld3(pr.emission);
@@ -236,13 +236,13 @@ __device__ __forceinline__ Vertex shade_lambert(const DeviceScene& s, const HitI
 
 // metal.rchit.glsl:7-70
 __device__ __forceinline__ Vertex shade_metal(const DeviceScene& s, const HitInfo& h, const InstanceProperties& pr,
-                                              V3 rd, uint32_t& rng, bool inside, float& acc) {
+                                              V3 rd, uint32_t& rng, bool inside, float& acc, const M3* frame = nullptr) {
     Vertex v;
     v.skip = false;
     v.inside = inside;
     if (pr.cullBackface != 0u && !h.front) { skip_vertex(h, rd, v); return v; }
     V3 n, albedo;
-    if (!apply_textures<false, true>(s, h, pr, rd, rng, n, albedo)) { skip_vertex(h, rd, v); return v; }
+    if (!apply_textures<false, true>(s, h, pr, rd, rng, n, albedo, frame)) { skip_vertex(h, rd, v); return v; }
     v.color = albedo;
     v.albedo = v.color;
     v.emission = ld3(pr.emission);
@@ -258,7 +258,7 @@ __device__ __forceinline__ Vertex shade_metal(const DeviceScene& s, const HitInf
 // dielectric.rchit.glsl:40-113 (the Fresnel term uses the unperturbed normal; the normal map bends the
 // reflected and refracted directions; the albedo texture tints without an alpha test)
 __device__ __forceinline__ Vertex shade_dielectric(const DeviceScene& s, const HitInfo& h, const InstanceProperties& pr,
-                                                   V3 ro, V3 rd, uint32_t& rng, bool inside, float& acc) {
+                                                   V3 ro, V3 rd, uint32_t& rng, bool inside, float& acc, const M3* frame = nullptr) {
     Vertex v;
     v.skip = false;
     const float ri = h.front ? 1.0f / pr.ior : pr.ior;
@@ -269,7 +269,7 @@ __device__ __forceinline__ Vertex shade_dielectric(const DeviceScene& s, const H
     const float refl = reflectance(cosT, ri);
     const bool prevInside = inside;
     V3 n, albedo;
-    apply_textures<false, false>(s, h, pr, rd, rng, n, albedo);
+    apply_textures<false, false>(s, h, pr, rd, rng, n, albedo, frame);
     v.inside = inside;
     if (cannot || refl > rng_next(rng)) {
         v.newD = fuzzy_reflection(unitDir, n, pr.roughness, rng);
