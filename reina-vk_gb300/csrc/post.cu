@@ -5,8 +5,8 @@
 // The reference's kernel has kernelSize = int(radiusPx * 3 + 0.5) taps on each side.  Its sums run over the taps
 // in order (so do these), a NaN or infinite pixel spreads over the whole kernel as it does there, and the
 // sum of the weights counts out-of-image and thresholded taps (blurCommon.h.glsl:24-31).
-// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.144 ms, against 1.558 ms with a thread
-// per pixel that summed every tap; 671x296, radius 0.86: 21 us against 36 us.
+// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.152 ms, against 1.558 ms with a thread
+// per pixel that summed every tap; 671x296, radius 0.86: 24 us against 36 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,8 +21,10 @@ constexpr int kPostBlock = 256;
 
 // gauss(x, sigma) = exp(-x^2 / (2 sigma^2)) is exactly 0 in float beyond |x| = sqrt(2 * 104) |sigma| (exp(-104) is
 // below half of the smallest subnormal): such taps add p * 0 to the sums, which changes them only where p
-// is not finite.  The passes below therefore sum the `near` taps, |i| <= near, and take the kernel's whole
-// width only where a row or column range holds a value that is not finite.
+// is not finite.  The passes below therefore sum the `near` taps, |i| <= near, of the finite values (the others stand
+// as zeros), and blocks that another value reaches add those to the sums afterwards, over the kernel's whole width
+// (one NaN pixel: 1920x1080 at radius 5 0.163 ms, 0.602 ms when such blocks summed every tap; 320x200 at radius 9
+// 50 us against 111 us).
 static int near_taps(int K, float sigma) {
     const double reach = std::ceil(14.45 * std::fabs((double)sigma)) + 1.0;
     return reach < (double)K ? (int)reach : K;   // (a NaN sigma keeps K)
@@ -96,56 +98,63 @@ __device__ __forceinline__ bool not_finite(float a, float b, float c) {
     return !(fabsf(a) < INFINITY && fabsf(b) < INFINITY && fabsf(c) < INFINITY);
 }
 
-// One output of either pass, tap by tap over the kernel's whole width as the reference sums them.  fetch(i)
-// gives the pixel of tap i and whether it counts.
-template <class Fetch>
-__device__ __forceinline__ float3 blur_all_taps(int at, int end, const BloomTaps& t, const float* w_at0, Fetch fetch) {
-    float cr = 0.0f, cg = 0.0f, cb = 0.0f;
-    const int i0 = max(-t.K, -at), i1 = min(t.K, end - 1 - at);
-    for (int i = i0; i <= i1; ++i) {
-        float3 p;
-        if (!fetch(i, p)) continue;
-        const float wgt = i < -t.near || i > t.near ? 0.0f : w_at0[i];
-        cr += p.x * wgt;
-        cg += p.y * wgt;
-        cb += p.z * wgt;
-    }
-    return make_float3(cr, cg, cb);
-}
-
 __device__ __forceinline__ bool below(const float4& p, float threshold) {
     return p.x * 0.299f + p.y * 0.587f + p.z * 0.114f < threshold;
 }
 
-// Outputs [x0, x1) of a row of blurX with a thread per output and every tap; returns whether one is not finite.
-__device__ __noinline__ bool blur_x_all_taps(const float4* __restrict__ src, float* __restrict__ dst, size_t plane, int W, int x0,
-                                             int x1, const BloomTaps& t, float threshold, float wsum) {
-    bool flag = false;
-    for (int x = x0 + (int)threadIdx.x; x < x1; x += blockDim.x) {
-        const float3 c = blur_all_taps(x, W, t, t.w + t.near, [&](int i, float3& v) {
-            const float4 p = __ldg(src + x + i);
-            v = make_float3(p.x, p.y, p.z);
-            return !below(p, threshold);
-        });
-        const float3 m = make_float3(blur_mean(c.x, wsum), blur_mean(c.y, wsum), blur_mean(c.z, wsum));
-        flag = flag || not_finite(m.x, m.y, m.z);
-        dst[x] = m.x;
-        dst[plane + x] = m.y;
-        dst[2 * plane + x] = m.z;
+// What the values that a warp left out of its sums (they are not finite) add to them: to every output they reach, at
+// weight zero NaN.  stage: the warp's sums of channel ch for the pixels from xw on.  (This function and its like for
+// blurY stay out of line: inlined they cost every block a microsecond of instruction fetches.)
+__device__ __noinline__ void add_not_finite_x(float* stage, const float4* __restrict__ src, int W, int xw, int xe, int ch,
+                                              const BloomTaps t, float threshold) {
+    const int lane = threadIdx.x & 31;
+    auto weight = [&](int d) { return d < -t.near || d > t.near ? 0.0f : t.w[t.near + d]; };
+    auto value = [&](int x) {
+        const float4 p = __ldg(src + x);
+        return below(p, threshold) ? 0.0f : (ch == 0 ? p.x : (ch == 1 ? p.y : p.z));
+    };
+    uint32_t nan_to = 0u;   // outputs xw + 32 k + lane that a NaN reaches
+    const int first = max(0, xw - t.K), last = min(W - 1, min(xw + kXChunk, xe) - 1 + t.K);
+    bool infinite = false;
+    for (int pass = 0; pass < 2; ++pass) {   // NaNs; then infinities, if there are any
+#pragma unroll 2
+        for (int x32 = first; x32 <= last; x32 += 32) {
+            const float v = x32 + lane <= last ? value(x32 + lane) : 0.0f;
+            infinite = infinite || fabsf(v) == INFINITY;
+            for (uint32_t m = __ballot_sync(0xFFFFFFFFu, pass == 0 ? !(v == v) : fabsf(v) == INFINITY); m; m &= m - 1u) {
+                const int from = __ffs(m) - 1, at = x32 + from;
+                const float u = __shfl_sync(0xFFFFFFFFu, v, from);
+#pragma unroll 1
+                for (int k = 0; k < kXOut; ++k) {
+                    const int x = xw + 32 * k + lane, d = at - x;
+                    if (d < -t.K || d > t.K || x >= xe) continue;
+                    if (pass == 0) nan_to |= 1u << k;
+                    else stage[32 * k + lane] += u * weight(d);
+                }
+            }
+        }
+        if (pass == 1 || !__any_sync(0xFFFFFFFFu, infinite)) break;
+#pragma unroll 1
+        for (int k = 0; k < kXOut; ++k) {   // finite values whose sum overflows: in order, the infinities among them
+            const int x = xw + 32 * k + lane;
+            if (x >= xe || !not_finite(stage[32 * k + lane], 0.0f, 0.0f)) continue;
+            float sum = 0.0f;
+            for (int i = max(-t.K, -x); i <= min(t.K, W - 1 - x); ++i) sum += value(x + i) * weight(i);
+            stage[32 * k + lane] = sum;
+        }
     }
-    return flag;
+    for (; nan_to; nan_to &= nan_to - 1u) stage[32 * (__ffs(nan_to) - 1) + lane] = NAN;
+    __syncwarp();
 }
 
 // blurX of one segment (kXSeg pixels) of a row per block, into one plane per channel.  The thresholded pixels of
 // the segment and its `near` neighbours lie in shared memory, a plane per channel (zeros stand for taps
-// outside the image and below the threshold); a warp has a channel of a quarter of the segment (four warps that
-// took the channels in turn left a small image's few blocks waiting: 671x296 at radius 0.86, 43 us a call, 34 us
-// so), and a thread sums kXOut neighbouring outputs from a register window, so a tap costs kXOut FMAs, one shared load and a quarter of a weight load (kXOut is
-// odd: the threads' windows start in different banks).  A warp's outputs go through shared memory to leave
-// in full lines.  The pixels that only taps of weight zero reach are read for values that are not finite.
-// SHARED false: a kernel too wide for a block's shared memory, every tap read from memory.  Bound by the FP32
-// issue rate.
-template <bool SHARED>
+// outside the image, below the threshold and not finite); a warp has a channel of a quarter of the segment (four
+// warps that took the channels in turn left a small image's few blocks waiting: 671x296 at radius 0.86, 43 us a
+// call, 34 us so), and a thread sums kXOut neighbouring outputs from a register window, so a tap costs kXOut FMAs,
+// one shared load and a quarter of a weight load (kXOut is odd: the threads' windows start in different banks).  A
+// warp's outputs go through shared memory to leave in full lines.  The pixels that only taps of weight zero reach
+// are read for values that are not finite.  Bound by the FP32 issue rate.
 __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restrict__ in, float* __restrict__ out, int W, int H, int pitch,
                                                          size_t plane, BloomTaps t, float threshold, int* __restrict__ flags) {
     extern __shared__ float row[];
@@ -154,81 +163,113 @@ __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restric
     const int stride = xe - xs + 2 * t.near + 2 * kXStep;   // plane length: from pixel xs - near, and zeros behind
     const float4* src = in + (size_t)y * W;
     float* dst = out + (size_t)y * pitch;
-    bool bad = !SHARED;
-    if (SHARED) {
+    bool bad = false;
 #pragma unroll 4
-        for (int j = threadIdx.x; j < stride; j += kXThreads) {
-            const int x = xs + j - t.near;
-            float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (x >= 0 && x < W) p = __ldg(src + x);
-            if (below(p, threshold)) p.x = p.y = p.z = 0.0f;
-            bad = bad || not_finite(p.x, p.y, p.z);
-            row[j] = p.x;
-            row[stride + j] = p.y;
-            row[2 * stride + j] = p.z;
-        }
-        const int far = t.K - t.near;
-        for (int j = threadIdx.x; j < 2 * far; j += blockDim.x) {
-            const int x = j < far ? xs - t.K + j : xe + t.near + (j - far);
-            if (x < 0 || x >= W) continue;
-            const float4 p = __ldg(src + x);
-            bad = bad || (!below(p, threshold) && not_finite(p.x, p.y, p.z));
-        }
+    for (int j = threadIdx.x; j < stride; j += kXThreads) {
+        const int x = xs + j - t.near;
+        float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (x >= 0 && x < W) p = __ldg(src + x);
+        if (below(p, threshold)) p.x = p.y = p.z = 0.0f;
+        bad = bad || not_finite(p.x, p.y, p.z);
+        row[j] = not_finite(p.x, 0.0f, 0.0f) ? 0.0f : p.x;
+        row[stride + j] = not_finite(p.y, 0.0f, 0.0f) ? 0.0f : p.y;
+        row[2 * stride + j] = not_finite(p.z, 0.0f, 0.0f) ? 0.0f : p.z;
+    }
+    const int far = t.K - t.near;
+    for (int j = threadIdx.x; j < 2 * far; j += blockDim.x) {
+        const int x = j < far ? xs - t.K + j : xe + t.near + (j - far);
+        if (x < 0 || x >= W) continue;
+        const float4 p = __ldg(src + x);
+        bad = bad || (!below(p, threshold) && not_finite(p.x, p.y, p.z));
     }
     wait_for_previous();   // the weights; the pixels above were there before the call's first kernel began
     const float wsum = *t.sum;
     const int any_bad = __syncthreads_or(bad ? 1 : 0);
     bool flag = false;
-    if (any_bad) {
-        flag = blur_x_all_taps(src, dst, plane, W, xs, xe, t, threshold, wsum);
-    } else {
-        const int steps = (2 * t.near + 1 + kXStep - 1) / kXStep;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = warp / 4;
-        float* stage = row + 3 * stride + warp * kXChunk;
-        const int x0 = (warp % 4) * kXChunk, xw = xs + x0;   // the warp's first output
-        if (xw < xe) {
-            float acc[kXOut], win[kXStep];   // win[k % kXStep] holds v[k]
+    const int steps = (2 * t.near + 1 + kXStep - 1) / kXStep;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = warp / 4;
+    float* stage = row + 3 * stride + warp * kXChunk;
+    const int x0 = (warp % 4) * kXChunk, xw = xs + x0;   // the warp's first output
+    if (xw < xe) {
+        float acc[kXOut], win[kXStep];   // win[k % kXStep] holds v[k]
 #pragma unroll
-            for (int r = 0; r < kXOut; ++r) acc[r] = 0.0f;
-            if (xw + lane * kXOut < xe) {
-                const float* v = row + ch * stride + x0 + lane * kXOut;   // output r sums v[r + i] w[i], i in order
-                const float4* w4 = reinterpret_cast<const float4*>(t.w);
+        for (int r = 0; r < kXOut; ++r) acc[r] = 0.0f;
+        if (xw + lane * kXOut < xe) {
+            const float* v = row + ch * stride + x0 + lane * kXOut;   // output r sums v[r + i] w[i], i in order
+            const float4* w4 = reinterpret_cast<const float4*>(t.w);
 #pragma unroll
-                for (int r = 0; r < kXOut; ++r) win[r] = v[r];
+            for (int r = 0; r < kXOut; ++r) win[r] = v[r];
 #pragma unroll 1
-                for (int s = 0; s < steps; ++s) {
+            for (int s = 0; s < steps; ++s) {
 #pragma unroll
-                    for (int g = 0; g < kXStep / 4; ++g) {
-                        const float4 wg = __ldg(w4 + g);
-                        const float wk[4] = {wg.x, wg.y, wg.z, wg.w};
+                for (int g = 0; g < kXStep / 4; ++g) {
+                    const float4 wg = __ldg(w4 + g);
+                    const float wk[4] = {wg.x, wg.y, wg.z, wg.w};
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int i = 4 * g + k;
-                            win[(i + kXOut) % kXStep] = v[i + kXOut];
+                    for (int k = 0; k < 4; ++k) {
+                        const int i = 4 * g + k;
+                        win[(i + kXOut) % kXStep] = v[i + kXOut];
 #pragma unroll
-                            for (int r = 0; r < kXOut; ++r) acc[r] += win[(i + r) % kXStep] * wk[k];
-                        }
+                        for (int r = 0; r < kXOut; ++r) acc[r] += win[(i + r) % kXStep] * wk[k];
                     }
-                    v += kXStep;
-                    w4 += kXStep / 4;
                 }
+                v += kXStep;
+                w4 += kXStep / 4;
             }
-            __syncwarp();
+        }
+        __syncwarp();
 #pragma unroll
-            for (int r = 0; r < kXOut; ++r) stage[lane * kXOut + r] = acc[r];
-            __syncwarp();
+        for (int r = 0; r < kXOut; ++r) stage[lane * kXOut + r] = acc[r];
+        __syncwarp();
+        if (any_bad) add_not_finite_x(stage, src, W, xw, xe, ch, t, threshold);
 #pragma unroll
-            for (int k = 0; k < kXOut; ++k) {
-                const int x = xw + 32 * k + lane;
-                if (x >= xe) break;
-                const float m = blur_mean(stage[32 * k + lane], wsum);
-                flag = flag || !(fabsf(m) < INFINITY);
-                dst[ch * plane + x] = m;
-            }
+        for (int k = 0; k < kXOut; ++k) {
+            const int x = xw + 32 * k + lane;
+            if (x >= xe) break;
+            const float m = blur_mean(stage[32 * k + lane], wsum);
+            flag = flag || !(fabsf(m) < INFINITY);
+            dst[ch * plane + x] = m;
         }
     }
     const int any_flag = __syncthreads_or(flag ? 1 : 0);
     if (threadIdx.x == 0) flags[(size_t)seg * H + y] = any_flag;
+}
+
+// blurX of `rows` whole rows or, with rows = 1, of one segment of a row per block, a thread per output, every tap
+// read from memory and summed in order as the reference does: kernels too wide for a block's shared memory.
+__global__ void __launch_bounds__(kXThreads) k_blur_x_all_taps(const float4* __restrict__ in, float* __restrict__ out, int W, int H,
+                                                               int pitch, size_t plane, BloomTaps t, float threshold,
+                                                               int* __restrict__ flags, int rows) {
+    __shared__ int row_flags[kXThreads];
+    const unsigned blocks = (unsigned)((H + rows - 1) / rows);
+    const int y0 = (int)(blockIdx.x % blocks) * rows, seg = (int)(blockIdx.x / blocks);
+    const int xs = seg * kXSeg, n = min(W, xs + kXSeg) - xs;
+    if ((int)threadIdx.x < rows) row_flags[threadIdx.x] = 0;
+    wait_for_previous();
+    const float wsum = *t.sum;
+    __syncthreads();
+    for (int j = threadIdx.x; j < min(rows, H - y0) * n; j += kXThreads) {
+        const int dy = j / n, x = xs + j % n;
+        const float4* src = in + (size_t)(y0 + dy) * W;
+        float* dst = out + (size_t)(y0 + dy) * pitch + x;
+        float cr = 0.0f, cg = 0.0f, cb = 0.0f;
+        const int i0 = max(-t.K, -x), i1 = min(t.K, W - 1 - x);
+        for (int i = i0; i <= i1; ++i) {
+            const float4 p = __ldg(src + x + i);
+            if (below(p, threshold)) continue;
+            const float wgt = i < -t.near || i > t.near ? 0.0f : t.w[t.near + i];
+            cr += p.x * wgt;
+            cg += p.y * wgt;
+            cb += p.z * wgt;
+        }
+        const float3 m = make_float3(blur_mean(cr, wsum), blur_mean(cg, wsum), blur_mean(cb, wsum));
+        if (not_finite(m.x, m.y, m.z)) row_flags[dy] = 1;
+        dst[0] = m.x;
+        dst[plane] = m.y;
+        dst[2 * plane] = m.z;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < min(rows, H - y0)) flags[(size_t)seg * H + y0 + threadIdx.x] = row_flags[threadIdx.x];
 }
 
 // combine.comp.glsl:15-27 then tonemapping.comp.glsl:66-84 (exposure, ACES fitted, clamp, RGBA8 UNORM).
@@ -256,6 +297,55 @@ __device__ __forceinline__ float3 aces_fitted(float3 c) {
 __device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool valid) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+// The same for a thread's kYOut outputs of blurY.
+constexpr int kSumCh = 32 * kYWarps;
+__device__ __noinline__ void add_not_finite(float* sums, const float* __restrict__ blurred_x, int pitch, size_t plane, int W, int H,
+                                            int x, int y0, const BloomTaps t, const int* __restrict__ flags) {
+    const int lane = threadIdx.x & 31;
+    auto weight = [&](int d) { return d < -t.near || d > t.near ? 0.0f : __ldg(t.w + kYOut + t.near + d); };
+    const int first = max(0, y0 - t.K), last = min(H - 1, y0 + kYOut - 1 + t.K);
+    uint32_t nan_to[3] = {0u, 0u, 0u};   // per channel: outputs that a NaN reaches
+    bool infinite = false;
+    for (int pass = 0; pass < 2; ++pass) {   // NaNs; then infinities, if there are any
+        for (int y32 = first; y32 <= last; y32 += 32) {   // a lane per row's flag, then the flagged rows, four at a time
+            const bool flagged = y32 + lane <= last && __ldg(flags + (size_t)((x - lane) / kXSeg) * H + y32 + lane) != 0;
+            for (uint32_t m = __ballot_sync(0xFFFFFFFFu, flagged); m;) {
+                int ys[4];
+                float v[4][3];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    ys[j] = m ? y32 + __ffs(m) - 1 : -1;
+                    m &= m - 1u;
+                    const float* p = blurred_x + (size_t)ys[j] * pitch + x;
+                    for (int ch = 0; ch < 3; ++ch) v[j][ch] = ys[j] >= 0 && x < W ? __ldg(p + ch * plane) : 0.0f;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int r0 = max(0, ys[j] - t.K - y0), r1 = min(kYOut - 1, ys[j] + t.K - y0);
+                    for (int ch = 0; ch < 3; ++ch) {
+                        infinite = infinite || fabsf(v[j][ch]) == INFINITY;
+                        if (pass == 0 && !(v[j][ch] == v[j][ch])) nan_to[ch] |= (2u << r1) - (1u << r0);
+                        if (pass == 1 && fabsf(v[j][ch]) == INFINITY)
+                            for (int r = r0; r <= r1; ++r) sums[(3 * r + ch) * kSumCh] += v[j][ch] * weight(ys[j] - y0 - r);
+                    }
+                }
+            }
+        }
+        if (pass == 1 || !__any_sync(0xFFFFFFFFu, infinite)) break;
+#pragma unroll 1
+        for (int k = 0; k < 3 * kYOut && x < W; ++k) {   // finite values whose sum overflows: in order, the infinities among them
+            if (!not_finite(sums[k * kSumCh], 0.0f, 0.0f)) continue;
+            const float* p = blurred_x + (k % 3) * plane + x;
+            const int at = y0 + k / 3;
+            float sum = 0.0f;
+            for (int y = max(first, at - t.K); y <= min(last, at + t.K); ++y) sum += __ldg(p + (size_t)y * pitch) * weight(y - at);
+            sums[k * kSumCh] = sum;
+        }
+    }
+    for (int ch = 0; ch < 3; ++ch)
+        for (; nan_to[ch]; nan_to[ch] &= nan_to[ch] - 1u) sums[(3 * (__ffs(nan_to[ch]) - 1) + ch) * kSumCh] = NAN;
 }
 
 // blurY, combine and tone map: a lane per column, kYOut consecutive rows per thread, 32 columns x 48 rows a block.
@@ -287,86 +377,76 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
     // the sums of a thread's outputs, [output][channel][thread] over the ring once it is read: the epilogue then loops
     // (unrolled over the outputs with their divisions it had a small image wait on instruction fetches)
     float* sums = &ring[0][0] + threadIdx.x;
-    constexpr int kSumCh = 32 * kYWarps;
     static_assert(sizeof(ring) >= sizeof(float) * kYOut * 3 * kSumCh);
-    if (any_bad) {
-        if (x < W) {
-#pragma unroll 1
-            for (int r = 0; r < kYOut && y0 + r < H; ++r) {
-                const float3 c = blur_all_taps(y0 + r, H, t, t.w + kYOut + t.near, [&](int i, float3& v) {
-                    const float* p = blurred_x + (size_t)(y0 + r + i) * pitch + x;
-                    v = make_float3(__ldg(p), __ldg(p + plane), __ldg(p + 2 * plane));
-                    return true;
-                });
-                sums[(3 * r + 0) * kSumCh] = c.x;
-                sums[(3 * r + 1) * kSumCh] = c.y;
-                sums[(3 * r + 2) * kSumCh] = c.z;
+    float cr[kYOut], cg[kYOut], cb[kYOut];
+#pragma unroll
+    for (int r = 0; r < kYOut; ++r) cr[r] = cg[r] = cb[r] = 0.0f;
+    // chunk c: rows [yb - near + kYRows c, + kYRows); those with a row of the image only
+    const int base = yb - t.near;
+    const int c0 = base < 0 ? -base / kYRows : 0;
+    const int c1 = (min(2 * t.near + kYOut * kYWarps, H - base) + kYRows - 1) / kYRows;
+    const float* col = blurred_x + (x - lane);
+    auto fill = [&](int c) {
+        if (c < c1) {
+            float* dst = ring[c % kYStages];
+            for (int k = threadIdx.x; k < kYRows * 3 * 8; k += 32 * kYWarps) {
+                const int row = k / 24, ch = k / 8 % 3, part = k % 8, y = base + c * kYRows + row;
+                const bool in_image = y >= 0 && y < H && x - lane + 4 * part < pitch;
+                copy16_or_zero(dst + 4 * k, in_image ? col + ch * plane + (size_t)y * pitch + 4 * part : blurred_x, in_image);
             }
         }
-    } else {
-        float cr[kYOut], cg[kYOut], cb[kYOut];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int c = 0; c < kYStages - 1; ++c) fill(c0 + c);
+    float win[kYOut];   // win[(s - r) mod kYOut]: the weight of step s (row y0 - near + s) for output r
 #pragma unroll
-        for (int r = 0; r < kYOut; ++r) cr[r] = cg[r] = cb[r] = 0.0f;
-        // chunk c: rows [yb - near + kYRows c, + kYRows); those with a row of the image only
-        const int base = yb - t.near;
-        const int c0 = base < 0 ? -base / kYRows : 0;
-        const int c1 = (min(2 * t.near + kYOut * kYWarps, H - base) + kYRows - 1) / kYRows;
-        const float* col = blurred_x + (x - lane);
-        auto fill = [&](int c) {
-            if (c < c1) {
-                float* dst = ring[c % kYStages];
-                for (int k = threadIdx.x; k < kYRows * 3 * 8; k += 32 * kYWarps) {
-                    const int row = k / 24, ch = k / 8 % 3, part = k % 8, y = base + c * kYRows + row;
-                    const bool in_image = y >= 0 && y < H && x - lane + 4 * part < pitch;
-                    copy16_or_zero(dst + 4 * k, in_image ? col + ch * plane + (size_t)y * pitch + 4 * part : blurred_x, in_image);
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        for (int c = 0; c < kYStages - 1; ++c) fill(c0 + c);
-        float win[kYOut];   // win[(s - r) mod kYOut]: the weight of step s (row y0 - near + s) for output r
-#pragma unroll
-        for (int r = 0; r < kYOut; ++r) win[r] = 0.0f;
-        bool begun = false;
-        for (int c = c0; c < c1; ++c) {
-            fill(c + kYStages - 1);
-            asm volatile("cp.async.wait_group %0;" ::"n"(kYStages - 1) : "memory");
-            __syncthreads();
-#pragma unroll 1
-            for (int g = 0; g < kYRows / kYOut; ++g) {
-                const int s = c * kYRows + g * kYOut - warp * kYOut;
-                if (s < 0 || s >= 2 * t.near + kYOut) continue;
-                const float* w = t.w + kYOut + s;   // zeros before and after the 2 near + 1 weights
-                if (!begun) {   // the window before this warp's first step
-#pragma unroll
-                    for (int r = 1; r < kYOut; ++r) win[kYOut - r] = __ldg(w - r);
-                    begun = true;
-                }
-                const float* p = ring[c % kYStages] + g * (kYOut * 3 * 32) + lane;
-                float4 wg;
-#pragma unroll
-                for (int k = 0; k < kYOut; ++k) {
-                    if (k % 4 == 0) wg = __ldg(reinterpret_cast<const float4*>(w + k));
-                    win[k] = k % 4 == 0 ? wg.x : (k % 4 == 1 ? wg.y : (k % 4 == 2 ? wg.z : wg.w));
-                    const float pr = p[(3 * k + 0) * 32], pg = p[(3 * k + 1) * 32], pb = p[(3 * k + 2) * 32];
-#pragma unroll
-                    for (int r = 0; r < kYOut; ++r) {
-                        const float wgt = win[(k - r + kYOut) % kYOut];
-                        cr[r] += pr * wgt;
-                        cg[r] += pg * wgt;
-                        cb[r] += pb * wgt;
-                    }
-                }
-            }
+    for (int r = 0; r < kYOut; ++r) win[r] = 0.0f;
+    bool begun = false;
+    for (int c = c0; c < c1; ++c) {
+        fill(c + kYStages - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kYStages - 1) : "memory");
+        __syncthreads();
+        if (any_bad) {   // values that are not finite are left out here: the window pads the kernel with zeros
+            float* chunk = ring[c % kYStages];
+            for (int k = threadIdx.x; k < kYRows * 3 * 32; k += 32 * kYWarps)
+                if (not_finite(chunk[k], 0.0f, 0.0f)) chunk[k] = 0.0f;
             __syncthreads();
         }
+#pragma unroll 1
+        for (int g = 0; g < kYRows / kYOut; ++g) {
+            const int s = c * kYRows + g * kYOut - warp * kYOut;
+            if (s < 0 || s >= 2 * t.near + kYOut) continue;
+            const float* w = t.w + kYOut + s;   // zeros before and after the 2 near + 1 weights
+            if (!begun) {   // the window before this warp's first step
 #pragma unroll
-        for (int r = 0; r < kYOut; ++r) {
-            sums[(3 * r + 0) * kSumCh] = cr[r];
-            sums[(3 * r + 1) * kSumCh] = cg[r];
-            sums[(3 * r + 2) * kSumCh] = cb[r];
+                for (int r = 1; r < kYOut; ++r) win[kYOut - r] = __ldg(w - r);
+                begun = true;
+            }
+            const float* p = ring[c % kYStages] + g * (kYOut * 3 * 32) + lane;
+            float4 wg;
+#pragma unroll
+            for (int k = 0; k < kYOut; ++k) {
+                if (k % 4 == 0) wg = __ldg(reinterpret_cast<const float4*>(w + k));
+                win[k] = k % 4 == 0 ? wg.x : (k % 4 == 1 ? wg.y : (k % 4 == 2 ? wg.z : wg.w));
+                const float pr = p[(3 * k + 0) * 32], pg = p[(3 * k + 1) * 32], pb = p[(3 * k + 2) * 32];
+#pragma unroll
+                for (int r = 0; r < kYOut; ++r) {
+                    const float wgt = win[(k - r + kYOut) % kYOut];
+                    cr[r] += pr * wgt;
+                    cg[r] += pg * wgt;
+                    cb[r] += pb * wgt;
+                }
+            }
         }
+        __syncthreads();
     }
+#pragma unroll
+    for (int r = 0; r < kYOut; ++r) {
+        sums[(3 * r + 0) * kSumCh] = cr[r];
+        sums[(3 * r + 1) * kSumCh] = cg[r];
+        sums[(3 * r + 2) * kSumCh] = cb[r];
+    }
+    if (any_bad) add_not_finite(sums, blurred_x, pitch, plane, W, H, x, y0, t, flags);
     if (x >= W) return;
     const int rows = min(kYOut, H - y0);
 #pragma unroll 4
@@ -430,14 +510,16 @@ void postprocess(PostWorkspace& ws, const float* d_accum, int W, int H, const Bl
     check_cuda(cudaGetLastError(), "postprocess launch");
     float* ping = ws.ping.as<float>();
     const size_t shared = sizeof(float) * (3 * ((size_t)std::min(W, kXSeg) + 2 * (size_t)tx.near + 2 * kXStep) + 3 * kXSeg);
-    const unsigned xblocks = (unsigned)segs * (unsigned)H;
+    const int rows = 1;
     if (shared <= kXMaxShared) {
         if (shared > 48 * 1024)
-            check_cuda(cudaFuncSetAttribute(k_blur_x<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXMaxShared),
+            check_cuda(cudaFuncSetAttribute(k_blur_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXMaxShared),
                        "cudaFuncSetAttribute");
-        launch_after(k_blur_x<true>, xblocks, kXThreads, shared, st, accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
+        launch_after(k_blur_x, (unsigned)segs * (unsigned)H, kXThreads, shared, st, accum, ping, W, H, pitch, plane, tx, bloom.threshold,
+                     flags);
     } else {
-        launch_after(k_blur_x<false>, xblocks, kXThreads, 0, st, accum, ping, W, H, pitch, plane, tx, bloom.threshold, flags);
+        launch_after(k_blur_x_all_taps, (unsigned)segs * (unsigned)((H + rows - 1) / rows), kXThreads, 0, st, accum, ping, W, H, pitch,
+                     plane, tx, bloom.threshold, flags, rows);
     }
     const unsigned blocks = (unsigned)((W + 31) / 32) * (unsigned)((H + kYOut * kYWarps - 1) / (kYOut * kYWarps));
     launch_after(k_blur_y_tonemap, blocks, 32 * kYWarps, 0, st, ping, pitch, plane, accum, reinterpret_cast<float4*>(d_combined),
