@@ -236,7 +236,9 @@ __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restric
 }
 
 // blurX of `rows` whole rows or, with rows = 1, of one segment of a row per block, a thread per output, every tap
-// read from memory and summed in order as the reference does: kernels too wide for a block's shared memory.
+// read from memory and summed in order as the reference does: kernels too wide for a block's shared memory, and
+// images so narrow that a block per row would be nearly empty (below 32 pixels: 1x65536 at radius 0.05 252 us with
+// k_blur_x and 45 us here, 24x20000 at radius 0.1 92 and 33 us; 31x31 the same).
 __global__ void __launch_bounds__(kXThreads) k_blur_x_all_taps(const float4* __restrict__ in, float* __restrict__ out, int W, int H,
                                                                int pitch, size_t plane, BloomTaps t, float threshold,
                                                                int* __restrict__ flags, int rows) {
@@ -510,8 +512,9 @@ void postprocess(PostWorkspace& ws, const float* d_accum, int W, int H, const Bl
     check_cuda(cudaGetLastError(), "postprocess launch");
     float* ping = ws.ping.as<float>();
     const size_t shared = sizeof(float) * (3 * ((size_t)std::min(W, kXSeg) + 2 * (size_t)tx.near + 2 * kXStep) + 3 * kXSeg);
-    const int rows = 1;
-    if (shared <= kXMaxShared) {
+    // Images up to 31 pixels wide give a block of the general form little to do but its launch and its barriers.
+    const int rows = W < 32 ? kXThreads / W : 1;
+    if (rows == 1 && shared <= kXMaxShared) {
         if (shared > 48 * 1024)
             check_cuda(cudaFuncSetAttribute(k_blur_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXMaxShared),
                        "cudaFuncSetAttribute");
