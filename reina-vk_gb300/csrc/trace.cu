@@ -289,16 +289,16 @@ static int persistent_grid(int sm_count) {
 // Rays up to which a chunk's rays come from 8 places.  Neighbouring rays are alike, and so are the rays of a chunk of
 // them: a cast of little more than a round waits for the warps whose 32 rays are all long.  In a longer cast the queue
 // evens that out, and the coherence of a chunk is worth more; in a small scene it is from fewer rays on.  Chunks of
-// neighbours against spread ones, closest hit, us (means over six scenes and ray sets of each size):
-//                              1,620 triangles   30,420         338,000        64 instances of 5,120
-//     45,000, half a camera's  31.7  28.4        47.0  40.7     64.0  59.9     86.1  72.4
-//     90,100, a camera's       37.8  34.7        59.9  50.6     82.5  71.7     99.1  84.3
-//     125,000, half random     39.6  41.0        59.2  56.1     81.4  79.2      100  92.2
-//     185,000, a camera's      51.4              74.8  71.0      101  94.2      120   112
-//     302,882, half random     62.3              81.1  85.1      107   111      123   122
-// (one such set, runs of 1, 2, 4, 8 neighbouring rays: 136, 129, 128, 142 us).  Rays in random order: within 2 %.
+// neighbours against spread ones, closest hit, us (means over four to six scenes and ray sets of each size):
+//                              1,620 triangles   5,120        15,680       81,920       64 instances of 5,120
+//     45,000, half a camera's  30.8  28.3        34.6  30.7   41.0  35.8   51.0  48.0   85.5  69.5
+//     96,100, a camera's       37.3  34.4        42.5  38.6   51.3  44.7   64.3  59.4   97.9  86.4
+//     122,500, a camera's      40.8  43.1        46.2  47.0   56.5  52.6   71.5  68.3    101  96.2
+//     160,000, a camera's      44.0  51.3        49.5  57.7   60.0  62.9   75.8  74.7    110   115
+//     168,100, half random     43.6  47.3        48.3  50.3   58.0  56.2   71.5  70.5    105  97.6
+// (one set of 302,882, runs of 1, 2, 4, 8 neighbouring rays: 136, 129, 128, 142 us).  Rays in random order: within 3 %.
 static uint64_t spread_limit(const DeviceScene& s, int sm_count) {
-    return (s.inst_trav || s.node_count >= 512 ? 1280ull : 600ull) * (uint64_t)std::max(1, sm_count);
+    return (s.inst_trav || s.node_count >= 1024 ? 1280ull : 700ull) * (uint64_t)std::max(1, sm_count);
 }
 
 template <bool ANY, bool COUNT, bool TWO>
