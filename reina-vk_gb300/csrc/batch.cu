@@ -855,6 +855,7 @@ void BatchEngine::launch_body(Lane& L, const Packed& pk, cudaStream_t st) {
     for (auto& g : L.graphs)
         if (g.shape == w) slot = &g;
     if (!slot) {
+        make_room(L, w.bounces);
         cudaStream_t cap;
         check_cuda(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "cudaStreamCreate");
         cudaGraph_t graph = nullptr;
@@ -880,7 +881,22 @@ void BatchEngine::launch_body(Lane& L, const Packed& pk, cudaStream_t st) {
         L.graphs.push_back(g);
         slot = &L.graphs.back();
     }
+    slot->used = submissions_;
     check_cuda(cudaGraphLaunch(slot->exec, st), "cudaGraphLaunch");
+}
+
+// Destroys the lane's graphs used longest ago until one of `bounces` more fits into kGraphBounces.  The lane is free,
+// so none of them is running.
+void BatchEngine::make_room(Lane& L, uint32_t bounces) {
+    uint64_t held = 0;
+    for (const GraphSlot& g : L.graphs) held += g.shape.bounces;
+    while (!L.graphs.empty() && held + bounces > kGraphBounces) {
+        const auto oldest = std::min_element(L.graphs.begin(), L.graphs.end(),
+                                             [](const GraphSlot& a, const GraphSlot& b) { return a.used < b.used; });
+        held -= oldest->shape.bounces;
+        cudaGraphExecDestroy(oldest->exec);
+        L.graphs.erase(oldest);
+    }
 }
 
 BatchLaunch BatchEngine::wave_view(const Lane& L) const {
@@ -1047,6 +1063,7 @@ bool BatchEngine::submit_wave(const std::vector<BatchJob*>& jobs, bool fifo, std
         Lane& D = lane_of(pk.after - 1);
         if (&D != &L) check_cuda(cudaStreamWaitEvent(L.stream, D.finished, 0), "cudaStreamWaitEvent");
     }
+    ++submissions_;
     launch_body(L, pk, L.stream);
     if (prev) check_cuda(cudaStreamWaitEvent(L.stream, prev->finished, 0), "cudaStreamWaitEvent");
     launch_finish(L, pk, L.stream);

@@ -19,6 +19,9 @@ namespace rt {
 
 constexpr uint32_t kMaxWaveSegments = 1024;
 constexpr size_t kBatchPathBytes = 164;   // path state and queues of a wave slot
+// Bounces of the wave graphs that a lane keeps: about 130 KB of device and 20 KB of host memory each (graphs of 10
+// to 329 bounces, one of each, took 7 GB and 2.4 GB).  A hundred shapes of ten bounces fit.
+constexpr uint64_t kGraphBounces = 1024;
 struct BatchLaunch;                       // the kernels' view of a wave (batch.cu)
 
 // Per-job data the kernels read (one table per wave, holding the jobs present in that wave).
@@ -152,6 +155,7 @@ private:
     struct GraphSlot {
         Shape shape;
         cudaGraphExec_t exec = nullptr;
+        uint64_t used = 0;   // submissions_ at its last launch
     };
     struct Lane {
         size_t index = 0;
@@ -175,6 +179,7 @@ private:
     Packed pack(const std::vector<BatchJob*>& jobs, bool fifo, Lane& L);
     // Descriptor upload + wave body (init and the bounce kernels) on `s`.
     void launch_body(Lane& L, const Packed& pk, cudaStream_t s);
+    void make_room(Lane& L, uint32_t bounces);
     void launch_sequence(const BatchLaunch& B, const Shape& w, cudaStream_t main, bool fork);
     void launch_trace(const BatchLaunch& B, const Shape& w, bool extend, int cur, uint32_t* bounce, cudaStream_t st);
     template <bool MIXED, bool TWO, bool COUNT>
@@ -202,6 +207,7 @@ private:
     RenderStats work_;
     uint32_t waves_ = 0;
     uint64_t submitted_ = 0, retired_ = 0;   // waves launched / waited for
+    uint64_t submissions_ = 0;               // waves launched since the engine was made
     int blocks_ext_ = 0, blocks_shade_[5] = {0, 0, 0, 0, 0}, blocks_sh_ = 0, blocks_simple_ = 0;
     int blocks_plain_[2][2][2] = {};       // grids of the default grid-form variant: [extend][two][count]
     int blocks_coop_[2][2][2][2] = {};     // of the cooperative form: [extend][mixed][two][count]
