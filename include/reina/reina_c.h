@@ -75,16 +75,18 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
  *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
  *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and
- *            batches take wave_refill, where 0 and REINA_REFILL_GRID leave the form to the engine: eight
- *            lanes per ray for calls of few paths (at most 96 per SM, 192 of a two-level scene, 352 of a flat
- *            one of 512 or more nodes), above that cooperative for flat scenes of 512 or more nodes and for
- *            two-level calls of 2^20 or more paths, else the grid form (1920x1080, 16 spp of that scene 75.3 ms
- *            grid, 48.8 ms cooperative; a 256x256 Cornell room 1.36 against 1.85 ms); calls that return work
- *            counters run the grid form.
+ *            batches take wave_refill, where 0 and REINA_REFILL_GRID (which reina_ctx_get_tuning returns for
+ *            either) leave the form to the engine: eight lanes per ray for calls of few paths (at most 96 per SM,
+ *            192 of a two-level scene, 352 of a flat one of 512 or more nodes), above that cooperative for flat
+ *            scenes of 512 or more nodes and for two-level calls of 2^20 or more paths, else the grid form
+ *            (1920x1080, 16 spp of that scene 75.3 ms grid, 48.8 ms cooperative; a 256x256 Cornell room 1.36
+ *            against 1.85 ms); calls that return work counters run the grid form.  REINA_REFILL_GRID_ALWAYS asks
+ *            for the grid form whatever the call.
  *   trace_block: threads per block of the grid-form traversal kernels (ray cast, wavefront extend and
- *            shadow): 64, 128 or 256 (default 128).  Grid form only.
+ *            shadow): 64, 128 or 256 (default 128).  Grid form only: of frames and batches where the engine
+ *            chooses it or wave_refill asks for it, and not for two-level scenes or calls that count.
  *   trace_stack: shared-memory traversal stack entries per thread, 8, 12 or 16 (default 12); deeper
- *            levels spill to local memory.
+ *            levels spill to local memory.  Where trace_block applies.
  *   trace_order: the order a grid-form ray cast traces its rays in (below).
  *   wave_paths: path slots of one wave of a batched render or frame (0 = REINA_DEFAULT_WAVE_PATHS);
  *            the path state costs 164 bytes per slot and wave in flight (wave_lanes): the waves run on
@@ -113,7 +115,7 @@ typedef struct reina_tuning {
                                   * (0 = REINA_DEFAULT_WAVE_LANES) */
     uint32_t wave_refill;        /* launch form of the wavefront extension and shadow kernels (frames,
                                   * batches): like `refill`, but 0 = the default REINA_REFILL_GRID, with which
-                                  * the engine chooses */
+                                  * the engine chooses, or REINA_REFILL_GRID_ALWAYS */
 } reina_tuning;
 /* REINA_ORDER_INPUT traces ray i on thread i.  REINA_ORDER_COHERENT first bins the rays by direction
  * octant and origin cell (Morton order on an 8^3 grid over the origins' bounds) and traces them in that
@@ -122,7 +124,7 @@ typedef struct reina_tuning {
  * ray sets (on the 1.3M-triangle workload: random half 0.513 vs 0.525 ms, camera half 0.49 vs 0.46 ms);
  * the autotuner tries both. */
 enum { REINA_ORDER_INPUT = 0, REINA_ORDER_COHERENT = 1 };
-enum { REINA_REFILL_GRID = 255 };
+enum { REINA_REFILL_GRID = 255, REINA_REFILL_GRID_ALWAYS = 254 };
 /* Waves of 2^21 slots, 8 in flight (2.75 GB of path state).  Every wave ends in a tail of a few long
  * paths at low occupancy (late bounces are latency-bound chains of node fetches), which the other waves
  * in flight fill.  On a 256-scene batch (3.1 G paths): one wave in flight 12.94 s at 2^21 slots and

@@ -75,7 +75,8 @@ void TuneCache::load(const std::string& path) {
         std::string rest;
         is.clear();
         if (is >> rest) fail(REINA_ERR_IO, path + ":" + std::to_string(lineno) + ": trailing text in autotune entry");
-        if (kind > kTuneBatch || !valid_trace_config(e.trace) || wave > (1u << 26))
+        const bool waves = kind == kTuneRender || kind == kTuneBatch;
+        if (kind > kTuneBatch || !(waves ? valid_wave_config(e.trace) : valid_trace_config(e.trace)) || wave > (1u << 26))
             fail(REINA_ERR_IO, path + ":" + std::to_string(lineno) + ": invalid autotune entry");
         e.wave_paths = wave;
         add[std::make_tuple(kind, tb, sb)] = e;

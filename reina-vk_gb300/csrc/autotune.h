@@ -33,7 +33,7 @@ public:
     size_t size() const;
     // Text format, one entry per line:
     //   kind tri_bucket size_bucket refill block stack wave_paths best_ms default_ms [order]
-    // (order: 0 input ray order, the default when absent; 1 coherence order)
+    // (refill: TraceConfig::refill; order: 0 input ray order, the default when absent; 1 coherence order)
     // Lines starting with '#' are comments.  load() merges into the cache (later lines win).
     void save(const std::string& path) const;
     void load(const std::string& path);

@@ -691,8 +691,8 @@ void BatchEngine::launch_coop(const BatchLaunch& B, bool extend, int cur, uint32
     else kb_shadow_coop<MIXED, TWO, COUNT><<<grid, kCoopBlock, shared, st>>>(B, B.jobs, bounce, refill_at);
 }
 
-// The form of a call's waves: cooperative traversal where it was asked for (reina_tuning.wave_refill), else by
-// the jobs' scenes and paths.  A call of few paths waits for each bounce's longest ray, so it traces with eight
+// The form of a call's waves: cooperative traversal or the grid form where it was asked for (reina_tuning.wave_refill),
+// else by the jobs' scenes and paths.  A call of few paths waits for each bounce's longest ray, so it traces with eight
 // lanes per ray (frames of 8 bounces with 4.6k / 12k / 30k / 46k paths, us, grid or cooperative against wide: 3 nodes
 // 268 / 271 / 285 / 303 against 223 / 258 / 322 / 410; zoo of 12 instances 962 / 995 / 1061 / 1096 against 656 / 788 /
 // 1036 / 1409; 64 instances 1275 / 1340 / 1428 / 1503 against 749 / 925 / 1231 / 1692; 82k triangles 743 / 789 / 851 / 894
@@ -727,7 +727,8 @@ void BatchEngine::choose_form(const std::vector<BatchJob*>& jobs) {
     }
     const uint64_t wide_paths = (two ? 192ull : nodes >= kCoopNodes ? 352ull : 96ull) * sm_count_;
     wide_ = trace_.refill == 0 && !count_ && paths <= wide_paths;
-    coop_ = trace_.refill > 0 || (!count_ && !wide_ && (two ? paths >= kCoopTwoLevelPaths : nodes >= kCoopNodes));
+    coop_ = trace_.refill > 0 ||
+            (trace_.refill == 0 && !count_ && !wide_ && (two ? paths >= kCoopTwoLevelPaths : nodes >= kCoopNodes));
     wave_limit_ = UINT32_MAX;
     if (!coop_ && paths >= kOverlapPaths) {
         const uint64_t waves = std::max<uint64_t>(std::min<uint64_t>(kOverlapWaves, lanes_.size()), (paths + capacity_ - 1) / capacity_);

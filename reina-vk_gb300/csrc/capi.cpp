@@ -182,6 +182,10 @@ rt::TraceConfig trace_for(const reina_ctx* ctx, uint32_t kind, uint64_t triangle
 // reina_tuning's refill fields <-> TraceConfig::refill (0 = grid form).
 int refill_from_abi(uint32_t v, int dflt) { return v == 0 ? dflt : (v == REINA_REFILL_GRID ? 0 : (int)v); }
 uint32_t refill_to_abi(int r) { return r == 0 ? (uint32_t)REINA_REFILL_GRID : (uint32_t)r; }
+int wave_refill_from_abi(uint32_t v) {
+    return v == REINA_REFILL_GRID_ALWAYS ? rt::kGridAlways : refill_from_abi(v, rt::kDefaultWaveRefill);
+}
+uint32_t wave_refill_to_abi(int r) { return r == rt::kGridAlways ? (uint32_t)REINA_REFILL_GRID_ALWAYS : refill_to_abi(r); }
 
 }  // namespace
 
@@ -247,8 +251,8 @@ int reina_ctx_set_tuning(reina_ctx* ctx, const reina_tuning* t) {
     return guard([&] {
         need(ctx && t, "NULL argument");
         need(t->refill <= 32 || t->refill == REINA_REFILL_GRID, "refill must be in 0..32 or REINA_REFILL_GRID");
-        need(t->wave_refill <= 32 || t->wave_refill == REINA_REFILL_GRID,
-             "wave_refill must be in 0..32 or REINA_REFILL_GRID");
+        need(t->wave_refill <= 32 || t->wave_refill == REINA_REFILL_GRID || t->wave_refill == REINA_REFILL_GRID_ALWAYS,
+             "wave_refill must be in 0..32, REINA_REFILL_GRID or REINA_REFILL_GRID_ALWAYS");
         need((t->batch_flags & ~(uint32_t)(REINA_BATCH_NO_GRAPHS | REINA_BATCH_FAIR_SHARE)) == 0, "unknown batch flags");
         need(t->wave_lanes <= 16, "wave_lanes must be in 0..16");
         const uint32_t lanes = t->wave_lanes ? t->wave_lanes : (uint32_t)REINA_DEFAULT_WAVE_LANES;
@@ -262,7 +266,7 @@ int reina_ctx_set_tuning(reina_ctx* ctx, const reina_tuning* t) {
         tc.sort = t->trace_order == REINA_ORDER_COHERENT ? 1 : 0;
         need(rt::valid_trace_config(tc), "trace_block must be 64, 128 or 256 and trace_stack 8, 12 or 16");
         rt::TraceConfig wc = tc;
-        wc.refill = refill_from_abi(t->wave_refill, rt::kDefaultWaveRefill);
+        wc.refill = wave_refill_from_abi(t->wave_refill);
         wc.sort = 0;
         const bool engine_changed = wc.block != ctx->wave_trace.block || wc.stack != ctx->wave_trace.stack ||
                                     wc.refill != ctx->wave_trace.refill;
@@ -283,7 +287,7 @@ int reina_ctx_get_tuning(const reina_ctx* ctx, reina_tuning* out) {
         need(ctx && out, "NULL argument");
         std::memset(out, 0, sizeof(*out));
         out->refill = refill_to_abi(ctx->trace.refill);
-        out->wave_refill = refill_to_abi(ctx->wave_trace.refill);
+        out->wave_refill = wave_refill_to_abi(ctx->wave_trace.refill);
         out->trace_block = (uint32_t)ctx->trace.block;
         out->trace_stack = (uint32_t)ctx->trace.stack;
         out->trace_order = ctx->trace.sort ? REINA_ORDER_COHERENT : REINA_ORDER_INPUT;
@@ -1090,7 +1094,7 @@ void fill_tuning(const reina_ctx* ctx, uint32_t kind, const rt::TuneEntry& e, re
     std::memset(t, 0, sizeof(*t));
     const bool wave = kind == rt::kTuneRender || kind == rt::kTuneBatch;
     t->refill = refill_to_abi(wave ? ctx->trace.refill : e.trace.refill);
-    t->wave_refill = refill_to_abi(wave ? e.trace.refill : ctx->wave_trace.refill);
+    t->wave_refill = wave_refill_to_abi(wave ? e.trace.refill : ctx->wave_trace.refill);
     t->trace_block = (uint32_t)e.trace.block;
     t->trace_stack = (uint32_t)e.trace.stack;
     t->trace_order = e.trace.sort ? REINA_ORDER_COHERENT : REINA_ORDER_INPUT;

@@ -21,6 +21,9 @@ constexpr int kDefaultRefill = 8;
 // engine's and the server's grid form, and the batch engine's own choice by scene and paths
 // (BatchEngine::choose_form, which holds the measurements).
 constexpr int kDefaultWaveRefill = 0;
+// Of those kernels only: the grid form whatever the engine would choose (block size and stack depth apply to every
+// wave of a flat scene then).
+constexpr int kGridAlways = -1;
 
 // Launch configuration of the traversal kernels: block size (64, 128, 256) and shared-memory stack
 // entries per thread (8, 12, 16) of the grid form, or the cooperative persistent form with its refill
@@ -33,6 +36,7 @@ struct TraceConfig {
     int sort = 0;                 // ray casts (grid form): 1 = trace the rays in coherence order
 };
 bool valid_trace_config(const TraceConfig& c);
+bool valid_wave_config(const TraceConfig& c);   // of the wavefront kernels: kGridAlways too
 
 // `d_next` is a device u32 used as the ray-fetch counter (reset by the launcher); n < 2^32.
 void launch_raycast(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_hits, bool any, uint32_t* d_err,

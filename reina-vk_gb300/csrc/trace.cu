@@ -392,6 +392,12 @@ bool valid_trace_config(const TraceConfig& c) {
     return block_ok && stack_ok && c.refill >= 0 && c.refill <= 32 && (c.sort == 0 || c.sort == 1);
 }
 
+bool valid_wave_config(const TraceConfig& c) {
+    TraceConfig t = c;
+    if (t.refill == kGridAlways) t.refill = 0;
+    return valid_trace_config(t);
+}
+
 void launch_raycast(const DeviceScene& s, const Ray* d_rays, uint64_t n, Hit* d_hits, bool any, uint32_t* d_err,
                     uint32_t* d_next, int sm_count, const TraceConfig& cfg, cudaStream_t st) {
     if (n == 0) return;

@@ -34,7 +34,10 @@ RAY_CLOSEST = 0
 RAY_ANY = 1
 MISS = 0xFFFFFFFF
 ACCEL_AUTO, ACCEL_FLAT, ACCEL_TWO_LEVEL = 0, 1, 2
-REFILL_GRID = 255   # tuning.refill: one thread per ray (grid form); 0 = the default cooperative form
+# tuning.refill: one thread per ray (grid form), 0 = the default cooperative form; tuning.wave_refill: the engine
+# chooses, as for 0
+REFILL_GRID = 255
+REFILL_GRID_ALWAYS = 254   # tuning.wave_refill: the grid form whatever the call
 
 RAY_DTYPE = np.dtype([("org", np.float32, 3), ("tmin", np.float32), ("dir", np.float32, 3), ("tmax", np.float32)])
 HIT_DTYPE = np.dtype([("prim", np.uint32), ("t", np.float32), ("u", np.float32), ("v", np.float32)])
