@@ -756,18 +756,22 @@ typedef struct reina_tune_result {
  * afterwards. */
 int reina_autotune_raycast(reina_ctx* ctx, const reina_scene* scene, const void* d_rays, uint64_t count,
                            void* d_hits, uint32_t flags, void* stream, reina_tune_result* out_result);
-/* Times one-sample frames of the render (scratch image; the caller's images are not touched). */
+/* Times frames of the render with as few samples as leave the wave engine's choice of form what it is for the whole
+ * one (scratch image; the caller's images are not touched): that choice, the grid form in the other block sizes and
+ * stack depths and the cooperative form.  The default is kept unless another is at least 2 % faster, and the entry
+ * holds for frames whose paths (pixels, times samples in REINA_MODE_NEE_MIS), up to 2^20, are within a factor of two
+ * of this one's; others run as without an entry. */
 int reina_autotune_render(reina_ctx* ctx, const reina_scene* scene, const RtPushConsts* push_consts,
                           const reina_render_options* options, reina_tune_result* out_result);
-/* Times a batched render of (up to 32 of) the jobs at no more than 2 samples per pixel, into scratch
- * images. */
+/* Times a batched render of (up to 32 of) the jobs, with their samples scaled down to about four of the largest
+ * waves, into scratch images. */
 int reina_autotune_batch(reina_ctx* ctx, const reina_render_job* jobs, uint32_t count, reina_tune_result* out_result);
 int reina_autotune_set_mode(reina_ctx* ctx, uint32_t mode);
 /* The cached configuration for a workload, if any (*out_found = 0 when there is none). */
 int reina_autotune_lookup(reina_ctx* ctx, uint32_t kind, uint64_t triangles, uint64_t work_size,
                           reina_tuning* out_tuning, int32_t* out_found);
 /* Writes / merges the cache as text, one "kind tri_bucket size_bucket refill block stack wave_paths
- * best_ms default_ms" line per entry. */
+ * best_ms default_ms" line per entry (frames: wave_paths holds the paths that the entry is for, 0 for any). */
 int reina_autotune_save(reina_ctx* ctx, const char* path);
 int reina_autotune_load(reina_ctx* ctx, const char* path);
 

@@ -1,9 +1,11 @@
 // Autotuner cache (see autotune.h).
 #include "autotune.h"
 
+#include <algorithm>
 #include <fstream>
 #include <sstream>
 
+#include "batch.h"
 #include "errors.h"
 
 namespace rt {
@@ -85,8 +87,11 @@ void TuneCache::load(const std::string& path) {
     for (const auto& [k, e] : add) map_[k] = e;
 }
 
-std::vector<TraceConfig> trace_candidates(bool with_order) {
-    std::vector<TraceConfig> out;
+bool holds_for_paths(const TuneEntry& e, uint64_t paths) {
+    return e.wave_paths == 0 || paths == 0 || tune_bucket(std::min(paths, kFormPaths)) == tune_bucket(e.wave_paths);
+}
+
+static void add_grid(std::vector<TraceConfig>& out) {
     for (int block : {64, 128, 256})
         for (int stack : {8, 12, 16}) {
             TraceConfig c;
@@ -95,17 +100,32 @@ std::vector<TraceConfig> trace_candidates(bool with_order) {
             c.refill = 0;
             out.push_back(c);
         }
-    if (with_order) {   // ray casts: also coherence order, in the default block size and stack depth
-        TraceConfig c;
-        c.refill = 0;
-        c.sort = 1;
-        out.push_back(c);
-    }
-    for (int refill : {4, 8, 16}) {   // the cooperative form
+}
+static void add_cooperative(std::vector<TraceConfig>& out) {
+    for (int refill : {4, 8, 16}) {
         TraceConfig c;
         c.refill = refill;
         out.push_back(c);
     }
+}
+
+std::vector<TraceConfig> raycast_candidates() {
+    std::vector<TraceConfig> out;
+    add_grid(out);
+    TraceConfig c;   // coherence order, in the default block size and stack depth
+    c.refill = 0;
+    c.sort = 1;
+    out.push_back(c);
+    add_cooperative(out);
+    return out;
+}
+
+std::vector<TraceConfig> render_candidates(bool pass_by_pass) {
+    std::vector<TraceConfig> out;
+    add_grid(out);
+    for (TraceConfig& c : out)
+        if (!pass_by_pass && (c.block != kTraceBlock || c.stack != kDefaultTraceStack)) c.refill = kGridAlways;
+    add_cooperative(out);
     return out;
 }
 

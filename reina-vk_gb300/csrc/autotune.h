@@ -18,7 +18,8 @@ enum TuneKind : uint32_t { kTuneRaycastClosest = 0, kTuneRaycastAny = 1, kTuneRe
 
 struct TuneEntry {
     TraceConfig trace;
-    uint32_t wave_paths = 0;      // batched renders only (0 = default)
+    uint32_t wave_paths = 0;      // batched renders: slots of a wave (0 = default); frames: paths of the call that was
+                                  // timed, up to kFormPaths (0 = any, 1 = pass by pass)
     double best_ms = 0.0;
     double default_ms = 0.0;
 };
@@ -43,8 +44,15 @@ private:
     std::map<std::tuple<uint32_t, uint32_t, uint32_t>, TuneEntry> map_;
 };
 
-// Candidate traversal configurations: the grid form in every block size x stack depth, and (for ray
-// casts) the persistent form at two refill thresholds.
-std::vector<TraceConfig> trace_candidates(bool with_order);
+// Whether a frame's entry holds for a call of `paths` paths on the wave engine, which chooses the form of its waves by
+// them (0: a call that does not, such as one pass by pass): calls within a factor of two of the timed one.
+bool holds_for_paths(const TuneEntry& e, uint64_t paths);
+
+// Candidate traversal configurations of ray casts: the grid form in every block size x stack depth and in coherence
+// order, and the cooperative form at three refill thresholds.
+std::vector<TraceConfig> raycast_candidates();
+// Of frames: the default (on the wave engine the form it chooses), the grid form in every other block size x stack
+// depth, and the cooperative form.
+std::vector<TraceConfig> render_candidates(bool pass_by_pass);
 
 }  // namespace rt

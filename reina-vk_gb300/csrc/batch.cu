@@ -714,7 +714,7 @@ void BatchEngine::launch_coop(const BatchLaunch& B, bool extend, int cur, uint32
 // 19.8 as three).
 void BatchEngine::choose_form(const std::vector<BatchJob*>& jobs) {
     constexpr uint32_t kCoopNodes = 512;
-    constexpr uint64_t kCoopTwoLevelPaths = 1ull << 20;
+    constexpr uint64_t kCoopTwoLevelPaths = kFormPaths;
     constexpr uint64_t kOverlapPaths = 1ull << 18, kOverlapWaves = 3;
     uint64_t paths = 0;   // that waves could hold at once: one sample per pixel of a job in the reference's mode
     uint32_t nodes = 0;

@@ -22,6 +22,8 @@ constexpr size_t kBatchPathBytes = 164;   // path state and queues of a wave slo
 // Bounces of the wave graphs that a lane keeps: about 130 KB of device and 20 KB of host memory each (graphs of 10
 // to 329 bounces, one of each, took 7 GB and 2.4 GB).  A hundred shapes of ten bounces fit.
 constexpr uint64_t kGraphBounces = 1024;
+// Paths from which on the form of a call's waves no longer depends on their number (choose_form).
+constexpr uint64_t kFormPaths = 1ull << 20;
 struct BatchLaunch;                       // the kernels' view of a wave (batch.cu)
 
 // Per-job data the kernels read (one table per wave, holding the jobs present in that wave).

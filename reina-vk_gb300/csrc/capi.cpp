@@ -169,14 +169,28 @@ void* host_device_pointer(void* p, int device) {
     return const_cast<void*>(host_device_pointer(static_cast<const void*>(p), device));
 }
 
-// The traversal configuration for a workload: the cached autotuned one when the context uses the
-// cache and has an entry, else the context's tuning.
+// The traversal configuration of a ray cast: the cached autotuned one when the context uses the cache and has an entry,
+// else the context's tuning.
 rt::TraceConfig trace_for(const reina_ctx* ctx, uint32_t kind, uint64_t triangles, uint64_t size) {
     rt::TuneEntry e;
     if (ctx->autotune_mode == REINA_AUTOTUNE_CACHED &&
         ctx->tune.get(kind, rt::tune_bucket(triangles), rt::tune_bucket(size), &e))
         return e.trace;
-    return kind == rt::kTuneRender || kind == rt::kTuneBatch ? ctx->wave_trace : ctx->trace;
+    return ctx->trace;
+}
+
+// Paths that the wave engine's choice of form goes by for a frame, and the configuration of a frame like trace_for's.
+uint64_t frame_paths(const RtPushConsts& pc, const rt::RenderOpts& r) {
+    const uint64_t px = (uint64_t)r.width * r.height;
+    return r.mode == REINA_MODE_NEE_MIS ? px * pc.samplesPerPixel : px;
+}
+rt::TraceConfig frame_trace(const reina_ctx* ctx, const rt::Scene& s, const RtPushConsts& pc, const rt::RenderOpts& r, bool engine) {
+    rt::TuneEntry e;
+    if (ctx->autotune_mode == REINA_AUTOTUNE_CACHED &&
+        ctx->tune.get(rt::kTuneRender, rt::tune_bucket(s.triangle_count()), rt::tune_bucket((uint64_t)r.width * r.height), &e) &&
+        rt::holds_for_paths(e, engine ? frame_paths(pc, r) : 0))
+        return e.trace;
+    return ctx->wave_trace;
 }
 
 // reina_tuning's refill fields <-> TraceConfig::refill (0 = grid form).
@@ -589,7 +603,7 @@ int reina_render_device(reina_ctx* ctx, const reina_scene* scene, const RtPushCo
         need(ctx != nullptr, "ctx is NULL");
         const rt::Scene& s = built_scene(scene);
         rt::RenderOpts r = render_opts(pc, o);
-        r.trace = trace_for(ctx, rt::kTuneRender, s.triangle_count(), (uint64_t)r.width * r.height);
+        r.trace = frame_trace(ctx, s, *pc, r, !r.megakernel && !r.pass_by_pass);
         check_render_scene(s, pc, o);
         need(d_accum != nullptr && ((uintptr_t)d_accum % 16) == 0, "accumulation buffer must be non-NULL and 16-byte aligned");
         use_device(ctx);
@@ -608,7 +622,7 @@ int reina_render_device_noalloc(reina_ctx* ctx, const reina_scene* scene, const 
         need(ctx != nullptr, "ctx is NULL");
         const rt::Scene& s = built_scene(scene);
         rt::RenderOpts r = render_opts(pc, o);
-        r.trace = trace_for(ctx, rt::kTuneRender, s.triangle_count(), (uint64_t)r.width * r.height);
+        r.trace = frame_trace(ctx, s, *pc, r, false);
         check_render_scene(s, pc, o);
         need(d_accum != nullptr && ((uintptr_t)d_accum % 16) == 0, "accumulation buffer must be non-NULL and 16-byte aligned");
         use_device(ctx);
@@ -624,7 +638,7 @@ int reina_render(reina_ctx* ctx, const reina_scene* scene, const RtPushConsts* p
         need(ctx != nullptr, "ctx is NULL");
         const rt::Scene& s = built_scene(scene);
         rt::RenderOpts r = render_opts(pc, o);
-        r.trace = trace_for(ctx, rt::kTuneRender, s.triangle_count(), (uint64_t)r.width * r.height);
+        r.trace = frame_trace(ctx, s, *pc, r, !r.megakernel && !r.pass_by_pass);
         check_render_scene(s, pc, o);
         need(accum != nullptr, "accumulation buffer is NULL");
         use_device(ctx);
@@ -1098,7 +1112,7 @@ void fill_tuning(const reina_ctx* ctx, uint32_t kind, const rt::TuneEntry& e, re
     t->trace_block = (uint32_t)e.trace.block;
     t->trace_stack = (uint32_t)e.trace.stack;
     t->trace_order = e.trace.sort ? REINA_ORDER_COHERENT : REINA_ORDER_INPUT;
-    t->wave_paths = e.wave_paths ? e.wave_paths : ctx->wave_paths;
+    t->wave_paths = kind == rt::kTuneBatch && e.wave_paths ? e.wave_paths : ctx->wave_paths;
     t->batch_flags = ctx->batch_flags;
     t->wave_lanes = ctx->wave_lanes;
 }
@@ -1119,7 +1133,7 @@ void finish_tune(reina_ctx* ctx, uint32_t kind, uint64_t tris, uint64_t size, co
     }
 }
 
-// The default launch configuration of a tuning kind (ray casts: cooperative; renders and batches: grid).
+// The default launch configuration of a tuning kind (ray casts: cooperative; renders and batches: the engine's choice).
 bool is_default(const rt::TraceConfig& c, uint32_t kind) {
     const int refill = kind == rt::kTuneRender || kind == rt::kTuneBatch ? rt::kDefaultWaveRefill : rt::kDefaultRefill;
     return c.refill == refill && c.block == rt::kTraceBlock && c.stack == rt::kDefaultTraceStack && c.sort == 0;
@@ -1140,7 +1154,7 @@ int reina_autotune_raycast(reina_ctx* ctx, const reina_scene* scene, const void*
         need(count < (1ull << 32), "at most 2^32 - 1 rays per call");
         use_device(ctx);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const auto cands = rt::trace_candidates(true);
+        const auto cands = rt::raycast_candidates();
         rt::TuneEntry best;
         best.best_ms = 1e30;
         for (const rt::TraceConfig& c : cands) {
@@ -1171,23 +1185,25 @@ int reina_autotune_render(reina_ctx* ctx, const reina_scene* scene, const RtPush
         need(!r.megakernel, "the autotuner times the wavefront (options.flags must be 0)");
         check_render_scene(s, pc, o);
         use_device(ctx);
-        RtPushConsts one = *pc;
-        one.samplesPerPixel = 1;
-        one.sampleBatch = 0;
+        // the frame with as few samples as leave the engine's choice of form what it is for the whole one
         const size_t P = (size_t)r.width * r.height;
+        const uint64_t paths = frame_paths(*pc, r);
+        RtPushConsts few = *pc;
+        few.samplesPerPixel = paths > P && !r.pass_by_pass ? (uint32_t)std::min<uint64_t>(pc->samplesPerPixel, (rt::kFormPaths + P - 1) / P) : 1;
+        few.sampleBatch = 0;
         ctx->accum.reserve(P * 4 * sizeof(float));
         cudaStream_t st = ctx->streams[0];
-        const auto cands = rt::trace_candidates(false);
+        const auto cands = rt::render_candidates(r.pass_by_pass);
         rt::TuneEntry best;
         best.best_ms = 1e30;
         for (const rt::TraceConfig& c : cands) {
             r.trace = c;
             const double ms = time_calls(st, 2, [&] {
                 if (r.pass_by_pass)
-                    rt::render_frame(ctx->render, s.device_view(), one, r, ctx->accum.as<float>(), nullptr, ctx->sm_count,
+                    rt::render_frame(ctx->render, s.device_view(), few, r, ctx->accum.as<float>(), nullptr, ctx->sm_count,
                                      st, nullptr);
                 else   // the default form: the frame as the wave engine's one job
-                    render_on_engine(ctx, scene, &one, o, r, ctx->accum.get(), nullptr, false, st, nullptr);
+                    render_on_engine(ctx, scene, &few, o, r, ctx->accum.get(), nullptr, false, st, nullptr);
             });
             if (is_default(c, rt::kTuneRender)) best.default_ms = ms;
             if (ms < best.best_ms) {
@@ -1195,6 +1211,12 @@ int reina_autotune_render(reina_ctx* ctx, const reina_scene* scene, const RtPush
                 best.trace = c;
             }
         }
+        // an entry other than the default takes the choice of form from the engine: only for a gain beyond the noise
+        if (best.best_ms > 0.98 * best.default_ms) {
+            best.best_ms = best.default_ms;
+            best.trace = reina_ctx::wave_default();
+        }
+        best.wave_paths = r.pass_by_pass ? 1u : (uint32_t)std::min<uint64_t>(paths, rt::kFormPaths);
         finish_tune(ctx, rt::kTuneRender, s.triangle_count(), P, best, (uint32_t)cands.size(), out);
     });
 }
@@ -1245,7 +1267,7 @@ int reina_autotune_batch(reina_ctx* ctx, const reina_render_job* jobs, uint32_t 
                     waves.push_back(fit_wave(w, samples));
             const uint32_t default_wave = fit_wave(REINA_DEFAULT_WAVE_PATHS, samples);
             for (uint32_t wave : waves)
-                for (int refill : {rt::kDefaultWaveRefill, rt::kDefaultRefill}) {   // the grid form, the cooperative form
+                for (int refill : {rt::kDefaultWaveRefill, rt::kDefaultRefill}) {   // the engine's choice, the cooperative form
                     rt::TraceConfig c;
                     c.refill = refill;
                     ctx->wave_paths = wave;

@@ -44,3 +44,14 @@ def test_refused_entries(R, own_ctx, tmp_path, line):
     p.write_text(line + "\n")
     with pytest.raises(R.ReinaError):
         R.autotune_load(own_ctx, p)
+
+
+def test_paths_of_a_frames_entry(R, own_ctx, tmp_path):
+    """A frame's entry keeps the paths it was timed with in the wave_paths column; as tuning it is no wave size."""
+    src, out = tmp_path / "in.txt", tmp_path / "out.txt"
+    src.write_text("2 10 12 8 128 12 65536 1 2\n3 10 12 8 128 12 65536 1 2\n")
+    R.autotune_load(own_ctx, src)
+    assert R.autotune_lookup(own_ctx, R.TUNE_RENDER, 1 << 10, 1 << 12)["wave_paths"] == R.DEFAULT_WAVE_PATHS
+    assert R.autotune_lookup(own_ctx, R.TUNE_BATCH, 1 << 10, 1 << 12)["wave_paths"] == 65536
+    R.autotune_save(own_ctx, out)
+    assert "2 10 12 8 128 12 65536 1 2 0" in out.read_text().splitlines()
