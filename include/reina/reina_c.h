@@ -65,13 +65,14 @@ void reina_ctx_destroy(reina_ctx* ctx);
 int reina_ctx_sm_count(const reina_ctx* ctx);
 
 /* Launch parameters of the traversal kernels and of batched renders (no counterpart in the reference,
- * whose traversal and scheduling belong to the Vulkan implementation).  Every setting gives the same results; only speed
- * differs.  0 selects the default of a field.
+ * whose traversal and scheduling belong to the Vulkan implementation).  Every setting gives the same results;
+ * only speed differs.  0 selects the default of a field.
  *   refill: the traversal launch form.  1..32 (0 = the default, 8): the warp-cooperative persistent form
  *            (block 128): warps keep 32 rays in flight, take new rays once `refill` of their lanes are idle,
  *            and share each step's triangle tests and the finished rays' hit refinement over all 32 lanes (at
- *            the default, casts of at most 192 rays per SM, 256 in scenes of 512 or more nodes and two-level ones, run
- *            eight lanes per ray instead: 1,000 rays of an 81,920-triangle scene 25 us a call against 35 us);
+ *            the default, casts of at most 192 rays per SM, 256 in scenes of 512 or more nodes and two-level
+ *            ones, run eight lanes per ray instead: 1,000 rays of an 81,920-triangle scene 25 us a call against
+ *            35 us);
  *            REINA_REFILL_GRID: one thread per ray (the grid form).  On the 1.3M-triangle ray cast
  *            (2,097,152 rays) closest hit 0.42 ms cooperative against 0.80 ms grid; on 256 instances of a
  *            20,480-triangle model 0.93 against 1.48 ms.  Ray casts only: the wavefront kernels of frames and
@@ -92,10 +93,10 @@ int reina_ctx_sm_count(const reina_ctx* ctx);
  *            the path state costs 164 bytes per slot and wave in flight (wave_lanes): the waves run on
  *            streams of their own, so that one wave's last bounces (few long paths) overlap the next
  *            waves' first ones.  Cooperative waves (wave_refill) take the slots of all lanes and run one
- *            after the other, since each fills the GPU by itself.  A wave holds any number of samples of a pixel of a NEE+MIS job and at
- *            most one of a job in the reference's mode; a batch gets no more slots than one wave can
- *            hold of it, rounded up to a power of two (at least 2^16); an engine already built with
- *            more slots than that (up to wave_paths) is reused.
+ *            after the other, since each fills the GPU by itself.  A wave holds any number of samples of a
+ *            pixel of a NEE+MIS job and at most one of a job in the reference's mode; a batch gets no more
+ *            slots than one wave can hold of it, rounded up to a power of two (at least 2^16); an engine
+ *            already built with more slots than that (up to wave_paths) is reused.
  *   batch_flags: REINA_BATCH_NO_GRAPHS launches each wave's kernels one by one instead of replaying a
  *            captured CUDA graph.  Waves are packed with the jobs in list order, each taking all it can
  *            use (one sample of each of its pixels), so that a wave holds few scenes and their data

@@ -1,10 +1,10 @@
-// Multi-job wavefront engine.  A wave is a set of path slots, each one (job, pixel, sample); it runs the
-// same kernel sequence as the single-frame wavefront (init, extend, per-material shade, shadow, finish),
-// with every kernel reading its path's job record for the scene, camera and integrator options.  A job
-// contributes at most one sample per pixel to a wave and its samples are scheduled in order, so each
-// pixel's samples are summed in sample order: a job's image does not depend on the jobs it shares waves
-// with.  The per-wave launch sequence is captured once per shape (bounces, materials, traversal form) into a
-// CUDA graph and replayed; only the wave descriptor (segments + job table) is copied in before each wave.
+// Multi-job wavefront engine.  A wave is a set of path slots, each one (job, pixel, sample); it runs the same
+// kernel sequence as the single-frame wavefront (init, extend, per-material shade, shadow, finish), with every
+// kernel reading its path's job record for the scene, camera and integrator options.  A job's samples are
+// scheduled in order (any number of a pixel's in one wave in NEE+MIS mode, one in the reference's mode) and
+// summed in sample order: a job's image does not depend on the jobs it shares waves with.  The per-wave launch
+// sequence is captured once per shape (bounces, materials, traversal form) into a CUDA graph and replayed;
+// only the wave descriptor (segments + job table) is copied in before each wave.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -691,13 +691,13 @@ void BatchEngine::launch_coop(const BatchLaunch& B, bool extend, int cur, uint32
     else kb_shadow_coop<MIXED, TWO, COUNT><<<grid, kCoopBlock, shared, st>>>(B, B.jobs, bounce, refill_at);
 }
 
-// The form of a call's waves: cooperative traversal or the grid form where it was asked for (reina_tuning.wave_refill),
-// else by the jobs' scenes and paths.  A call of few paths waits for each bounce's longest ray, so it traces with eight
-// lanes per ray (frames of 8 bounces with 4.6k / 12k / 30k / 46k paths, us, grid or cooperative against wide: 3 nodes
-// 268 / 271 / 285 / 303 against 223 / 258 / 322 / 410; zoo of 12 instances 962 / 995 / 1061 / 1096 against 656 / 788 /
-// 1036 / 1409; 64 instances 1275 / 1340 / 1428 / 1503 against 749 / 925 / 1231 / 1692; 82k triangles 743 / 789 / 851 / 894
-// against 492 / 521 / 601 / 703, and 63k paths 934 against 816).  (Counting waves without that request run the grid form, whose counts repeat from
-// run to run.)
+// The form of a call's waves: cooperative traversal or the grid form where it was asked for
+// (reina_tuning.wave_refill), else by the jobs' scenes and paths.  A call of few paths waits for each bounce's
+// longest ray, so it traces with eight lanes per ray (frames of 8 bounces with 4.6k / 12k / 30k / 46k paths, us,
+// grid or cooperative against wide: 3 nodes 268 / 271 / 285 / 303 against 223 / 258 / 322 / 410; zoo of 12 instances
+// 962 / 995 / 1061 / 1096 against 656 / 788 / 1036 / 1409; 64 instances 1275 / 1340 / 1428 / 1503 against 749 / 925
+// / 1231 / 1692; 82k triangles 743 / 789 / 851 / 894 against 492 / 521 / 601 / 703, and 63k paths 934 against 816).
+// (Counting waves without that request run the grid form, whose counts repeat from run to run.)
 //
 // The cooperative kernels fill every SM until their queue is empty, so waves of that form run one after the other,
 // as large as the path state of all lanes allows (the launches' tails are what they lose: a 1920x1080, 16
@@ -997,7 +997,6 @@ BatchEngine::Packed BatchEngine::pack(const std::vector<BatchJob*>& jobs, bool f
         pk.shape.nee = pk.shape.nee || (j->opt.mode == kModeNeeMis && j->scene.emissive_count > 0);
         pk.shape.two = pk.shape.two || j->scene.inst_trav != nullptr;
         pk.shape.materials |= j->scene.material_mask;
-        pk.shape.nodes = std::max(pk.shape.nodes, j->scene.node_count);
         const uint64_t c0 = j->cursor;
         const uint32_t ws = wave_pos;
         uint64_t m = take[a];
@@ -1098,7 +1097,7 @@ void BatchEngine::run_all(const std::vector<BatchJob*>& jobs, cudaStream_t st, b
         check_cuda(cudaEventRecord(caller_, st), "cudaEventRecord");
         for (Lane& L : lanes_) L.ordered = false;
         for (;;) {
-            if (!lane_free()) wait_oldest();   // reuse the lane of the wave two back
+            if (!lane_free()) wait_oldest();   // reuse the lane of the oldest wave
             if (!submit_wave(jobs, fifo)) break;
         }
         while (pending()) wait_oldest();

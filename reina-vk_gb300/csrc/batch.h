@@ -88,7 +88,7 @@ struct BatchJob {
 
 class BatchEngine {
 public:
-    // `lanes` path-state buffers (1 to 4) of `wave_capacity` slots each; waves rotate over them so that
+    // `lanes` path-state buffers (1 to 16) of `wave_capacity` slots each; waves rotate over them so that
     // one wave's last bounces overlap the next waves' first ones.
     BatchEngine(int device, int sm_count, uint32_t wave_capacity, bool use_graphs,
                 const TraceConfig& trace = TraceConfig(), int lanes = 1);
@@ -148,7 +148,6 @@ private:
         bool count = false;      // counting kernels (traversal work)
         bool coop = false;       // cooperative traversal
         uint32_t wide = 0;       // traversal with eight lanes per ray: its blocks
-        uint32_t nodes = 0;      // most BVH8 nodes of a scene of the wave (not part of the sequence)
         bool operator==(const Shape& o) const {
             return bounces == o.bounces && materials == o.materials && nee == o.nee && two == o.two && mixed == o.mixed &&
                    count == o.count && coop == o.coop && wide == o.wide;

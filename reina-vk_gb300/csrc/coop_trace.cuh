@@ -266,14 +266,14 @@ __device__ __noinline__ void coop_store_finished(uint32_t n_fin, const DeviceSce
     store(item, c, valid);
 }
 
-// Traces items [0, n) of the caller's list.  load(i, o, d) gives item i's ray (origin and tmin, direction and
-// tmax); with MIXED it also returns the item's scene (batched waves mix scenes), otherwise every item uses
-// `uniform`.  store(i, hit, valid) is called by all 32 lanes together with up to 32 finished items (valid
-// marks the lanes holding one).  `next` is the global fetch counter (zero at launch); a warp refills its idle
-// lanes once at most `refill_at` lanes still trace.  Requires blocks of kCoopBlock threads and
-// coop_shared_bytes() of dynamic shared memory.  Returns the device error bits of the warp's rays.  TWO: scenes may be two-level.  VISITS: node visits per lane between two rounds of the
-// warp's bookkeeping (the triangles found meanwhile are tested at the next flush, so the closest distance a
-// visit culls with may lag by up to VISITS - 1 visits: a few more nodes, same hits).
+// Traces items [0, n) of the caller's list.  load(i, o, d) gives item i's ray (origin and tmin, direction and tmax);
+// with MIXED it also returns the item's scene (batched waves mix scenes), otherwise every item uses `uniform`.
+// store(i, hit, valid) is called by all 32 lanes together with up to 32 finished items (valid marks the lanes
+// holding one).  `next` is the global fetch counter (zero at launch); a warp refills its idle lanes once at most
+// `refill_at` lanes still trace.  Requires blocks of kCoopBlock threads and coop_shared_bytes() of dynamic shared
+// memory.  Returns the device error bits of the warp's rays.  TWO: scenes may be two-level.  VISITS: node visits per
+// lane between two rounds of the warp's bookkeeping (the triangles found meanwhile are tested at the next flush, so
+// the closest distance a visit culls with may lag by up to VISITS - 1 visits: a few more nodes, same hits).
 template <bool ANY, bool COUNT, bool REFINE, bool MIXED, bool TWO, int SS = kCoopStack, uint32_t FLUSH = kFlushGroups,
           int VISITS = TWO ? kCoopVisitsTwo : kCoopVisits, class Load, class Store>
 __device__ __forceinline__ uint32_t coop_trace(const DeviceScene& uniform, uint32_t n, uint32_t* next, uint32_t refill_at,

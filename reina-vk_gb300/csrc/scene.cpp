@@ -19,7 +19,6 @@ void mat4_identity(float m[16]) {
     for (int i = 0; i < 16; ++i) m[i] = (i % 5 == 0) ? 1.0f : 0.0f;
 }
 
-// Models::addModel (src/scene/Models.cpp:24-92): append to the global buffers with offsets.
 // Largest entry (0 of none), in lanes of its own so that the compiler's loop is not one chain of branches.
 static uint32_t largest(const std::vector<uint32_t>& v) {
     uint32_t m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -39,6 +38,7 @@ static void append_offset(std::vector<uint32_t>& dst, const std::vector<uint32_t
         for (size_t i = base; i < dst.size(); ++i) dst[i] += offset;
 }
 
+// Models::addModel (src/scene/Models.cpp:24-92): append to the global buffers with offsets.
 uint32_t Scene::define_object(ModelData&& model) {
     if (built_) fail(REINA_ERR_STATE, "Could not add model; buffers are already built");
     if (model.vertices.size() % 4 != 0) fail(REINA_ERR_INVALID, "vertices must hold 4 floats per vertex");

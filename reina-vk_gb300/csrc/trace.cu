@@ -1,6 +1,6 @@
 // Ray-cast kernels (closest hit / any hit) over the BVH8, in three launch forms — one thread per ray
-// (grid), persistent warps with dynamic ray fetch, and eight lanes per ray — and, for the grid form, in several block sizes
-// and shared-memory stack depths (the autotuner's choices; every variant computes the same hits).
+// (grid), persistent warps with dynamic ray fetch, and eight lanes per ray — and, for the grid form, in several
+// block sizes and shared-memory stack depths (the autotuner's choices; every variant computes the same hits).
 #include <cuda_runtime.h>
 
 #include <algorithm>
