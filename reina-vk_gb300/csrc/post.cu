@@ -98,8 +98,13 @@ __device__ __forceinline__ bool not_finite(float a, float b, float c) {
     return !(fabsf(a) < INFINITY && fabsf(b) < INFINITY && fabsf(c) < INFINITY);
 }
 
+// a ka + b kb + c kc with the products fused so.  The sums of three products below say which product is rounded by
+// itself: left to the compiler that changed with the code around them, and bytes of the image with it.
+__device__ __forceinline__ float sum3(float a, float ka, float b, float kb, float c, float kc) {
+    return __fmaf_rn(c, kc, __fmaf_rn(a, ka, __fmul_rn(b, kb)));
+}
 __device__ __forceinline__ bool below(const float4& p, float threshold) {
-    return p.x * 0.299f + p.y * 0.587f + p.z * 0.114f < threshold;
+    return sum3(p.x, 0.299f, p.y, 0.587f, p.z, 0.114f) < threshold;
 }
 
 // What the values that a warp left out of its sums (they are not finite) add to them: to every output they reach, at
@@ -283,17 +288,16 @@ __device__ __forceinline__ uint8_t to_unorm8(float v) {
 
 __device__ __forceinline__ float3 aces_fitted(float3 c) {
     // color * ACESInputMat: GLSL row vector times a matrix built from columns -> dot with each column
-    float3 v = make_float3(c.x * 0.59719f + c.y * 0.35458f + c.z * 0.04823f, c.x * 0.07600f + c.y * 0.90834f + c.z * 0.01566f,
-                           c.x * 0.02840f + c.y * 0.13383f + c.z * 0.83777f);
+    float3 v = make_float3(sum3(c.x, 0.59719f, c.y, 0.35458f, c.z, 0.04823f), sum3(c.x, 0.07600f, c.y, 0.90834f, c.z, 0.01566f),
+                           sum3(c.x, 0.02840f, c.y, 0.13383f, c.z, 0.83777f));
     auto fit = [](float x) {
-        const float a = x * (x + 0.0245786f) - 0.000090537f;
-        const float b = x * (0.983729f * x + 0.4329510f) + 0.238081f;
+        const float a = __fmaf_rn(x, x + 0.0245786f, -0.000090537f);
+        const float b = __fmaf_rn(x, __fmaf_rn(0.983729f, x, 0.4329510f), 0.238081f);
         return a / b;
     };
     v = make_float3(fit(v.x), fit(v.y), fit(v.z));
-    float3 o = make_float3(v.x * 1.60475f + v.y * -0.53108f + v.z * -0.07367f, v.x * -0.10208f + v.y * 1.10813f + v.z * -0.00605f,
-                           v.x * -0.00327f + v.y * -0.07276f + v.z * 1.07602f);
-    return o;
+    return make_float3(sum3(v.x, 1.60475f, v.y, -0.53108f, v.z, -0.07367f), sum3(v.y, 1.10813f, v.x, -0.10208f, v.z, -0.00605f),
+                       sum3(v.x, -0.00327f, v.y, -0.07276f, v.z, 1.07602f));
 }
 
 __device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool valid) {
