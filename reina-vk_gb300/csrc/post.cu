@@ -84,16 +84,26 @@ __global__ void __launch_bounds__(kPostBlock) k_bloom_weights(BloomTaps tx, Bloo
 }
 
 // c / wsum.  A quotient of a tiny c would take the division's slow path, and where little passes the threshold
-// most sums are zeros or the Gaussian's tails: those are divided at 2^64 times their size, unless the quotient may be
-// subnormal (scaled back it would be rounded a second time; settling that by the division's remainder cost every mean
-// more, 1920x1080 at radius 5 158 -> 163 us, than the slow path costs the few: 671x296 at radius 0.86, mostly below
-// the threshold, 29.6 -> 32.8 us, 1920x1080 157.4 -> 157.6 us).
-__device__ __forceinline__ float blur_mean(float c, float wsum) {
-    if (!(wsum >= 0.0001f)) return wsum < 0.0001f ? 0.0f : wsum;
-    const bool tiny = fabsf(c) < 0x1p-60f && fabsf(c) >= wsum * 0x1p-125f, zero = c == 0.0f;
-    const float q = (zero ? wsum : (tiny ? c * 0x1p64f : c)) / wsum;
-    return zero ? c : (tiny ? q * 0x1p-64f : q);
-}
+// most sums are zeros or the Gaussian's tails: those are divided at 2^64 times their size.  Scaled back, a
+// subnormal quotient is rounded a second time, which goes wrong only where the first one left it midway between
+// two subnormals: settle() lets the division's remainder decide on which side of the midpoint it lies.  (Leaving
+// subnormal quotients to the plain division took 33 us instead of 19 us for 671x296 at radius 0.86 with few
+// pixels above the threshold.)
+struct Mean {
+    float n, q, r;   // scaled dividend and quotient, c / wsum but for settle()
+    __device__ __forceinline__ Mean(float c, float wsum) {
+        const bool tiny = fabsf(c) < 0x1p-60f, zero = c == 0.0f;
+        n = zero ? wsum : (tiny ? c * 0x1p64f : c);
+        q = n / wsum;
+        r = zero ? c : (tiny ? q * 0x1p-64f : q);
+        if (!(wsum >= 0.0001f)) r = wsum < 0.0001f ? 0.0f : wsum;
+    }
+    __device__ __forceinline__ void settle(float wsum) {
+        const float left = q - r * 0x1p64f, rest = fmaf(-q, wsum, n);   // exact where r is subnormal
+        if (fabsf(left) == 0x1p-86f && rest != 0.0f && (rest > 0.0f) == (left > 0.0f)) r += copysignf(0x1p-149f, left);
+    }
+};
+constexpr float kSettle = 0x1p-62f;   // means with |q| below it may be subnormal
 __device__ __forceinline__ bool not_finite(float a, float b, float c) {
     return !(fabsf(a) < INFINITY && fabsf(b) < INFINITY && fabsf(c) < INFINITY);
 }
@@ -175,10 +185,15 @@ __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restric
         float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (x >= 0 && x < W) p = __ldg(src + x);
         if (below(p, threshold)) p.x = p.y = p.z = 0.0f;
-        bad = bad || not_finite(p.x, p.y, p.z);
-        row[j] = not_finite(p.x, 0.0f, 0.0f) ? 0.0f : p.x;
-        row[stride + j] = not_finite(p.y, 0.0f, 0.0f) ? 0.0f : p.y;
-        row[2 * stride + j] = not_finite(p.z, 0.0f, 0.0f) ? 0.0f : p.z;
+        if (not_finite(p.x, p.y, p.z)) {
+            bad = true;
+            p.x = not_finite(p.x, 0.0f, 0.0f) ? 0.0f : p.x;
+            p.y = not_finite(p.y, 0.0f, 0.0f) ? 0.0f : p.y;
+            p.z = not_finite(p.z, 0.0f, 0.0f) ? 0.0f : p.z;
+        }
+        row[j] = p.x;
+        row[stride + j] = p.y;
+        row[2 * stride + j] = p.z;
     }
     const int far = t.K - t.near;
     for (int j = threadIdx.x; j < 2 * far; j += blockDim.x) {
@@ -230,10 +245,10 @@ __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restric
 #pragma unroll
         for (int k = 0; k < kXOut; ++k) {
             const int x = xw + 32 * k + lane;
-            if (x >= xe) break;
-            const float m = blur_mean(stage[32 * k + lane], wsum);
-            flag = flag || !(fabsf(m) < INFINITY);
-            dst[ch * plane + x] = m;
+            Mean m(stage[32 * k + lane], wsum);
+            if (fabsf(m.q) < kSettle) m.settle(wsum);
+            flag = flag || !(fabsf(m.r) < INFINITY);
+            if (x < xe) dst[ch * plane + x] = m.r;
         }
     }
     const int any_flag = __syncthreads_or(flag ? 1 : 0);
@@ -269,11 +284,14 @@ __global__ void __launch_bounds__(kXThreads) k_blur_x_all_taps(const float4* __r
             cg += p.y * wgt;
             cb += p.z * wgt;
         }
-        const float3 m = make_float3(blur_mean(cr, wsum), blur_mean(cg, wsum), blur_mean(cb, wsum));
-        if (not_finite(m.x, m.y, m.z)) row_flags[dy] = 1;
-        dst[0] = m.x;
-        dst[plane] = m.y;
-        dst[2 * plane] = m.z;
+        Mean mr(cr, wsum), mg(cg, wsum), mb(cb, wsum);
+        mr.settle(wsum);
+        mg.settle(wsum);
+        mb.settle(wsum);
+        if (not_finite(mr.r, mg.r, mb.r)) row_flags[dy] = 1;
+        dst[0] = mr.r;
+        dst[plane] = mg.r;
+        dst[2 * plane] = mb.r;
     }
     __syncthreads();
     if ((int)threadIdx.x < min(rows, H - y0)) flags[(size_t)seg * H + y0 + threadIdx.x] = row_flags[threadIdx.x];
@@ -455,13 +473,17 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
     if (any_bad) add_not_finite(sums, blurred_x, pitch, plane, W, H, x, y0, t, flags);
     if (x >= W) return;
     const int rows = min(kYOut, H - y0);
-#pragma unroll 4
+#pragma unroll 6
     for (int r = 0; r < rows; ++r) {
         const size_t i = (size_t)(y0 + r) * W + x;
         const float4 o = __ldg(orig + i);
-        const float3 c = make_float3(o.x + blur_mean(sums[(3 * r + 0) * kSumCh], wsum) * intensity,
-                                     o.y + blur_mean(sums[(3 * r + 1) * kSumCh], wsum) * intensity,
-                                     o.z + blur_mean(sums[(3 * r + 2) * kSumCh], wsum) * intensity);
+        Mean mr(sums[(3 * r + 0) * kSumCh], wsum), mg(sums[(3 * r + 1) * kSumCh], wsum), mb(sums[(3 * r + 2) * kSumCh], wsum);
+        if (fminf(fminf(fabsf(mr.q), fabsf(mg.q)), fabsf(mb.q)) < kSettle) {   // one branch for the three
+            mr.settle(wsum);
+            mg.settle(wsum);
+            mb.settle(wsum);
+        }
+        const float3 c = make_float3(o.x + mr.r * intensity, o.y + mg.r * intensity, o.z + mb.r * intensity);
         if (combined) combined[i] = make_float4(c.x, c.y, c.z, 1.0f);
         const float3 m = aces_fitted(make_float3(c.x * exposure_scale, c.y * exposure_scale, c.z * exposure_scale));
         out[i] = make_uchar4(to_unorm8(m.x), to_unorm8(m.y), to_unorm8(m.z), 255);
