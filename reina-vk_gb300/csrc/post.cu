@@ -5,7 +5,7 @@
 // The reference's kernel has kernelSize = int(radiusPx * 3 + 0.5) taps on each side.  Its sums run over the taps
 // in order (so do these), a NaN or infinite pixel spreads over the whole kernel as it does there, and the
 // sum of the weights counts out-of-image and thresholded taps (blurCommon.h.glsl:24-31).
-// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.153 ms, against 1.561 ms with a thread
+// 1920x1080, radius 5 (289 and 163 taps a side, 72 of them not zero): 0.152 ms, against 1.561 ms with a thread
 // per pixel that summed every tap; 671x296, radius 0.86: 19 us against 37 us.
 #include <cuda_runtime.h>
 
@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(kPostBlock) k_bloom_weights(BloomTaps tx, Bloo
 // subnormal quotient is rounded a second time, which goes wrong only where the first one left it midway between
 // two subnormals: settle() lets the division's remainder decide on which side of the midpoint it lies.  (Leaving
 // subnormal quotients to the plain division took 33 us instead of 19 us for 671x296 at radius 0.86 with few
-// pixels above the threshold.)
+// pixels above the threshold.)  The reference's guard against weight sums below 0.0001 has nothing to guard: the
+// middle weight is exp(-0) = 1, or the sum is NaN (radius 0), and so are the image's pixels.
 struct Mean {
     float n, q, r;   // scaled dividend and quotient, c / wsum but for settle()
     __device__ __forceinline__ Mean(float c, float wsum) {
@@ -96,7 +97,6 @@ struct Mean {
         n = zero ? wsum : (tiny ? c * 0x1p64f : c);
         q = n / wsum;
         r = zero ? c : (tiny ? q * 0x1p-64f : q);
-        if (!(wsum >= 0.0001f)) r = wsum < 0.0001f ? 0.0f : wsum;
     }
     __device__ __forceinline__ void settle(float wsum) {
         const float left = q - r * 0x1p64f, rest = fmaf(-q, wsum, n);   // exact where r is subnormal
@@ -245,10 +245,11 @@ __global__ void __launch_bounds__(kXThreads, 3) k_blur_x(const float4* __restric
 #pragma unroll
         for (int k = 0; k < kXOut; ++k) {
             const int x = xw + 32 * k + lane;
+            if (x >= xe) break;
             Mean m(stage[32 * k + lane], wsum);
             if (fabsf(m.q) < kSettle) m.settle(wsum);
             flag = flag || !(fabsf(m.r) < INFINITY);
-            if (x < xe) dst[ch * plane + x] = m.r;
+            dst[ch * plane + x] = m.r;
         }
     }
     const int any_flag = __syncthreads_or(flag ? 1 : 0);
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(32 * kYWarps, 6) k_blur_y_tonemap(const float*
     if (any_bad) add_not_finite(sums, blurred_x, pitch, plane, W, H, x, y0, t, flags);
     if (x >= W) return;
     const int rows = min(kYOut, H - y0);
-#pragma unroll 6
+#pragma unroll 4
     for (int r = 0; r < rows; ++r) {
         const size_t i = (size_t)(y0 + r) * W + x;
         const float4 o = __ldg(orig + i);
